@@ -9,14 +9,17 @@
 //
 // The reference sweeps the lines of each direction in lexicographic order,
 // Gauss-Seidel style: an x line (j,k) reads the new values of lines (j-1,k)
-// and (j,k-1) and the old values of (j+1,k) and (j,k+1).  Lines on one
-// anti-diagonal j + k = d read only lines of d-1 (new) and d+1 (old), so
-// one launch per anti-diagonal, in increasing d, solves every line of it at
-// once and reproduces the lexicographic sweep exactly (y lines: i + k, z
-// lines: i + j).  Each thread solves one line by the reference's Thomas
-// recursion with the coefficients formed row by row in the reference's
-// operation order; this file is compiled without FMA contraction, so the
-// result is bit-identical to the sequential sweep.
+// and (j,k-1) and the old values of (j+1,k) and (j,k+1).  A sweep is
+// therefore a chain of lines, and a line a chain of rows; everything that
+// is not on those chains is taken off them.  The pivots of the Thomas
+// recursion depend on the coefficients alone: k_ad_factor forms them for
+// all lines at once.  k_ad_sweep then runs the lines as a wavefront, one
+// block per column of lines (all k of one j, say), each block waiting for
+// its neighbour's line through a progress counter in global memory, so the
+// blocks work on one anti-diagonal without a launch between diagonals.
+// Every operation of a row is the reference's, in its order, and this file
+// is compiled without FMA contraction: the result is bit-identical to the
+// sequential sweep.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -30,9 +33,14 @@
 namespace fg {
 namespace ad {
 
+// 1-D arrays of each axis (reference indexing 0..n+1): the share of cell i
+// in the value at its lower node (CORE_GRID.F90:194-202), 1/width, and
+// set_solve_ad's couplings
+struct MetAxis {
+  const double *f, *di, *am, *ap;
+};
 struct Met {
-  const double *x, *y, *z, *xc, *yc, *zc, *dxi, *dyi, *dzi;
-  const double *amx, *apx, *amy, *apy, *amz, *apz;  // set_solve_ad
+  MetAxis a[3];
 };
 
 struct Dims {
@@ -41,80 +49,368 @@ struct Dims {
   __device__ __forceinline__ long long id(int i, int j, int k) const { return i + NX * (j + NY * (long long)k); }
 };
 
-struct Coef {
-  double amx, apx, acx, amy, apy, acy, amz, apz, acz;
+// the coupling to the lower and upper neighbour along one axis and the
+// axis's share of the diagonal (CORE_SOLVE_AD.F90:215-330): diffusion, then
+// the implicit convection of the faces f0 and f1 of cell s, central for
+// 25 <= i <= 375 (the reference's switch is on i for all three directions),
+// first-order upwind elsewhere
+struct AxisCoef {
+  double lo, hi, ac;
 };
-
-__device__ __forceinline__ double fint(const double *x, const double *xc, int i) {
-  return (x[i] - xc[i - 1]) / (xc[i] - xc[i - 1]);
+__device__ __forceinline__ AxisCoef axis_coef(const MetAxis &m, int s, double f0, double f1, double half_dt,
+                                              bool central) {
+  AxisCoef q;
+  const double am = m.am[s], ap = m.ap[s], di = m.di[s];
+  q.ac = -(am + ap);
+  if (central) {
+    const double t0 = m.f[s], t1 = m.f[s + 1];
+    q.lo = am - half_dt * f0 * (1.0 - t0) * di;
+    q.hi = ap + half_dt * f1 * t1 * di;
+    q.ac = q.ac + half_dt * (f1 * (1.0 - t1) - f0 * t0) * di;
+  } else {
+    const double s0 = copysign(1.0, f0), s1 = copysign(1.0, f1);
+    q.lo = am - half_dt * (0.5 * (1.0 + s0)) * f0 * di;
+    q.hi = ap + half_dt * (0.5 * (1.0 - s1)) * f1 * di;
+    q.ac = q.ac + half_dt * (f1 * (0.5 * (1.0 + s1)) - f0 * (0.5 * (1.0 - s0))) * di;
+  }
+  return q;
 }
 
-// the coefficients of cell (i,j,k) as every sweep and the residual form
-// them (CORE_SOLVE_AD.F90:215-330): diffusion, then the implicit
-// convection of each direction, central for 25 <= i <= 375 (the
-// reference's switch is on i for all three directions), first-order
-// upwind elsewhere
-__device__ void cell(const Dims &d, const Met &m, const double *fu, const double *fv, const double *fw,
-                     double half_dt, int i, int j, int k, Coef &q) {
-  const long long id = d.id(i, j, k);
-  const long long ip = id + 1, jp = id + d.NX, kp = id + d.NX * d.NY;
-  const bool central = (i >= 25) && (i <= 375);
-  double hyb1, hyb2, tmp1, tmp2;
-  q.amx = m.amx[i]; q.apx = m.apx[i]; q.acx = -(q.amx + q.apx);
-  q.amy = m.amy[j]; q.apy = m.apy[j]; q.acy = -(q.amy + q.apy);
-  q.amz = m.amz[k]; q.apz = m.apz[k]; q.acz = -(q.amz + q.apz);
-  const double fu0 = fu[id], fu1 = fu[ip], fv0 = fv[id], fv1 = fv[jp], fw0 = fw[id], fw1 = fw[kp];
-  hyb1 = 0.5 * (1.0 + copysign(1.0, fu0)); hyb2 = 0.5 * (1.0 - copysign(1.0, fu1));
-  tmp1 = 1.0 - fint(m.x, m.xc, i); tmp2 = fint(m.x, m.xc, i + 1);
-  if (central) {
-    q.amx = q.amx - half_dt * fu0 * tmp1 * m.dxi[i];
-    q.apx = q.apx + half_dt * fu1 * tmp2 * m.dxi[i];
-  } else {
-    q.amx = q.amx - half_dt * hyb1 * fu0 * m.dxi[i];
-    q.apx = q.apx + half_dt * hyb2 * fu1 * m.dxi[i];
-  }
-  hyb1 = 0.5 * (1.0 - copysign(1.0, fu0)); hyb2 = 0.5 * (1.0 + copysign(1.0, fu1));
-  tmp1 = fint(m.x, m.xc, i); tmp2 = 1.0 - fint(m.x, m.xc, i + 1);
-  if (central) q.acx = q.acx + half_dt * (fu1 * tmp2 - fu0 * tmp1) * m.dxi[i];
-  else q.acx = q.acx + half_dt * (fu1 * hyb2 - fu0 * hyb1) * m.dxi[i];
+struct Faces {
+  const double *f[3];  // face_u, face_v, face_w
+};
+template <int NC>
+struct Comps {
+  double *v[NC];
+  const double *r[NC];
+};
 
-  hyb1 = 0.5 * (1.0 + copysign(1.0, fv0)); hyb2 = 0.5 * (1.0 - copysign(1.0, fv1));
-  tmp1 = 1.0 - fint(m.y, m.yc, j); tmp2 = fint(m.y, m.yc, j + 1);
-  if (central) {
-    q.amy = q.amy - half_dt * fv0 * tmp1 * m.dyi[j];
-    q.apy = q.apy + half_dt * fv1 * tmp2 * m.dyi[j];
-  } else {
-    q.amy = q.amy - half_dt * hyb1 * fv0 * m.dyi[j];
-    q.apy = q.apy + half_dt * hyb2 * fv1 * m.dyi[j];
-  }
-  hyb1 = 0.5 * (1.0 - copysign(1.0, fv0)); hyb2 = 0.5 * (1.0 + copysign(1.0, fv1));
-  tmp1 = fint(m.y, m.yc, j); tmp2 = 1.0 - fint(m.y, m.yc, j + 1);
-  if (central) q.acy = q.acy + half_dt * (fv1 * tmp2 - fv0 * tmp1) * m.dyi[j];
-  else q.acy = q.acy + half_dt * (fv1 * hyb2 - fv0 * hyb1) * m.dyi[j];
+__device__ __forceinline__ bool central_at(int i) { return i >= 25 && i <= 375; }
 
-  hyb1 = 0.5 * (1.0 + copysign(1.0, fw0)); hyb2 = 0.5 * (1.0 - copysign(1.0, fw1));
-  tmp1 = 1.0 - fint(m.z, m.zc, k); tmp2 = fint(m.z, m.zc, k + 1);
-  if (central) {
-    q.amz = q.amz - half_dt * fw0 * tmp1 * m.dzi[k];
-    q.apz = q.apz + half_dt * fw1 * tmp2 * m.dzi[k];
-  } else {
-    q.amz = q.amz - half_dt * hyb1 * fw0 * m.dzi[k];
-    q.apz = q.apz + half_dt * hyb2 * fw1 * m.dzi[k];
+// 1 on fluid non-ghost cells, 0 elsewhere
+__device__ __forceinline__ double fluid(const int8_t *ib, const int8_t *gh, long long id) {
+  return (1.0 - (double)ib[id]) * (1.0 - (double)abs((int)gh[id]));
+}
+
+// 1 / pivot of every row of every line along AXIS (CORE_TDMA.F90:22-27),
+// rows 1..n, one thread per line.  Bound by the recurrence's division; the
+// coefficients of FCHUNK rows are formed ahead of it so that their loads
+// overlap.  Lines along y and z: neighbouring threads hold neighbouring i.
+constexpr int FCHUNK = 4;
+template <int AXIS>
+__global__ void __launch_bounds__(128)
+k_ad_factor(Dims d, Met m, const int8_t *__restrict__ ib, const int8_t *__restrict__ gh, Faces F, double half_dt,
+            double *__restrict__ binv) {
+  const int np = AXIS == 0 ? d.ny - 1 : d.nx - 1, nq = AXIS == 2 ? d.ny - 1 : d.nz - 1;
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= (long long)np * nq) return;
+  const int p = 1 + (int)(t % np), q = 1 + (int)(t / np);
+  const int n = AXIS == 0 ? d.nx : AXIS == 1 ? d.ny : d.nz;
+  const long long st[3] = {1, d.NX, d.NX * d.NY};
+  constexpr int P = AXIS == 0 ? 1 : 0, Q = AXIS == 2 ? 1 : 2;
+  const long long base = st[P] * p + st[Q] * q, step = st[AXIS];
+  double bi = 1.0, c_prev = 0.0;
+  for (int s0 = 1; s0 < n; s0 += FCHUNK) {
+    double lo[FCHUNK], hi[FCHUNK], ac[FCHUNK];
+#pragma unroll
+    for (int u = 0; u < FCHUNK; ++u) {
+      const int s = s0 + u;
+      lo[u] = hi[u] = 0.0;
+      ac[u] = 1.0;
+      if (s < n) {
+        const long long id = base + step * s;
+        const bool ce = central_at(AXIS == 0 ? s : p);
+        const double *fo = F.f[AXIS], *fp = F.f[P], *fq = F.f[Q];
+        const AxisCoef o = axis_coef(m.a[AXIS], s, fo[id], fo[id + step], half_dt, ce);
+        const AxisCoef a = axis_coef(m.a[P], p, fp[id], fp[id + st[P]], half_dt, ce);
+        const AxisCoef b = axis_coef(m.a[Q], q, fq[id], fq[id + st[Q]], half_dt, ce);
+        const double rib = fluid(ib, gh, id);
+        lo[u] = o.lo * rib;
+        hi[u] = o.hi * rib;
+        // acx + acy + acz
+        const double sum = AXIS == 0 ? o.ac + a.ac + b.ac : AXIS == 1 ? a.ac + o.ac + b.ac : a.ac + b.ac + o.ac;
+        ac[u] = 1.0 + sum * rib;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < FCHUNK; ++u) {
+      if (s0 + u < n) {
+        bi = 1.0 / (ac[u] - lo[u] * (c_prev * bi));
+        c_prev = hi[u];
+        binv[base + step * (s0 + u)] = bi;
+      }
+    }
   }
-  hyb1 = 0.5 * (1.0 - copysign(1.0, fw0)); hyb2 = 0.5 * (1.0 + copysign(1.0, fw1));
-  tmp1 = fint(m.z, m.zc, k); tmp2 = 1.0 - fint(m.z, m.zc, k + 1);
-  if (central) q.acz = q.acz + half_dt * (fw1 * tmp2 - fw0 * tmp1) * m.dzi[k];
-  else q.acz = q.acz + half_dt * (fw1 * hyb2 - fw0 * hyb1) * m.dzi[k];
+  binv[base + step * n] = 1.0 / (1.0 - 0.0 * (c_prev * bi));
+}
+
+__device__ __forceinline__ int ld_acquire(const int *p) {
+  int v;
+  asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_release(int *p, int v) {
+  asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+__device__ __forceinline__ void bar_sync(int id, int threads) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ void bar_arrive(int id, int threads) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
+// One sweep along AXIS of NC velocity components at once (they share the
+// coefficients and do not read one another).  A block takes a column of
+// lines (the second transverse index q when COLQ, else the first, p) and
+// solves its lines in increasing order of the other index; line l of column
+// c reads the new line l of column c - 1, announced in done[c - 1], and the
+// new line l - 1 of its own column.  Columns are drawn from a ticket, so a
+// column's predecessor has always started: the waits end.  Each is bounded
+// all the same; one that runs out sets *err and the blocks return.
+//
+// Warps: 0 runs the recurrence (lane c = component c) through shared
+// memory; 1 waits for the neighbour column and fetches its line; the others
+// hold R rows per thread, form the next line's coefficients while the
+// recurrence runs, then its right-hand sides, and relax.  The recurrence
+// (3 dependent operations per row down, 2 up) is the chain that bounds the
+// sweep: about (columns + lines) times one line.  Measured at 192x96x96
+// cells on a B200: see k_ad_sweep's launch in fg_itsolv_ad_device.
+constexpr int SW_POLLS = 1 << 23;
+template <int AXIS, bool COLQ, int R, int NC>
+__global__ void __launch_bounds__(64 + 512)
+k_ad_sweep(Dims d, Met m, const int8_t *__restrict__ ib, const int8_t *__restrict__ gh, Comps<NC> C, Faces F,
+           double half_dt, double omega, const double *__restrict__ binv, int *ticket, int *done, int *err) {
+  extern __shared__ __align__(16) double sw_smem[];
+  __shared__ int s_col, s_bad;
+  constexpr int P = AXIS == 0 ? 1 : 0, Q = AXIS == 2 ? 1 : 2;
+  constexpr int A = COLQ ? Q : P, B = COLQ ? P : Q;  // axes of the column index and of the line index
+  const int nn[3] = {d.nx, d.ny, d.nz};
+  const int n = nn[AXIS], nl = nn[B] - 1;
+  const long long st[3] = {1, d.NX, d.NX * d.NY};
+  const long long step = st[AXIS], sa = st[A], sb = st[B];
+  double2 *s_ab = reinterpret_cast<double2 *>(sw_smem);  // (lower coupling, 1/pivot) of row s
+  double *s_g = sw_smem + 2 * (n + 1);                   // gamma of row s + 1
+  double *s_u = s_g + (n + 1);                           // right-hand sides, then the solution
+  double *s_nb = s_u + NC * (n + 1);                     // the neighbour column's line
+  const int tid = threadIdx.x, nt = blockDim.x, warp = tid >> 5, lane = tid & 31;
+  if (tid == 0) {
+    s_col = 1 + atomicAdd(ticket, 1);
+    s_bad = 0;
+  }
+  __syncthreads();
+  const int c = s_col;
+  const long long col = sa * c;
+  const int np = nt - 64;  // row threads
+  enum { B_LINE = 1, B_RHS = 2, B_SOL = 3, B_STORED = 4 };
+
+  if (warp == 0) {
+    for (int l = 1; l <= nl; ++l) {
+      bar_sync(B_LINE, nt);
+      if (s_bad) return;
+      bar_sync(B_RHS, nt);
+      if (lane < NC) {
+        double *u = s_u + lane * (n + 1);
+        constexpr int U = 8;
+        double x = u[0];
+        int s = 1;
+        double2 ab[U];
+        double rr[U];
+        if (n >= U) {
+#pragma unroll
+          for (int e = 0; e < U; ++e) { ab[e] = s_ab[s + e]; rr[e] = u[s + e]; }
+          for (; s + 2 * U - 1 <= n; s += U) {
+            double2 ab1[U];
+            double rr1[U];
+#pragma unroll
+            for (int e = 0; e < U; ++e) { ab1[e] = s_ab[s + U + e]; rr1[e] = u[s + U + e]; }
+#pragma unroll
+            for (int e = 0; e < U; ++e) { x = (rr[e] - ab[e].x * x) * ab[e].y; u[s + e] = x; }
+#pragma unroll
+            for (int e = 0; e < U; ++e) { ab[e] = ab1[e]; rr[e] = rr1[e]; }
+          }
+#pragma unroll
+          for (int e = 0; e < U; ++e) { x = (rr[e] - ab[e].x * x) * ab[e].y; u[s + e] = x; }
+          s += U;
+        }
+        for (; s <= n; ++s) {
+          const double2 w = s_ab[s];
+          x = (u[s] - w.x * x) * w.y;
+          u[s] = x;
+        }
+        s = n - 1;
+        if (n - 1 >= U) {
+          double gg[U];
+#pragma unroll
+          for (int e = 0; e < U; ++e) { gg[e] = s_g[s - e]; rr[e] = u[s - e]; }
+          for (; s - 2 * U + 1 >= 1; s -= U) {
+            double gg1[U], rr1[U];
+#pragma unroll
+            for (int e = 0; e < U; ++e) { gg1[e] = s_g[s - U - e]; rr1[e] = u[s - U - e]; }
+#pragma unroll
+            for (int e = 0; e < U; ++e) { x = rr[e] - gg[e] * x; u[s - e] = x; }
+#pragma unroll
+            for (int e = 0; e < U; ++e) { gg[e] = gg1[e]; rr[e] = rr1[e]; }
+          }
+#pragma unroll
+          for (int e = 0; e < U; ++e) { x = rr[e] - gg[e] * x; u[s - e] = x; }
+          s -= U;
+        }
+        for (; s >= 1; --s) {
+          x = u[s] - s_g[s] * x;
+          u[s] = x;
+        }
+      }
+      __syncwarp();
+      bar_sync(B_SOL, nt - 32);
+      bar_sync(B_STORED, nt - 32);  // the row threads arrive after their stores
+      if (lane == 0) {
+        __threadfence();
+        st_release(done + c, l);
+      }
+    }
+    return;
+  }
+
+  if (warp == 1) {
+    int seen = 0;
+    for (int l = 1; l <= nl; ++l) {
+      if (c > 1 && seen < l) {
+        if (lane == 0) {
+          int polls = 0;
+          while ((seen = ld_acquire(done + c - 1)) < l) {
+            if (++polls > SW_POLLS || ((polls & 1023) == 0 && ld_acquire(err))) {
+              atomicExch(err, 1);
+              s_bad = 1;
+              seen = nl;
+              break;
+            }
+            __nanosleep(20);
+          }
+        }
+        seen = __shfl_sync(0xffffffffu, seen, 0);
+        __syncwarp();
+      }
+      const long long nb = col - sa + sb * l;
+      for (int s = 1 + lane; s < n; s += 32) {
+#pragma unroll
+        for (int e = 0; e < NC; ++e) s_nb[e * (n + 1) + s] = __ldcg(C.v[e] + nb + step * s);
+      }
+      bar_sync(B_LINE, nt);
+      if (s_bad) return;
+      bar_sync(B_RHS, nt);
+    }
+    return;
+  }
+
+  const int t = tid - 64;
+  double own[R][NC], prev[R][NC], hiA[R][NC], hiB[R][NC], rr[R][NC];
+  double cp0[R], cp1[R], cq0[R], cq1[R], am[R], g[R], bi[R], rib[R];
+  double end0[NC], end1[NC];  // rows 0 and n of the line (row thread 0)
+  // everything of line l that no line in flight changes; the line's own old
+  // values go to `own` later (relax still needs line l - 1's)
+  auto fetch = [&](int l, double (&o)[R][NC]) {
+    const long long b0 = col + sb * l;
+    const int p = COLQ ? l : c, q = COLQ ? c : l;
+#pragma unroll
+    for (int w = 0; w < R; ++w) {
+      const int s = 1 + t + np * w;
+      if (s < n) {
+        const long long id = b0 + step * s;
+        const bool ce = central_at(AXIS == 0 ? s : p);
+        const double *fo = F.f[AXIS], *fp = F.f[P], *fq = F.f[Q];
+        const double o0 = __ldg(fo + id), o1 = __ldg(fo + id + step);
+        const double p0 = __ldg(fp + id), p1 = __ldg(fp + id + st[P]);
+        const double q0 = __ldg(fq + id), q1 = __ldg(fq + id + st[Q]);
+        bi[w] = binv[id];
+        rib[w] = fluid(ib, gh, id);
+#pragma unroll
+        for (int e = 0; e < NC; ++e) {
+          rr[w][e] = C.r[e][id];
+          o[w][e] = __ldcg(C.v[e] + id);
+          hiA[w][e] = __ldcg(C.v[e] + id + sa);
+          hiB[w][e] = __ldcg(C.v[e] + id + sb);
+        }
+        const AxisCoef xo = axis_coef(m.a[AXIS], s, o0, o1, half_dt, ce);
+        const AxisCoef xp = axis_coef(m.a[P], p, p0, p1, half_dt, ce);
+        const AxisCoef xq = axis_coef(m.a[Q], q, q0, q1, half_dt, ce);
+        am[w] = xo.lo * rib[w];
+        g[w] = xo.hi * rib[w] * bi[w];
+        cp0[w] = xp.lo; cp1[w] = xp.hi;
+        cq0[w] = xq.lo; cq1[w] = xq.hi;
+      }
+    }
+    if (t == 0) {
+#pragma unroll
+      for (int e = 0; e < NC; ++e) {
+        end0[e] = __ldcg(C.v[e] + b0);
+        end1[e] = __ldcg(C.v[e] + b0 + step * n);
+      }
+    }
+  };
+  fetch(1, own);
+#pragma unroll
+  for (int w = 0; w < R; ++w) {
+    const int s = 1 + t + np * w;
+#pragma unroll
+    for (int e = 0; e < NC; ++e) prev[w][e] = s < n ? __ldcg(C.v[e] + col + step * s) : 0.0;
+  }
+  for (int l = 1; l <= nl; ++l) {
+    bar_sync(B_LINE, nt);
+    if (s_bad) return;
+#pragma unroll
+    for (int w = 0; w < R; ++w) {
+      const int s = 1 + t + np * w;
+      if (s < n) {
+#pragma unroll
+        for (int e = 0; e < NC; ++e) {
+          const double lowA = s_nb[e * (n + 1) + s], lowB = prev[w][e];
+          const double vp0 = COLQ ? lowB : lowA, vp1 = COLQ ? hiB[w][e] : hiA[w][e];
+          const double vq0 = COLQ ? lowA : lowB, vq1 = COLQ ? hiA[w][e] : hiB[w][e];
+          const double rh = rr[w][e] - (vp0 * cp0[w] + vp1 * cp1[w] + vq0 * cq0[w] + vq1 * cq1[w]);
+          s_u[e * (n + 1) + s] = rh * rib[w] + own[w][e] * (1.0 - rib[w]);
+        }
+        s_ab[s] = make_double2(am[w], bi[w]);
+        s_g[s] = g[w];
+      }
+    }
+    if (t == 0) {
+#pragma unroll
+      for (int e = 0; e < NC; ++e) {
+        s_u[e * (n + 1)] = end0[e];
+        s_u[e * (n + 1) + n] = end1[e];
+      }
+      s_ab[n] = make_double2(0.0, binv[col + sb * l + step * n]);
+    }
+    bar_sync(B_RHS, nt);
+    double nxt[R][NC];
+    if (l < nl) fetch(l + 1, nxt);
+    bar_sync(B_SOL, nt - 32);
+    const long long b0 = col + sb * l;
+#pragma unroll
+    for (int w = 0; w < R; ++w) {
+      const int s = 1 + t + np * w;
+      if (s < n) {
+#pragma unroll
+        for (int e = 0; e < NC; ++e) {
+          const double v = own[w][e] + omega * (s_u[e * (n + 1) + s] - own[w][e]);
+          __stcg(C.v[e] + b0 + step * s, v);
+          prev[w][e] = v;
+          own[w][e] = nxt[w][e];
+        }
+      }
+    }
+    bar_arrive(B_STORED, nt - 32);
+  }
 }
 
 // the lines of anti-diagonal `diag` along AXIS (0: x lines (j,k), j + k =
-// diag; 1: y lines (i,k); 2: z lines (i,j)); one thread per line, gam and
-// the forward values in the thread's slot of `scr` (2 (n+1) doubles)
+// diag; 1: y lines (i,k); 2: z lines (i,j)), one thread per line, gam and
+// the forward values in the thread's slot of `scr` (2 (n+1) doubles): for
+// lines longer than k_ad_sweep's rows per thread hold
 template <int AXIS>
-__global__ void k_ad_diag(Dims d, Met m, const int8_t *ib, const int8_t *gh, double *var, const double *r,
-                          const double *fu, const double *fv, const double *fw, double half_dt, double omega,
-                          int diag, double *scr) {
-  // the two transverse indices a (first) and b (second) of the line
+__global__ void k_ad_diag(Dims d, Met m, const int8_t *ib, const int8_t *gh, double *var, const double *r, Faces F,
+                          double half_dt, double omega, const double *binv, int diag, double *scr) {
+  constexpr int P = AXIS == 0 ? 1 : 0, Q = AXIS == 2 ? 1 : 2;
   const int amax = AXIS == 0 ? d.ny - 1 : d.nx - 1;
   const int bmax = AXIS == 2 ? d.ny - 1 : d.nz - 1;
   const int a0 = max(1, diag - bmax), a1 = min(amax, diag - 1);
@@ -123,93 +419,124 @@ __global__ void k_ad_diag(Dims d, Met m, const int8_t *ib, const int8_t *gh, dou
   if (a > a1) return;
   const int b = diag - a;
   const int n = AXIS == 0 ? d.nx : AXIS == 1 ? d.ny : d.nz;  // rows 0..n, unknowns 1..n-1
+  const long long st[3] = {1, d.NX, d.NX * d.NY};
+  const long long base = st[P] * a + st[Q] * b, step = st[AXIS];
   double *g = scr + (size_t)t * 2 * (n + 1), *u = g + (n + 1);
-  auto at = [&](int s) -> long long {
-    return AXIS == 0 ? d.id(s, a, b) : AXIS == 1 ? d.id(a, s, b) : d.id(a, b, s);
-  };
-  // row 0: the trivial equation u = var (diagonal 1)
-  double binv = 1.0 / 1.0;
-  u[0] = var[at(0)] * binv;
-  double c_prev = 0.0;
+  u[0] = var[base];  // row 0: the trivial equation u = var
+  double c_prev = 0.0, bi = 1.0;
   for (int s = 1; s <= n; ++s) {
-    double am, ac, ap, rh;
-    const long long id = at(s);
+    double am = 0.0, ap = 0.0, rh;
+    const long long id = base + step * s;
     if (s == n) {
-      am = 0.0; ap = 0.0; ac = 1.0; rh = var[id];
+      rh = var[id];
     } else {
-      const int i = AXIS == 0 ? s : a;
-      const int j = AXIS == 1 ? s : AXIS == 0 ? a : b;
-      const int k = AXIS == 2 ? s : b;
-      Coef q;
-      cell(d, m, fu, fv, fw, half_dt, i, j, k, q);
-      double lo, hi;  // the line's own couplings
-      if (AXIS == 0) {
-        rh = r[id] - (var[id - d.NX] * q.amy + var[id + d.NX] * q.apy + var[id - d.NX * d.NY] * q.amz +
-                      var[id + d.NX * d.NY] * q.apz);
-        lo = q.amx; hi = q.apx;
-      } else if (AXIS == 1) {
-        rh = r[id] - (var[id - 1] * q.amx + var[id + 1] * q.apx + var[id - d.NX * d.NY] * q.amz +
-                      var[id + d.NX * d.NY] * q.apz);
-        lo = q.amy; hi = q.apy;
-      } else {
-        rh = r[id] - (var[id - 1] * q.amx + var[id + 1] * q.apx + var[id - d.NX] * q.amy + var[id + d.NX] * q.apy);
-        lo = q.amz; hi = q.apz;
-      }
-      const double rib = (1.0 - (double)ib[id]) * (1.0 - (double)abs((int)gh[id]));
-      am = lo * rib;
-      ap = hi * rib;
-      ac = 1.0 + (q.acx + q.acy + q.acz) * rib;
+      const bool ce = central_at(AXIS == 0 ? s : a);
+      const double *fo = F.f[AXIS], *fp = F.f[P], *fq = F.f[Q];
+      const AxisCoef o = axis_coef(m.a[AXIS], s, fo[id], fo[id + step], half_dt, ce);
+      const AxisCoef x = axis_coef(m.a[P], a, fp[id], fp[id + st[P]], half_dt, ce);
+      const AxisCoef y = axis_coef(m.a[Q], b, fq[id], fq[id + st[Q]], half_dt, ce);
+      rh = r[id] - (var[id - st[P]] * x.lo + var[id + st[P]] * x.hi + var[id - st[Q]] * y.lo +
+                    var[id + st[Q]] * y.hi);
+      const double rib = fluid(ib, gh, id);
+      am = o.lo * rib;
+      ap = o.hi * rib;
       rh = rh * rib + var[id] * (1.0 - rib);
     }
     // CORE_TDMA.F90:22-27
-    const double gam = c_prev * binv;
-    binv = 1.0 / (ac - am * gam);
-    u[s] = (rh - am * u[s - 1]) * binv;
-    g[s] = gam;
+    g[s] = c_prev * bi;
+    bi = binv[id];
+    u[s] = (rh - am * u[s - 1]) * bi;
     c_prev = ap;
   }
-  for (int s = n - 1; s >= 0; --s) u[s] = u[s] - g[s + 1] * u[s + 1];
+  for (int s = n - 1; s >= 1; --s) u[s] = u[s] - g[s + 1] * u[s + 1];
   for (int s = 1; s <= n - 1; ++s) {
-    const long long id = at(s);
+    const long long id = base + step * s;
     var[id] = var[id] + omega * (u[s] - var[id]);
   }
 }
 
-// calc_residual_ad: per block the largest |res| and the first cell (in the
-// reference's k, j, i loop order) that has it
+// calc_residual_ad of NC components: per block the largest |res| and the
+// first cell (in the reference's k, j, i loop order) that has it.  One pass
+// forms the coefficients of a cell once for all components.
+template <int NC>
 __global__ void __launch_bounds__(256)
-k_ad_resid(Dims d, Met m, const int8_t *ib, const int8_t *gh, const double *var, const double *r, const double *fu,
-           const double *fv, const double *fw, double half_dt, double *pval, long long *pidx) {
-  const long long ni = d.nx - 1, nj = d.ny - 1, nt = ni * nj * (d.nz - 1);
+k_ad_resid(Dims d, Met m, const int8_t *__restrict__ ib, const int8_t *__restrict__ gh, Comps<NC> C, Faces F,
+           double half_dt, double *pval, long long *pidx) {
+  const int ni = d.nx - 1, nj = d.ny - 1;
+  const long long nt = (long long)ni * nj * (d.nz - 1);
   const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  double v = -1.0;
-  long long at = e;
+  double v[NC];
+  long long at[NC];
+#pragma unroll
+  for (int c = 0; c < NC; ++c) { v[c] = -1.0; at[c] = e; }
   if (e < nt) {
-    const int i = 1 + (int)(e % ni), j = 1 + (int)((e / ni) % nj), k = 1 + (int)(e / (ni * nj));
-    const long long id = d.id(i, j, k), sz = d.NX * d.NY;
-    Coef q;
-    cell(d, m, fu, fv, fw, half_dt, i, j, k, q);
-    double res = r[id] - var[id] * (1.0 + q.acx + q.acy + q.acz) - var[id - 1] * q.amx - var[id + 1] * q.apx -
-                 var[id - d.NX] * q.amy - var[id + d.NX] * q.apy - var[id - sz] * q.amz - var[id + sz] * q.apz;
-    res = res * (1.0 - (double)ib[id]) * (1.0 - (double)gh[id]);
-    v = fabs(res);
+    const long long row = e / ni;
+    const int i = 1 + (int)(e - row * ni), k = 1 + (int)(row / nj), j = 1 + (int)(row - (long long)(k - 1) * nj);
+    const long long sy = d.NX, sz = d.NX * d.NY, id = d.id(i, j, k);
+    const bool ce = central_at(i);
+    const AxisCoef x = axis_coef(m.a[0], i, F.f[0][id], F.f[0][id + 1], half_dt, ce);
+    const AxisCoef y = axis_coef(m.a[1], j, F.f[1][id], F.f[1][id + sy], half_dt, ce);
+    const AxisCoef z = axis_coef(m.a[2], k, F.f[2][id], F.f[2][id + sz], half_dt, ce);
+    const double fi = 1.0 - (double)ib[id], fg = 1.0 - (double)gh[id];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      const double *var = C.v[c];
+      double res = C.r[c][id] - var[id] * (1.0 + x.ac + y.ac + z.ac) - var[id - 1] * x.lo - var[id + 1] * x.hi -
+                   var[id - sy] * y.lo - var[id + sy] * y.hi - var[id - sz] * z.lo - var[id + sz] * z.hi;
+      res = res * fi * fg;
+      v[c] = fabs(res);
+    }
   }
-  // larger value wins; equal values: the earlier cell
+  __shared__ double sv[NC][8];
+  __shared__ long long sa[NC][8];
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+    // larger value wins; equal values: the earlier cell
+    for (int o = 16; o > 0; o >>= 1) {
+      const double ov = __shfl_down_sync(0xffffffffu, v[c], o);
+      const long long oa = __shfl_down_sync(0xffffffffu, at[c], o);
+      if (ov > v[c] || (ov == v[c] && oa < at[c])) { v[c] = ov; at[c] = oa; }
+    }
+    if ((threadIdx.x & 31) == 0) { sv[c][threadIdx.x >> 5] = v[c]; sa[c][threadIdx.x >> 5] = at[c]; }
+  }
+  __syncthreads();
+  if (threadIdx.x < NC) {
+    const int c = threadIdx.x;
+    double bv = sv[c][0];
+    long long ba = sa[c][0];
+    for (int w = 1; w < 8; ++w)
+      if (sv[c][w] > bv || (sv[c][w] == bv && sa[c][w] < ba)) { bv = sv[c][w]; ba = sa[c][w]; }
+    pval[(size_t)c * gridDim.x + blockIdx.x] = bv;
+    pidx[(size_t)c * gridDim.x + blockIdx.x] = ba;
+  }
+}
+
+// the largest of the nb block results of component blockIdx.x, into
+// out[2 c], out[2 c + 1] (the cell as an exact double).  The reference
+// starts from resm = 0 and keeps the first cell whose |res| exceeds the
+// running maximum.
+__global__ void __launch_bounds__(1024) k_ad_resid_max(const double *pval, const long long *pidx, int nb, double *out) {
+  const double *pv = pval + (size_t)blockIdx.x * nb;
+  const long long *pi = pidx + (size_t)blockIdx.x * nb;
+  double v = 0.0;
+  long long at = 0;
+  auto take = [&](double ov, long long oa) {
+    if (ov > v || (ov == v && ov > 0.0 && oa < at)) { v = ov; at = oa; }
+  };
+  for (int b = threadIdx.x; b < nb; b += 1024) take(pv[b], pi[b]);
+  __shared__ double sv[32];
+  __shared__ long long sa[32];
   for (int o = 16; o > 0; o >>= 1) {
     const double ov = __shfl_down_sync(0xffffffffu, v, o);
     const long long oa = __shfl_down_sync(0xffffffffu, at, o);
-    if (ov > v || (ov == v && oa < at)) { v = ov; at = oa; }
+    take(ov, oa);
   }
-  __shared__ double sv[8];
-  __shared__ long long sa[8];
   if ((threadIdx.x & 31) == 0) { sv[threadIdx.x >> 5] = v; sa[threadIdx.x >> 5] = at; }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int w = 1; w < 8; ++w)
-      if (sv[w] > v || (sv[w] == v && sa[w] < at)) { v = sv[w]; at = sa[w]; }
-    pval[blockIdx.x] = v;
-    pidx[blockIdx.x] = at;
-  }
+  if (threadIdx.x != 0) return;
+  for (int w = 1; w < 32; ++w) take(sv[w], sa[w]);
+  out[2 * blockIdx.x] = v;
+  out[2 * blockIdx.x + 1] = (double)at;
 }
 
 // ---- outer velocity boundaries (CORE_SET_OUTER_BC.F90:18-509, :739-823)
@@ -343,51 +670,50 @@ using namespace fg;
 namespace {
 
 // set_solve_ad on the host (CORE_SET_SOLVERS.F90:650-675) and the metric
-// arrays, uploaded into the case's buffer
+// arrays, uploaded into the case's buffer when the time step or the
+// viscosity changed
 fg_status ad_setup(fg_case *c, const fg_ad_params *prm, ad::Met &m, ad::Dims &d) {
   if (!c->prepared) {
     fg_status st = fg_mg_prepare(c);
     if (st != FG_OK) return st;
   }
   const HLevel &L = c->lev[0];
-  const int nx = c->nx, ny = c->ny, nz = c->nz;
-  std::vector<double> amx(nx + 2, 0.0), apx(nx + 2, 0.0), amy(ny + 2, 0.0), apy(ny + 2, 0.0), amz(nz + 2, 0.0),
-      apz(nz + 2, 0.0);
-  const double nu = prm->reinv, dt = prm->dt;
-  for (int i = 1; i <= nx - 1; ++i) {
-    amx[i] = (L.dxcinv[i]) * L.dxinv[i];
-    apx[i] = (L.dxcinv[i + 1]) * L.dxinv[i];
-    amx[i] = -(0.50 * dt * nu) * amx[i];
-    apx[i] = -(0.50 * dt * nu) * apx[i];
+  const int n[3] = {c->nx, c->ny, c->nz};
+  const size_t all = 4 * ((size_t)n[0] + n[1] + n[2] + 6);
+  if (!c->d_admet || c->admet_dt != prm->dt || c->admet_nu != prm->reinv) {
+    const double nu = prm->reinv, dt = prm->dt;
+    const std::vector<double> *x[3] = {&L.x, &L.y, &L.z}, *xc[3] = {&L.xc, &L.yc, &L.zc};
+    const std::vector<double> *di[3] = {&L.dxinv, &L.dyinv, &L.dzinv}, *dci[3] = {&L.dxcinv, &L.dycinv, &L.dzcinv};
+    std::vector<double> v;
+    v.reserve(all);
+    for (int a = 0; a < 3; ++a) {
+      const size_t N = (size_t)n[a] + 2;
+      std::vector<double> f(N, 0.0), am(N, 0.0), ap(N, 0.0);
+      for (int i = 1; i <= n[a]; ++i) f[i] = ((*x[a])[i] - (*xc[a])[i - 1]) / ((*xc[a])[i] - (*xc[a])[i - 1]);
+      for (int i = 1; i <= n[a] - 1; ++i) {
+        am[i] = (*dci[a])[i] * (*di[a])[i];
+        ap[i] = (*dci[a])[i + 1] * (*di[a])[i];
+        am[i] = -(0.50 * dt * nu) * am[i];
+        ap[i] = -(0.50 * dt * nu) * ap[i];
+      }
+      for (const std::vector<double> *p : {(const std::vector<double> *)&f, di[a], (const std::vector<double> *)&am,
+                                           (const std::vector<double> *)&ap})
+        v.insert(v.end(), p->begin(), p->begin() + N);
+    }
+    if (!c->d_admet) FG_CUDA(fg::dev_alloc(&c->d_admet, all * sizeof(double)));
+    FG_CUDA(cudaMemcpyAsync(c->d_admet, v.data(), all * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+    FG_CUDA(cudaStreamSynchronize(c->stream));  // v is pageable and goes out of scope
+    c->admet_dt = dt;
+    c->admet_nu = nu;
   }
-  for (int j = 1; j <= ny - 1; ++j) {
-    amy[j] = L.dycinv[j] * L.dyinv[j];
-    apy[j] = L.dycinv[j + 1] * L.dyinv[j];
-    amy[j] = -(0.50 * dt * nu) * amy[j];
-    apy[j] = -(0.50 * dt * nu) * apy[j];
-  }
-  for (int k = 1; k <= nz - 1; ++k) {
-    amz[k] = L.dzcinv[k] * L.dzinv[k];
-    apz[k] = L.dzcinv[k + 1] * L.dzinv[k];
-    amz[k] = -(0.50 * dt * nu) * amz[k];
-    apz[k] = -(0.50 * dt * nu) * apz[k];
-  }
-  std::vector<double> v;
-  const std::vector<double> *parts[] = {&L.x,     &L.y, &L.z,   &L.xc, &L.yc, &L.zc, &L.dxinv, &L.dyinv,
-                                        &L.dzinv, &amx, &apx,   &amy,  &apy,  &amz,  &apz};
-  for (const std::vector<double> *a : parts) v.insert(v.end(), a->begin(), a->end());
-  if (!c->d_admet) FG_CUDA(fg::dev_alloc(&c->d_admet, v.size() * sizeof(double)));
-  FG_CUDA(cudaMemcpyAsync(c->d_admet, v.data(), v.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-  FG_CUDA(cudaStreamSynchronize(c->stream));  // v is pageable and goes out of scope
-  const size_t NX = (size_t)nx + 2, NY = (size_t)ny + 2, NZ = (size_t)nz + 2;
   const double *p = c->d_admet;
-  m.x = p; m.y = m.x + NX; m.z = m.y + NY;
-  m.xc = m.z + NZ; m.yc = m.xc + NX; m.zc = m.yc + NY;
-  m.dxi = m.zc + NZ; m.dyi = m.dxi + NX; m.dzi = m.dyi + NY;
-  m.amx = m.dzi + NZ; m.apx = m.amx + NX; m.amy = m.apx + NX; m.apy = m.amy + NY; m.amz = m.apy + NY;
-  m.apz = m.amz + NZ;
-  d.nx = nx; d.ny = ny; d.nz = nz;
-  d.NX = (long long)NX; d.NY = (long long)NY;
+  for (int a = 0; a < 3; ++a) {
+    const size_t N = (size_t)n[a] + 2;
+    m.a[a] = {p, p + N, p + 2 * N, p + 3 * N};
+    p += 4 * N;
+  }
+  d.nx = n[0]; d.ny = n[1]; d.nz = n[2];
+  d.NX = (long long)n[0] + 2; d.NY = (long long)n[1] + 2;
   return FG_OK;
 }
 
@@ -474,11 +800,75 @@ fg_status enqueue_outer_ghost(fg_case *c, const ad::Dims &d, double *u, double *
 
 }  // namespace
 
-extern "C" {
+namespace {
 
-fg_status fg_itsolv_ad_device(fg_case *c, double *var, const double *r, const double *face_u, const double *face_v,
-                              const double *face_w, const fg_ad_params *prm) {
-  if (!c || !var || !r || !face_u || !face_v || !face_w || !ad_params_ok(prm)) return FG_BAD_INPUT;
+// rows one thread of k_ad_sweep holds for lines of n cells' unknowns, 0 when
+// the line is too long for it
+int sweep_rows(int n) { return n <= 512 ? 1 : n <= 1024 ? 2 : n <= 2048 ? 4 : 0; }
+
+size_t sweep_smem(int n, int nc) { return (size_t)(n + 1) * (3 + 2 * nc) * sizeof(double); }
+
+template <int AXIS, bool COLQ, int R, int NC>
+cudaError_t launch_sweep(const ad::Dims &d, const ad::Met &m, const int8_t *ib, const int8_t *gh,
+                         const ad::Comps<NC> &C, const ad::Faces &F, double half_dt, double omega,
+                         const double *binv, int *sync, cudaStream_t s) {
+  const int nn[3] = {d.nx, d.ny, d.nz};
+  constexpr int P = AXIS == 0 ? 1 : 0, Q = AXIS == 2 ? 1 : 2;
+  const int n = nn[AXIS], cols = nn[COLQ ? Q : P] - 1;
+  const int rows = ((n - 1 + R - 1) / R + 31) / 32 * 32;
+  const size_t sm = sweep_smem(n, NC);
+  auto kern = ad::k_ad_sweep<AXIS, COLQ, R, NC>;
+  if (sm > 48 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if (e != cudaSuccess) return e;
+  }
+  kern<<<cols, 64 + rows, sm, s>>>(d, m, ib, gh, C, F, half_dt, omega, binv, sync + 1, sync + 2, sync);
+  return cudaGetLastError();
+}
+
+template <int AXIS, bool COLQ, int NC>
+cudaError_t sweep_by_rows(const ad::Dims &d, const ad::Met &m, const int8_t *ib, const int8_t *gh,
+                          const ad::Comps<NC> &C, const ad::Faces &F, double half_dt, double omega,
+                          const double *binv, int *sync, cudaStream_t s) {
+  const int n = AXIS == 0 ? d.nx : AXIS == 1 ? d.ny : d.nz;
+  switch (sweep_rows(n)) {
+    case 1: return launch_sweep<AXIS, COLQ, 1, NC>(d, m, ib, gh, C, F, half_dt, omega, binv, sync, s);
+    case 2: return launch_sweep<AXIS, COLQ, 2, NC>(d, m, ib, gh, C, F, half_dt, omega, binv, sync, s);
+    default: return launch_sweep<AXIS, COLQ, 4, NC>(d, m, ib, gh, C, F, half_dt, omega, binv, sync, s);
+  }
+}
+
+template <int AXIS, int NC>
+cudaError_t sweep_axis(const ad::Dims &d, const ad::Met &m, const int8_t *ib, const int8_t *gh,
+                       const ad::Comps<NC> &C, const ad::Faces &F, double half_dt, double omega, double *binv,
+                       int *sync, double *scr, cudaStream_t s, long long &launches) {
+  const int np = AXIS == 0 ? d.ny - 1 : d.nx - 1, nq = AXIS == 2 ? d.ny - 1 : d.nz - 1;
+  const int n = AXIS == 0 ? d.nx : AXIS == 1 ? d.ny : d.nz;
+  const long long lines = (long long)np * nq;
+  ad::k_ad_factor<AXIS><<<(unsigned)((lines + 127) / 128), 128, 0, s>>>(d, m, ib, gh, F, half_dt, binv);
+  ++launches;
+  if (sweep_rows(n)) {
+    ++launches;
+    // y and z lines: a column holds all i of one plane, so a block's loads of
+    // neighbouring lines share sectors; x lines: the shorter of the two
+    // directions, which needs fewer blocks
+    if (AXIS != 0 || nq < np)
+      return sweep_by_rows<AXIS, true, NC>(d, m, ib, gh, C, F, half_dt, omega, binv, sync, s);
+    return sweep_by_rows<AXIS, false, NC>(d, m, ib, gh, C, F, half_dt, omega, binv, sync, s);
+  }
+  for (int e = 0; e < NC; ++e)
+    for (int diag = 2; diag <= np + nq; ++diag) {
+      const int nl = std::min(np, diag - 1) - std::max(1, diag - nq) + 1;
+      ad::k_ad_diag<AXIS><<<(unsigned)((nl + 63) / 64), 64, 0, s>>>(d, m, ib, gh, C.v[e], C.r[e], F, half_dt, omega,
+                                                                    binv, diag, scr);
+      ++launches;
+    }
+  return cudaGetLastError();
+}
+
+// one itsolv_ad pass of NC components: x, then y, then z sweeps
+template <int NC>
+fg_status ad_sweeps(fg_case *c, const ad::Comps<NC> &C, const ad::Faces &F, const fg_ad_params *prm) {
   cudaSetDevice(c->device);
   ad::Met m;
   ad::Dims d;
@@ -487,48 +877,49 @@ fg_status fg_itsolv_ad_device(fg_case *c, double *var, const double *r, const do
   const size_t nref = (size_t)(c->nx + 2) * (c->ny + 2) * (c->nz + 2);
   const int8_t *ib = c->d_refmask, *gh = c->d_refmask + nref;
   const double half_dt = prm->crank_nicolson ? 0.5 * prm->dt : 0.0;
-  // scratch: the longest anti-diagonal of any direction times the longest line
   const int nmax = std::max(c->nx, std::max(c->ny, c->nz));
-  const int lmax = std::max(std::min(c->ny, c->nz), std::max(std::min(c->nx, c->nz), std::min(c->nx, c->ny)));
-  double *scr = nullptr;
-  FG_CUDA(fg::dev_alloc(&scr, (size_t)lmax * 2 * (nmax + 1) * sizeof(double)));
-  cudaStream_t s = c->stream;
-  cudaError_t e = cudaSuccess;
-  long long launches = 0;
-  for (int axis = 0; axis < 3 && e == cudaSuccess; ++axis) {
-    const int amax = axis == 0 ? c->ny - 1 : c->nx - 1;
-    const int bmax = axis == 2 ? c->ny - 1 : c->nz - 1;
-    for (int diag = 2; diag <= amax + bmax && e == cudaSuccess; ++diag) {
-      const int nl = std::min(amax, diag - 1) - std::max(1, diag - bmax) + 1;
-      if (nl <= 0) continue;
-      const unsigned nb = (unsigned)((nl + 63) / 64);
-      if (axis == 0)
-        ad::k_ad_diag<0><<<nb, 64, 0, s>>>(d, m, ib, gh, var, r, face_u, face_v, face_w, half_dt, prm->omega_ad, diag,
-                                           scr);
-      else if (axis == 1)
-        ad::k_ad_diag<1><<<nb, 64, 0, s>>>(d, m, ib, gh, var, r, face_u, face_v, face_w, half_dt, prm->omega_ad, diag,
-                                           scr);
-      else
-        ad::k_ad_diag<2><<<nb, 64, 0, s>>>(d, m, ib, gh, var, r, face_u, face_v, face_w, half_dt, prm->omega_ad, diag,
-                                           scr);
-      ++launches;
-      e = cudaGetLastError();
-    }
+  // scratch: the pivots, per sweep an error flag, a ticket and the columns'
+  // progress, and for lines too long for k_ad_sweep one line per diagonal's
+  // thread
+  const size_t nsync = (size_t)nmax + 2;
+  size_t nscr = 0;
+  if (!sweep_rows(nmax)) {
+    const int lmax = std::max(std::min(c->ny, c->nz), std::max(std::min(c->nx, c->nz), std::min(c->nx, c->ny)));
+    nscr = (size_t)lmax * 2 * (nmax + 1);
   }
+  double *ws = nullptr;
+  FG_CUDA(fg::dev_alloc(&ws, (nref + nscr) * sizeof(double) + 3 * nsync * sizeof(int)));
+  double *binv = ws, *scr = ws + nref;
+  int *sync = reinterpret_cast<int *>(scr + nscr);
+  cudaStream_t s = c->stream;
+  long long launches = 0;
+  cudaError_t e = cudaMemsetAsync(sync, 0, 3 * nsync * sizeof(int), s);
+  const double om = prm->omega_ad;
+  if (e == cudaSuccess) e = sweep_axis<0, NC>(d, m, ib, gh, C, F, half_dt, om, binv, sync, scr, s, launches);
+  if (e == cudaSuccess) e = sweep_axis<1, NC>(d, m, ib, gh, C, F, half_dt, om, binv, sync + nsync, scr, s, launches);
+  if (e == cudaSuccess)
+    e = sweep_axis<2, NC>(d, m, ib, gh, C, F, half_dt, om, binv, sync + 2 * nsync, scr, s, launches);
   note_launches(launches);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  fg::dev_free(scr);
+  int gave_up[3] = {0, 0, 0};
+  for (int a = 0; a < 3 && e == cudaSuccess; ++a)
+    e = cudaMemcpyAsync(&gave_up[a], sync + a * nsync, sizeof(int), cudaMemcpyDeviceToHost, s);
+  const cudaError_t es = cudaStreamSynchronize(s);
+  if (e == cudaSuccess) e = es;
+  {
+    fg::IdleFree drained;  // the stream that used the scratch is idle
+    fg::dev_free(ws);
+  }
   if (e != cudaSuccess) {
     set_last_error(cudaGetErrorString(e), __FILE__, __LINE__);
     return FG_CUDA_ERROR;
   }
-  return FG_OK;
+  return gave_up[0] || gave_up[1] || gave_up[2] ? FG_TIMEOUT : FG_OK;
 }
 
-fg_status fg_calc_residual_ad_device(fg_case *c, const double *var, const double *r, const double *face_u,
-                                     const double *face_v, const double *face_w, const fg_ad_params *prm,
-                                     double *resm, int *loc) {
-  if (!c || !var || !r || !face_u || !face_v || !face_w || !ad_params_ok(prm) || !resm) return FG_BAD_INPUT;
+// calc_residual_ad of NC components: resm[c] and loc[3 c ..]
+template <int NC>
+fg_status ad_residuals(fg_case *c, const ad::Comps<NC> &C, const ad::Faces &F, const fg_ad_params *prm,
+                       double *resm, int *loc) {
   cudaSetDevice(c->device);
   ad::Met m;
   ad::Dims d;
@@ -540,39 +931,53 @@ fg_status fg_calc_residual_ad_device(fg_case *c, const double *var, const double
   const long long nt = (long long)(c->nx - 1) * (c->ny - 1) * (c->nz - 1);
   const unsigned nb = (unsigned)((nt + 255) / 256);
   double *pv = nullptr;
-  long long *pi = nullptr;
-  FG_CUDA(fg::dev_alloc(&pv, (size_t)nb * sizeof(double)));
-  cudaError_t e = fg::dev_alloc(&pi, (size_t)nb * sizeof(long long));
-  std::vector<double> hv(nb);
-  std::vector<long long> hi(nb);
-  if (e == cudaSuccess) {
-    ad::k_ad_resid<<<nb, 256, 0, c->stream>>>(d, m, ib, gh, var, r, face_u, face_v, face_w, half_dt, pv, pi);
-    note_launches(1);
-    e = cudaGetLastError();
+  FG_CUDA(fg::dev_alloc(&pv, (2 * NC * (size_t)nb + 2 * NC) * sizeof(double)));
+  long long *pi = reinterpret_cast<long long *>(pv + NC * (size_t)nb);
+  double *out = pv + 2 * NC * (size_t)nb;
+  ad::k_ad_resid<NC><<<nb, 256, 0, c->stream>>>(d, m, ib, gh, C, F, half_dt, pv, pi);
+  ad::k_ad_resid_max<<<NC, 1024, 0, c->stream>>>(pv, pi, (int)nb, out);
+  note_launches(2);
+  cudaError_t e = cudaGetLastError();
+  double h[2 * NC] = {};
+  if (e == cudaSuccess) e = cudaMemcpyAsync(h, out, sizeof(h), cudaMemcpyDeviceToHost, c->stream);
+  const cudaError_t es = cudaStreamSynchronize(c->stream);
+  if (e == cudaSuccess) e = es;
+  {
+    fg::IdleFree drained;  // the stream that used the scratch is idle
+    fg::dev_free(pv);
   }
-  if (e == cudaSuccess) e = cudaMemcpyAsync(hv.data(), pv, nb * sizeof(double), cudaMemcpyDeviceToHost, c->stream);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(hi.data(), pi, nb * sizeof(long long), cudaMemcpyDeviceToHost, c->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-  fg::dev_free(pv);
-  fg::dev_free(pi);
   if (e != cudaSuccess) {
     set_last_error(cudaGetErrorString(e), __FILE__, __LINE__);
     return FG_CUDA_ERROR;
   }
-  // the reference starts from resm = 0 and keeps the first cell whose |res|
-  // exceeds the running maximum
-  double v = 0.0;
-  long long at = 0;
-  for (unsigned q = 0; q < nb; ++q)
-    if (hv[q] > v || (hv[q] == v && hv[q] > 0.0 && hi[q] < at)) { v = hv[q]; at = hi[q]; }
-  *resm = v;
-  if (loc) {
-    const long long ni = c->nx - 1, nj = c->ny - 1;
-    loc[0] = v > 0.0 ? 1 + (int)(at % ni) : 1;
-    loc[1] = v > 0.0 ? 1 + (int)((at / ni) % nj) : 1;
-    loc[2] = v > 0.0 ? 1 + (int)(at / (ni * nj)) : 1;
+  const long long ni = c->nx - 1, nj = c->ny - 1;
+  for (int a = 0; a < NC; ++a) {
+    const double v = h[2 * a];
+    const long long at = (long long)h[2 * a + 1];
+    resm[a] = v;
+    if (!loc) continue;
+    loc[3 * a] = v > 0.0 ? 1 + (int)(at % ni) : 1;
+    loc[3 * a + 1] = v > 0.0 ? 1 + (int)((at / ni) % nj) : 1;
+    loc[3 * a + 2] = v > 0.0 ? 1 + (int)(at / (ni * nj)) : 1;
   }
   return FG_OK;
+}
+
+}  // namespace
+
+extern "C" {
+
+fg_status fg_itsolv_ad_device(fg_case *c, double *var, const double *r, const double *face_u, const double *face_v,
+                              const double *face_w, const fg_ad_params *prm) {
+  if (!c || !var || !r || !face_u || !face_v || !face_w || !ad_params_ok(prm)) return FG_BAD_INPUT;
+  return ad_sweeps<1>(c, {{var}, {r}}, {{face_u, face_v, face_w}}, prm);
+}
+
+fg_status fg_calc_residual_ad_device(fg_case *c, const double *var, const double *r, const double *face_u,
+                                     const double *face_v, const double *face_w, const fg_ad_params *prm,
+                                     double *resm, int *loc) {
+  if (!c || !var || !r || !face_u || !face_v || !face_w || !ad_params_ok(prm) || !resm) return FG_BAD_INPUT;
+  return ad_residuals<1>(c, {{const_cast<double *>(var)}, {r}}, {{face_u, face_v, face_w}}, prm, resm, loc);
 }
 
 fg_status fg_set_outer_velocity_bc_device(fg_case *c, const double *u, const double *v, const double *w,
@@ -611,13 +1016,14 @@ fg_status fg_solve_ad_device(fg_case *c, double *u, double *v, double *w, const 
   if (!vel_bc(vb, chk)) return FG_BAD_INPUT;
   int vzg[6];
   for (int f = 0; f < 6; ++f) vzg[f] = vb->type[f] == 2;
+  // u, v, w sweep together: a pass reads its own component and the faces
+  const ad::Comps<3> C = {{u, v, w}, {nlu, nlv, nlw}};
+  const ad::Faces F = {{face_u, face_v, face_w}};
   int iter = 0, loc[3] = {1, 1, 1};
   double res2 = 1.0e10;
   fg_status st = FG_OK;
   while (st == FG_OK && iter < itermax_ad && res2 > restol_ad) {
-    st = fg_itsolv_ad_device(c, u, nlu, face_u, face_v, face_w, prm);
-    if (st == FG_OK) st = fg_itsolv_ad_device(c, v, nlv, face_u, face_v, face_w, prm);
-    if (st == FG_OK) st = fg_itsolv_ad_device(c, w, nlw, face_u, face_v, face_w, prm);
+    st = ad_sweeps<3>(c, C, F, prm);
     if (st == FG_OK) st = fg_ghostcell_velocity_device(c, u, v, w, ubi_ghost, ubi_dead, itermax_gc, restol_gcv, nullptr);
     if (st == FG_OK) st = fg_face_vel_device(c, u, v, w, bc->bcxu, bc->bcyv, bc->bczw, face_u, face_v, face_w);
     if (st == FG_OK)
@@ -626,9 +1032,7 @@ fg_status fg_solve_ad_device(fg_case *c, double *u, double *v, double *w, const 
     if (st == FG_OK) st = fg_set_outer_ghost_velocity_device(c, u, v, w, bc);
     double r[3] = {0.0, 0.0, 0.0};
     int l[3][3];
-    const double *var[3] = {u, v, w}, *rhs[3] = {nlu, nlv, nlw};
-    for (int a = 0; a < 3 && st == FG_OK; ++a)
-      st = fg_calc_residual_ad_device(c, var[a], rhs[a], face_u, face_v, face_w, prm, &r[a], l[a]);
+    if (st == FG_OK) st = ad_residuals<3>(c, C, F, prm, r, &l[0][0]);
     if (st != FG_OK) break;
     int best = 0;
     res2 = std::fabs(r[0]);

@@ -104,7 +104,10 @@ struct fg_case {
   long long geom_version = 0;      // bumped by every prepare
   // per interpolation row, for row constants formed on the device: the
   // dp/dn index, its two factors, the fallback corners and weights
-  double *d_admet = nullptr;          // momentum sweeps: metrics and set_solve_ad coefficients
+  // momentum sweeps: metrics and set_solve_ad coefficients of one time step
+  // and viscosity
+  double *d_admet = nullptr;
+  double admet_dt = 0.0, admet_nu = 0.0;
   double *d_vbcmet = nullptr;         // outer velocity boundaries: node coordinates y, z
   void *d_rcg = nullptr;
   long long rcg_version = -1;
