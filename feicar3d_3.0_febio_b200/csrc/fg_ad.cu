@@ -13,7 +13,7 @@
 // therefore a chain of lines, and a line a chain of rows; everything that
 // is not on those chains is taken off them.  The pivots of the Thomas
 // recursion depend on the coefficients alone: k_ad_factor forms them for
-// all lines at once.  k_ad_sweep then runs the lines as a wavefront, one
+// all lines at once.  k_ad_sweeps then runs the lines as a wavefront, one
 // block per column of lines (all k of one j, say), each block waiting for
 // its neighbour's line through a progress counter in global memory, so the
 // blocks work on one anti-diagonal without a launch between diagonals.
@@ -92,56 +92,85 @@ __device__ __forceinline__ double fluid(const int8_t *ib, const int8_t *gh, long
   return (1.0 - (double)ib[id]) * (1.0 - (double)abs((int)gh[id]));
 }
 
-// 1 / pivot of every row of every line along AXIS (CORE_TDMA.F90:22-27),
-// rows 1..n, one thread per line.  Bound by the recurrence's division; the
-// coefficients of FCHUNK rows are formed ahead of it so that their loads
-// overlap.  Lines along y and z: neighbouring threads hold neighbouring i.
-constexpr int FCHUNK = 4;
+// 1 / pivot of every row of every line (CORE_TDMA.F90:22-27), rows 1..n,
+// blockIdx.y = axis.  A block takes 32 lines in tiles of FT_ROWS rows: warps
+// 1..8 form a tile's coefficients in shared memory (loads along i whatever
+// the axis) and store the pivots of the tile before last, while lane l of
+// warp 0 runs line l's recurrence, whose division is the bound, over the
+// tile between.  One thread per line did the loads, the coefficients and
+// the recurrence in turn: 310 + 123 + 114 us at 192x96x96 cells, 100 us as
+// one launch of this kernel.
+constexpr int FT_ROWS = 16, FT_LINES = 32, FT_WORK = 256;
+struct FactorTile {
+  double lo[FT_ROWS][FT_LINES + 1], hi[FT_ROWS][FT_LINES + 1], ac[FT_ROWS][FT_LINES + 1];
+};
 template <int AXIS>
-__global__ void __launch_bounds__(128)
-k_ad_factor(Dims d, Met m, const int8_t *__restrict__ ib, const int8_t *__restrict__ gh, Faces F, double half_dt,
-            double *__restrict__ binv) {
-  const int np = AXIS == 0 ? d.ny - 1 : d.nx - 1, nq = AXIS == 2 ? d.ny - 1 : d.nz - 1;
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (long long)np * nq) return;
-  const int p = 1 + (int)(t % np), q = 1 + (int)(t / np);
-  const int n = AXIS == 0 ? d.nx : AXIS == 1 ? d.ny : d.nz;
-  const long long st[3] = {1, d.NX, d.NX * d.NY};
+__device__ __forceinline__ void factor_lines(const Dims &d, const Met &m, const int8_t *__restrict__ ib,
+                                             const int8_t *__restrict__ gh, const Faces &F, double half_dt,
+                                             double *__restrict__ binv, FactorTile *tile) {
   constexpr int P = AXIS == 0 ? 1 : 0, Q = AXIS == 2 ? 1 : 2;
-  const long long base = st[P] * p + st[Q] * q, step = st[AXIS];
+  const int np = AXIS == 0 ? d.ny - 1 : d.nx - 1, nq = AXIS == 2 ? d.ny - 1 : d.nz - 1;
+  const int n = AXIS == 0 ? d.nx : AXIS == 1 ? d.ny : d.nz;
+  const int groups = (np + FT_LINES - 1) / FT_LINES;  // line groups of one q
+  if (blockIdx.x >= (unsigned)(groups * nq)) return;
+  const int p0 = 1 + FT_LINES * (int)(blockIdx.x % groups), q = 1 + blockIdx.x / groups;
+  const long long st[3] = {1, d.NX, d.NX * d.NY};
+  const long long base = st[P] * p0 + st[Q] * q, step = st[AXIS];
+  const int tid = threadIdx.x;
+  const int ntile = (n - 1 + FT_ROWS - 1) / FT_ROWS;
   double bi = 1.0, c_prev = 0.0;
-  for (int s0 = 1; s0 < n; s0 += FCHUNK) {
-    double lo[FCHUNK], hi[FCHUNK], ac[FCHUNK];
+  for (int k = 0; k < ntile + 2; ++k) {
+    if (tid < 32) {
+      if (k >= 1 && k <= ntile) {
+        FactorTile &t = tile[(k - 1) & 1];
+        const int rows = min(FT_ROWS, n - 1 - (k - 1) * FT_ROWS);
+        for (int r = 0; r < rows; ++r) {
+          bi = 1.0 / (t.ac[r][tid] - t.lo[r][tid] * (c_prev * bi));
+          c_prev = t.hi[r][tid];
+          t.ac[r][tid] = bi;
+        }
+      }
+    } else {
+      FactorTile &t = tile[k & 1];
 #pragma unroll
-    for (int u = 0; u < FCHUNK; ++u) {
-      const int s = s0 + u;
-      lo[u] = hi[u] = 0.0;
-      ac[u] = 1.0;
-      if (s < n) {
-        const long long id = base + step * s;
-        const bool ce = central_at(AXIS == 0 ? s : p);
-        const double *fo = F.f[AXIS], *fp = F.f[P], *fq = F.f[Q];
-        const AxisCoef o = axis_coef(m.a[AXIS], s, fo[id], fo[id + step], half_dt, ce);
-        const AxisCoef a = axis_coef(m.a[P], p, fp[id], fp[id + st[P]], half_dt, ce);
-        const AxisCoef b = axis_coef(m.a[Q], q, fq[id], fq[id + st[Q]], half_dt, ce);
-        const double rib = fluid(ib, gh, id);
-        lo[u] = o.lo * rib;
-        hi[u] = o.hi * rib;
-        // acx + acy + acz
-        const double sum = AXIS == 0 ? o.ac + a.ac + b.ac : AXIS == 1 ? a.ac + o.ac + b.ac : a.ac + b.ac + o.ac;
-        ac[u] = 1.0 + sum * rib;
+      for (int u = 0; u < FT_ROWS * FT_LINES / FT_WORK; ++u) {
+        const int e = tid - 32 + FT_WORK * u;
+        // neighbouring threads take neighbouring i: rows along x, lines else
+        const int r = AXIS == 0 ? e % FT_ROWS : e / FT_LINES, l = AXIS == 0 ? e / FT_ROWS : e % FT_LINES;
+        const int p = p0 + l;
+        if (p > np) continue;
+        const int sd = (k - 2) * FT_ROWS + r + 1, s = k * FT_ROWS + r + 1;
+        if (k >= 2 && sd < n) binv[base + st[P] * l + step * sd] = t.ac[r][l];
+        if (k < ntile && s < n) {
+          const long long id = base + st[P] * l + step * s;
+          const bool ce = central_at(AXIS == 0 ? s : p);
+          const double *fo = F.f[AXIS], *fp = F.f[P], *fq = F.f[Q];
+          const AxisCoef o = axis_coef(m.a[AXIS], s, fo[id], fo[id + step], half_dt, ce);
+          const AxisCoef a = axis_coef(m.a[P], p, fp[id], fp[id + st[P]], half_dt, ce);
+          const AxisCoef b = axis_coef(m.a[Q], q, fq[id], fq[id + st[Q]], half_dt, ce);
+          const double rib = fluid(ib, gh, id);
+          // acx + acy + acz
+          const double sum = AXIS == 0 ? o.ac + a.ac + b.ac : AXIS == 1 ? a.ac + o.ac + b.ac : a.ac + b.ac + o.ac;
+          t.lo[r][l] = o.lo * rib;
+          t.hi[r][l] = o.hi * rib;
+          t.ac[r][l] = 1.0 + sum * rib;
+        }
       }
     }
-#pragma unroll
-    for (int u = 0; u < FCHUNK; ++u) {
-      if (s0 + u < n) {
-        bi = 1.0 / (ac[u] - lo[u] * (c_prev * bi));
-        c_prev = hi[u];
-        binv[base + step * (s0 + u)] = bi;
-      }
-    }
+    __syncthreads();
   }
-  binv[base + step * n] = 1.0 / (1.0 - 0.0 * (c_prev * bi));
+  if (tid < 32 && p0 + tid <= np) binv[base + st[P] * tid + step * n] = 1.0 / (1.0 - 0.0 * (c_prev * bi));
+}
+
+// binv: one array of `nref` values per axis
+__global__ void __launch_bounds__(32 + FT_WORK)
+k_ad_factor(Dims d, Met m, const int8_t *__restrict__ ib, const int8_t *__restrict__ gh, Faces F, double half_dt,
+            double *__restrict__ binv, long long nref) {
+  extern __shared__ __align__(16) double ft_smem[];
+  FactorTile *tile = reinterpret_cast<FactorTile *>(ft_smem);
+  if (blockIdx.y == 0) factor_lines<0>(d, m, ib, gh, F, half_dt, binv, tile);
+  else if (blockIdx.y == 1) factor_lines<1>(d, m, ib, gh, F, half_dt, binv + nref, tile);
+  else factor_lines<2>(d, m, ib, gh, F, half_dt, binv + 2 * nref, tile);
 }
 
 __device__ __forceinline__ int ld_acquire(const int *p) {
@@ -159,55 +188,88 @@ __device__ __forceinline__ void bar_arrive(int id, int threads) {
   asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
-// One sweep along AXIS of NC velocity components at once (they share the
-// coefficients and do not read one another).  A block takes a column of
-// lines (the second transverse index q when COLQ, else the first, p) and
-// solves its lines in increasing order of the other index; line l of column
-// c reads the new line l of column c - 1, announced in done[c - 1], and the
-// new line l - 1 of its own column.  Columns are drawn from a ticket, so a
-// column's predecessor has always started: the waits end.  Each is bounded
+// The x, y and z sweeps of NC velocity components at once (the components
+// share the coefficients and do not read one another).  A block takes a
+// column of lines (x and y lines: all of one k; z lines: all of one j) and
+// solves them in increasing order of the other index (x: j; y and z: i).
+// Line l of a column reads the new line l of the column before, announced in
+// that column's progress counter, and the new line l - 1 of its own.
+//
+// The sweeps overlap.  The y column k may start once the x column k + 1 is
+// done (no x line still reads or writes plane k, and the plane it reads
+// above is swept); z line l may start once every y column has passed line
+// l + 1, which the last y column's counter tells (a column never passes the
+// one before it).  Columns are drawn from a ticket in the order x, y, z, so
+// whatever a block waits for has started: the waits end.  Each is bounded
 // all the same; one that runs out sets *err and the blocks return.
 //
 // Warps: 0 runs the recurrence (lane c = component c) through shared
-// memory; 1 waits for the neighbour column and fetches its line; the others
-// hold R rows per thread, form the next line's coefficients while the
-// recurrence runs, then its right-hand sides, and relax.  The recurrence
-// (3 dependent operations per row down, 2 up) is the chain that bounds the
-// sweep: about (columns + lines) times one line.  Measured at 192x96x96
-// cells on a B200: see k_ad_sweep's launch in fg_itsolv_ad_device.
+// memory; 1 waits for the neighbour column and fetches its line; 2 announces
+// the column's progress, so that nobody else waits for the stores to become
+// visible; the others hold R rows per thread, form the next line's
+// coefficients while the recurrence runs, then its right-hand sides, and
+// relax.  The recurrence, 3 dependent operations per row down and 2 up, is
+// what bounds the pass: it takes about 35 ns per row (65 cycles for the 5
+// operations), and (ny + nz) x lines, nx y lines and ny z lines follow one
+// another, with some 7 us more for each step from a column to the next.
+// Measured at 192x96x96 cells: 2.80 ms; one launch per direction, the
+// announcement made by warp 0: 4.30 ms; one launch per anti-diagonal with
+// the coefficients and pivots inside the line: 200 ms.
 constexpr int SW_POLLS = 1 << 23;
-template <int AXIS, bool COLQ, int R, int NC>
-__global__ void __launch_bounds__(64 + 512)
-k_ad_sweep(Dims d, Met m, const int8_t *__restrict__ ib, const int8_t *__restrict__ gh, Comps<NC> C, Faces F,
-           double half_dt, double omega, const double *__restrict__ binv, int *ticket, int *done, int *err) {
-  extern __shared__ __align__(16) double sw_smem[];
-  __shared__ int s_col, s_bad;
-  constexpr int P = AXIS == 0 ? 1 : 0, Q = AXIS == 2 ? 1 : 2;
-  constexpr int A = COLQ ? Q : P, B = COLQ ? P : Q;  // axes of the column index and of the line index
-  const int nn[3] = {d.nx, d.ny, d.nz};
-  const int n = nn[AXIS], nl = nn[B] - 1;
-  const long long st[3] = {1, d.NX, d.NX * d.NY};
-  const long long step = st[AXIS], sa = st[A], sb = st[B];
-  double2 *s_ab = reinterpret_cast<double2 *>(sw_smem);  // (lower coupling, 1/pivot) of row s
-  double *s_g = sw_smem + 2 * (n + 1);                   // gamma of row s + 1
-  double *s_u = s_g + (n + 1);                           // right-hand sides, then the solution
-  double *s_nb = s_u + NC * (n + 1);                     // the neighbour column's line
-  const int tid = threadIdx.x, nt = blockDim.x, warp = tid >> 5, lane = tid & 31;
-  if (tid == 0) {
-    s_col = 1 + atomicAdd(ticket, 1);
-    s_bad = 0;
+constexpr int SW_ROLES = 96;       // threads of the three warps that hold no rows
+constexpr int SW_ROW_THREADS = 512;
+struct SweepSync {
+  int *err, *ticket, *done[3];  // done[axis][column]
+};
+
+// false when the wait was given up
+__device__ __forceinline__ bool wait_for(const int *p, int v, int *err, int &seen) {
+  for (int polls = 1; (seen = ld_acquire(p)) < v; ++polls) {
+    if (polls > SW_POLLS || ((polls & 1023) == 0 && ld_acquire(err))) {
+      atomicExch(err, 1);
+      return false;
+    }
+    __nanosleep(20);
   }
-  __syncthreads();
-  const int c = s_col;
-  const long long col = sa * c;
-  const int np = nt - 64;  // row threads
-  enum { B_LINE = 1, B_RHS = 2, B_SOL = 3, B_STORED = 4 };
+  return true;
+}
+
+template <int AXIS, int R, int NC>
+__device__ __forceinline__ void sweep_column(const Dims &d, const Met &m, const int8_t *__restrict__ ib,
+                                             const int8_t *__restrict__ gh, const Comps<NC> &C, const Faces &F,
+                                             double half_dt, double omega, const double *__restrict__ binv,
+                                             const SweepSync &sync, int c, int &s_bad, double *smem) {
+  constexpr int P = AXIS == 0 ? 1 : 0, Q = AXIS == 2 ? 1 : 2;  // axes of the line index and of the column index
+  const int nn[3] = {d.nx, d.ny, d.nz};
+  const int n = nn[AXIS], nl = nn[P] - 1;
+  const long long st[3] = {1, d.NX, d.NX * d.NY};
+  const long long step = st[AXIS], sa = st[Q], sb = st[P], col = sa * c;
+  double2 *s_ab = reinterpret_cast<double2 *>(smem);  // (lower coupling, 1/pivot) of row s
+  double *s_g = smem + 2 * (n + 1);                   // gamma of row s + 1
+  double *s_u = s_g + (n + 1);                        // right-hand sides, then the solution
+  double *s_nb = s_u + NC * (n + 1);                  // the neighbour column's line
+  const int tid = threadIdx.x, nt = blockDim.x, warp = tid >> 5, lane = tid & 31;
+  const int np = nt - SW_ROLES;  // row threads
+  int *done = sync.done[AXIS];
+  // named barriers; those with two ids alternate by line, so that the
+  // announcing warp may be a line behind
+  enum { B_RHS = 1, B_SOL = 2, B_LINE = 3, B_STORED = 5 };
+  // the sweep before this one: x columns are all there is for x
+  const int *gate = AXIS == 0 ? nullptr : sync.done[AXIS - 1] + (AXIS == 1 ? min(c + 1, d.nz - 1) : d.nz - 1);
+  if (AXIS != 0) {
+    if (tid == 0) {
+      int seen;
+      if (!wait_for(gate, AXIS == 1 ? d.ny - 1 : min(2, d.nx - 1), sync.err, seen)) s_bad = 1;
+    }
+    __syncthreads();
+    if (s_bad) return;
+  }
 
   if (warp == 0) {
     for (int l = 1; l <= nl; ++l) {
-      bar_sync(B_LINE, nt);
+      bar_sync(B_LINE + (l & 1), nt);
       if (s_bad) return;
-      bar_sync(B_RHS, nt);
+      bar_sync(B_RHS, nt - 32);
       if (lane < NC) {
         double *u = s_u + lane * (n + 1);
         constexpr int U = 8;
@@ -261,62 +323,62 @@ k_ad_sweep(Dims d, Met m, const int8_t *__restrict__ ib, const int8_t *__restric
         }
       }
       __syncwarp();
-      bar_sync(B_SOL, nt - 32);
-      bar_sync(B_STORED, nt - 32);  // the row threads arrive after their stores
-      if (lane == 0) {
-        __threadfence();
-        st_release(done + c, l);
-      }
+      bar_sync(B_SOL, np + 32);
     }
     return;
   }
 
   if (warp == 1) {
-    int seen = 0;
+    int seen = 0, gseen = 0;
     for (int l = 1; l <= nl; ++l) {
-      if (c > 1 && seen < l) {
-        if (lane == 0) {
-          int polls = 0;
-          while ((seen = ld_acquire(done + c - 1)) < l) {
-            if (++polls > SW_POLLS || ((polls & 1023) == 0 && ld_acquire(err))) {
-              atomicExch(err, 1);
-              s_bad = 1;
-              seen = nl;
-              break;
-            }
-            __nanosleep(20);
-          }
-        }
-        seen = __shfl_sync(0xffffffffu, seen, 0);
-        __syncwarp();
+      bool ok = true;
+      if (lane == 0) {
+        if (c > 1 && seen < l) ok = wait_for(done + c - 1, l, sync.err, seen);
+        // the row threads fetch line l + 1 (and the values of l + 2) next
+        const int need = min(l + 2, d.nx - 1);
+        if (AXIS == 2 && ok && gseen < need) ok = wait_for(gate, need, sync.err, gseen);
+        if (!ok) s_bad = 1;
       }
+      __syncwarp();
       const long long nb = col - sa + sb * l;
       for (int s = 1 + lane; s < n; s += 32) {
 #pragma unroll
         for (int e = 0; e < NC; ++e) s_nb[e * (n + 1) + s] = __ldcg(C.v[e] + nb + step * s);
       }
-      bar_sync(B_LINE, nt);
+      bar_sync(B_LINE + (l & 1), nt);
       if (s_bad) return;
-      bar_sync(B_RHS, nt);
+      bar_sync(B_RHS, nt - 32);
     }
     return;
   }
 
-  const int t = tid - 64;
+  if (warp == 2) {
+    bar_arrive(B_LINE + 1, nt);  // lines 1 and 2 wait for no announcement
+    if (nl > 1) bar_arrive(B_LINE, nt);
+    for (int l = 1; l <= nl; ++l) {
+      bar_sync(B_STORED + (l & 1), np + 32);
+      if (s_bad) return;
+      if (lane == 0) st_release(done + c, l);
+      __syncwarp();
+      if (l + 2 <= nl) bar_arrive(B_LINE + (l & 1), nt);
+    }
+    return;
+  }
+
+  const int t = tid - SW_ROLES;
   double own[R][NC], prev[R][NC], hiA[R][NC], hiB[R][NC], rr[R][NC];
   double cp0[R], cp1[R], cq0[R], cq1[R], am[R], g[R], bi[R], rib[R];
-  double end0[NC], end1[NC];  // rows 0 and n of the line (row thread 0)
+  double end0[NC], end1[NC], endb = 1.0;  // rows 0 and n of the line (row thread 0)
   // everything of line l that no line in flight changes; the line's own old
   // values go to `own` later (relax still needs line l - 1's)
   auto fetch = [&](int l, double (&o)[R][NC]) {
     const long long b0 = col + sb * l;
-    const int p = COLQ ? l : c, q = COLQ ? c : l;
 #pragma unroll
     for (int w = 0; w < R; ++w) {
       const int s = 1 + t + np * w;
       if (s < n) {
         const long long id = b0 + step * s;
-        const bool ce = central_at(AXIS == 0 ? s : p);
+        const bool ce = central_at(AXIS == 0 ? s : l);
         const double *fo = F.f[AXIS], *fp = F.f[P], *fq = F.f[Q];
         const double o0 = __ldg(fo + id), o1 = __ldg(fo + id + step);
         const double p0 = __ldg(fp + id), p1 = __ldg(fp + id + st[P]);
@@ -331,8 +393,8 @@ k_ad_sweep(Dims d, Met m, const int8_t *__restrict__ ib, const int8_t *__restric
           hiB[w][e] = __ldcg(C.v[e] + id + sb);
         }
         const AxisCoef xo = axis_coef(m.a[AXIS], s, o0, o1, half_dt, ce);
-        const AxisCoef xp = axis_coef(m.a[P], p, p0, p1, half_dt, ce);
-        const AxisCoef xq = axis_coef(m.a[Q], q, q0, q1, half_dt, ce);
+        const AxisCoef xp = axis_coef(m.a[P], l, p0, p1, half_dt, ce);
+        const AxisCoef xq = axis_coef(m.a[Q], c, q0, q1, half_dt, ce);
         am[w] = xo.lo * rib[w];
         g[w] = xo.hi * rib[w] * bi[w];
         cp0[w] = xp.lo; cp1[w] = xp.hi;
@@ -345,6 +407,7 @@ k_ad_sweep(Dims d, Met m, const int8_t *__restrict__ ib, const int8_t *__restric
         end0[e] = __ldcg(C.v[e] + b0);
         end1[e] = __ldcg(C.v[e] + b0 + step * n);
       }
+      endb = binv[b0 + step * n];
     }
   };
   fetch(1, own);
@@ -355,18 +418,19 @@ k_ad_sweep(Dims d, Met m, const int8_t *__restrict__ ib, const int8_t *__restric
     for (int e = 0; e < NC; ++e) prev[w][e] = s < n ? __ldcg(C.v[e] + col + step * s) : 0.0;
   }
   for (int l = 1; l <= nl; ++l) {
-    bar_sync(B_LINE, nt);
-    if (s_bad) return;
+    bar_sync(B_LINE + (l & 1), nt);
+    if (s_bad) {
+      bar_arrive(B_STORED + (l & 1), np + 32);
+      return;
+    }
 #pragma unroll
     for (int w = 0; w < R; ++w) {
       const int s = 1 + t + np * w;
       if (s < n) {
 #pragma unroll
         for (int e = 0; e < NC; ++e) {
-          const double lowA = s_nb[e * (n + 1) + s], lowB = prev[w][e];
-          const double vp0 = COLQ ? lowB : lowA, vp1 = COLQ ? hiB[w][e] : hiA[w][e];
-          const double vq0 = COLQ ? lowA : lowB, vq1 = COLQ ? hiA[w][e] : hiB[w][e];
-          const double rh = rr[w][e] - (vp0 * cp0[w] + vp1 * cp1[w] + vq0 * cq0[w] + vq1 * cq1[w]);
+          const double rh = rr[w][e] - (prev[w][e] * cp0[w] + hiB[w][e] * cp1[w] +
+                                        s_nb[e * (n + 1) + s] * cq0[w] + hiA[w][e] * cq1[w]);
           s_u[e * (n + 1) + s] = rh * rib[w] + own[w][e] * (1.0 - rib[w]);
         }
         s_ab[s] = make_double2(am[w], bi[w]);
@@ -379,12 +443,12 @@ k_ad_sweep(Dims d, Met m, const int8_t *__restrict__ ib, const int8_t *__restric
         s_u[e * (n + 1)] = end0[e];
         s_u[e * (n + 1) + n] = end1[e];
       }
-      s_ab[n] = make_double2(0.0, binv[col + sb * l + step * n]);
+      s_ab[n] = make_double2(0.0, endb);
     }
-    bar_sync(B_RHS, nt);
+    bar_sync(B_RHS, nt - 32);
     double nxt[R][NC];
     if (l < nl) fetch(l + 1, nxt);
-    bar_sync(B_SOL, nt - 32);
+    bar_sync(B_SOL, np + 32);
     const long long b0 = col + sb * l;
 #pragma unroll
     for (int w = 0; w < R; ++w) {
@@ -399,14 +463,34 @@ k_ad_sweep(Dims d, Met m, const int8_t *__restrict__ ib, const int8_t *__restric
         }
       }
     }
-    bar_arrive(B_STORED, nt - 32);
+    bar_arrive(B_STORED + (l & 1), np + 32);
   }
+}
+
+template <int R, int NC>
+__global__ void __launch_bounds__(SW_ROLES + SW_ROW_THREADS)
+k_ad_sweeps(Dims d, Met m, const int8_t *__restrict__ ib, const int8_t *__restrict__ gh, Comps<NC> C, Faces F,
+            double half_dt, double omega, const double *__restrict__ binv, long long nref, SweepSync sync) {
+  extern __shared__ __align__(16) double sw_smem[];
+  __shared__ int s_ticket, s_bad;
+  if (threadIdx.x == 0) {
+    s_ticket = atomicAdd(sync.ticket, 1);
+    s_bad = 0;
+  }
+  __syncthreads();
+  const int t = s_ticket, nk = d.nz - 1;
+  if (t < nk)
+    sweep_column<0, R, NC>(d, m, ib, gh, C, F, half_dt, omega, binv, sync, 1 + t, s_bad, sw_smem);
+  else if (t < 2 * nk)
+    sweep_column<1, R, NC>(d, m, ib, gh, C, F, half_dt, omega, binv + nref, sync, 1 + t - nk, s_bad, sw_smem);
+  else
+    sweep_column<2, R, NC>(d, m, ib, gh, C, F, half_dt, omega, binv + 2 * nref, sync, 1 + t - 2 * nk, s_bad, sw_smem);
 }
 
 // the lines of anti-diagonal `diag` along AXIS (0: x lines (j,k), j + k =
 // diag; 1: y lines (i,k); 2: z lines (i,j)), one thread per line, gam and
 // the forward values in the thread's slot of `scr` (2 (n+1) doubles): for
-// lines longer than k_ad_sweep's rows per thread hold
+// lines longer than k_ad_sweeps' rows per thread hold
 template <int AXIS>
 __global__ void k_ad_diag(Dims d, Met m, const int8_t *ib, const int8_t *gh, double *var, const double *r, Faces F,
                           double half_dt, double omega, const double *binv, int diag, double *scr) {
@@ -802,60 +886,32 @@ fg_status enqueue_outer_ghost(fg_case *c, const ad::Dims &d, double *u, double *
 
 namespace {
 
-// rows one thread of k_ad_sweep holds for lines of n cells' unknowns, 0 when
-// the line is too long for it
-int sweep_rows(int n) { return n <= 512 ? 1 : n <= 1024 ? 2 : n <= 2048 ? 4 : 0; }
+// rows one thread of k_ad_sweeps holds for lines of up to n cells, 0 when a
+// line is too long for it
+int sweep_rows(int n) { return n <= ad::SW_ROW_THREADS ? 1 : n <= 1024 ? 2 : n <= 2048 ? 4 : 0; }
 
-size_t sweep_smem(int n, int nc) { return (size_t)(n + 1) * (3 + 2 * nc) * sizeof(double); }
-
-template <int AXIS, bool COLQ, int R, int NC>
-cudaError_t launch_sweep(const ad::Dims &d, const ad::Met &m, const int8_t *ib, const int8_t *gh,
-                         const ad::Comps<NC> &C, const ad::Faces &F, double half_dt, double omega,
-                         const double *binv, int *sync, cudaStream_t s) {
-  const int nn[3] = {d.nx, d.ny, d.nz};
-  constexpr int P = AXIS == 0 ? 1 : 0, Q = AXIS == 2 ? 1 : 2;
-  const int n = nn[AXIS], cols = nn[COLQ ? Q : P] - 1;
+template <int R, int NC>
+cudaError_t launch_sweeps(const ad::Dims &d, const ad::Met &m, const int8_t *ib, const int8_t *gh,
+                          const ad::Comps<NC> &C, const ad::Faces &F, double half_dt, double omega,
+                          const double *binv, long long nref, const ad::SweepSync &sync, cudaStream_t s) {
+  const int n = std::max(d.nx, std::max(d.ny, d.nz));
   const int rows = ((n - 1 + R - 1) / R + 31) / 32 * 32;
-  const size_t sm = sweep_smem(n, NC);
-  auto kern = ad::k_ad_sweep<AXIS, COLQ, R, NC>;
+  const size_t sm = (size_t)(n + 1) * (3 + 2 * NC) * sizeof(double);
+  auto kern = ad::k_ad_sweeps<R, NC>;
   if (sm > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return e;
   }
-  kern<<<cols, 64 + rows, sm, s>>>(d, m, ib, gh, C, F, half_dt, omega, binv, sync + 1, sync + 2, sync);
+  kern<<<2 * (d.nz - 1) + d.ny - 1, ad::SW_ROLES + rows, sm, s>>>(d, m, ib, gh, C, F, half_dt, omega, binv, nref, sync);
   return cudaGetLastError();
 }
 
-template <int AXIS, bool COLQ, int NC>
-cudaError_t sweep_by_rows(const ad::Dims &d, const ad::Met &m, const int8_t *ib, const int8_t *gh,
-                          const ad::Comps<NC> &C, const ad::Faces &F, double half_dt, double omega,
-                          const double *binv, int *sync, cudaStream_t s) {
-  const int n = AXIS == 0 ? d.nx : AXIS == 1 ? d.ny : d.nz;
-  switch (sweep_rows(n)) {
-    case 1: return launch_sweep<AXIS, COLQ, 1, NC>(d, m, ib, gh, C, F, half_dt, omega, binv, sync, s);
-    case 2: return launch_sweep<AXIS, COLQ, 2, NC>(d, m, ib, gh, C, F, half_dt, omega, binv, sync, s);
-    default: return launch_sweep<AXIS, COLQ, 4, NC>(d, m, ib, gh, C, F, half_dt, omega, binv, sync, s);
-  }
-}
-
+// a sweep along AXIS one anti-diagonal at a time
 template <int AXIS, int NC>
-cudaError_t sweep_axis(const ad::Dims &d, const ad::Met &m, const int8_t *ib, const int8_t *gh,
-                       const ad::Comps<NC> &C, const ad::Faces &F, double half_dt, double omega, double *binv,
-                       int *sync, double *scr, cudaStream_t s, long long &launches) {
+void diag_sweep(const ad::Dims &d, const ad::Met &m, const int8_t *ib, const int8_t *gh, const ad::Comps<NC> &C,
+                const ad::Faces &F, double half_dt, double omega, const double *binv, double *scr, cudaStream_t s,
+                long long &launches) {
   const int np = AXIS == 0 ? d.ny - 1 : d.nx - 1, nq = AXIS == 2 ? d.ny - 1 : d.nz - 1;
-  const int n = AXIS == 0 ? d.nx : AXIS == 1 ? d.ny : d.nz;
-  const long long lines = (long long)np * nq;
-  ad::k_ad_factor<AXIS><<<(unsigned)((lines + 127) / 128), 128, 0, s>>>(d, m, ib, gh, F, half_dt, binv);
-  ++launches;
-  if (sweep_rows(n)) {
-    ++launches;
-    // y and z lines: a column holds all i of one plane, so a block's loads of
-    // neighbouring lines share sectors; x lines: the shorter of the two
-    // directions, which needs fewer blocks
-    if (AXIS != 0 || nq < np)
-      return sweep_by_rows<AXIS, true, NC>(d, m, ib, gh, C, F, half_dt, omega, binv, sync, s);
-    return sweep_by_rows<AXIS, false, NC>(d, m, ib, gh, C, F, half_dt, omega, binv, sync, s);
-  }
   for (int e = 0; e < NC; ++e)
     for (int diag = 2; diag <= np + nq; ++diag) {
       const int nl = std::min(np, diag - 1) - std::max(1, diag - nq) + 1;
@@ -863,7 +919,6 @@ cudaError_t sweep_axis(const ad::Dims &d, const ad::Met &m, const int8_t *ib, co
                                                                     binv, diag, scr);
       ++launches;
     }
-  return cudaGetLastError();
 }
 
 // one itsolv_ad pass of NC components: x, then y, then z sweeps
@@ -876,33 +931,49 @@ fg_status ad_sweeps(fg_case *c, const ad::Comps<NC> &C, const ad::Faces &F, cons
   if (st != FG_OK) return st;
   const size_t nref = (size_t)(c->nx + 2) * (c->ny + 2) * (c->nz + 2);
   const int8_t *ib = c->d_refmask, *gh = c->d_refmask + nref;
-  const double half_dt = prm->crank_nicolson ? 0.5 * prm->dt : 0.0;
-  const int nmax = std::max(c->nx, std::max(c->ny, c->nz));
-  // scratch: the pivots, per sweep an error flag, a ticket and the columns'
-  // progress, and for lines too long for k_ad_sweep one line per diagonal's
-  // thread
-  const size_t nsync = (size_t)nmax + 2;
+  const double half_dt = prm->crank_nicolson ? 0.5 * prm->dt : 0.0, om = prm->omega_ad;
+  const int nmax = std::max(c->nx, std::max(c->ny, c->nz)), rows = sweep_rows(nmax);
+  // scratch: the pivots of the three directions; an error flag, a ticket and
+  // the columns' progress; for lines too long for k_ad_sweeps one line per
+  // thread of a diagonal
+  const size_t nsync = 2 + 3 * (size_t)nmax;
   size_t nscr = 0;
-  if (!sweep_rows(nmax)) {
+  if (!rows) {
     const int lmax = std::max(std::min(c->ny, c->nz), std::max(std::min(c->nx, c->nz), std::min(c->nx, c->ny)));
     nscr = (size_t)lmax * 2 * (nmax + 1);
   }
   double *ws = nullptr;
-  FG_CUDA(fg::dev_alloc(&ws, (nref + nscr) * sizeof(double) + 3 * nsync * sizeof(int)));
-  double *binv = ws, *scr = ws + nref;
+  FG_CUDA(fg::dev_alloc(&ws, (3 * nref + nscr) * sizeof(double) + nsync * sizeof(int)));
+  double *binv = ws, *scr = ws + 3 * nref;
   int *sync = reinterpret_cast<int *>(scr + nscr);
+  const ad::SweepSync sy = {sync, sync + 1, {sync + 2, sync + 2 + nmax, sync + 2 + 2 * nmax}};
   cudaStream_t s = c->stream;
-  long long launches = 0;
-  cudaError_t e = cudaMemsetAsync(sync, 0, 3 * nsync * sizeof(int), s);
-  const double om = prm->omega_ad;
-  if (e == cudaSuccess) e = sweep_axis<0, NC>(d, m, ib, gh, C, F, half_dt, om, binv, sync, scr, s, launches);
-  if (e == cudaSuccess) e = sweep_axis<1, NC>(d, m, ib, gh, C, F, half_dt, om, binv, sync + nsync, scr, s, launches);
+  long long launches = 1;
+  cudaError_t e = cudaMemsetAsync(sync, 0, nsync * sizeof(int), s);
+  const size_t ft = 2 * sizeof(ad::FactorTile);
   if (e == cudaSuccess)
-    e = sweep_axis<2, NC>(d, m, ib, gh, C, F, half_dt, om, binv, sync + 2 * nsync, scr, s, launches);
+    e = cudaFuncSetAttribute(ad::k_ad_factor, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ft);
+  if (e == cudaSuccess) {
+    auto groups = [](int np, int nq) { return (np + ad::FT_LINES - 1) / ad::FT_LINES * nq; };
+    const int nb = std::max(groups(d.ny - 1, d.nz - 1), std::max(groups(d.nx - 1, d.nz - 1), groups(d.nx - 1, d.ny - 1)));
+    ad::k_ad_factor<<<dim3(nb, 3), 32 + ad::FT_WORK, ft, s>>>(d, m, ib, gh, F, half_dt, binv, (long long)nref);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess && rows) {
+    launches += 1;
+    const long long nr = (long long)nref;
+    e = rows == 1   ? launch_sweeps<1, NC>(d, m, ib, gh, C, F, half_dt, om, binv, nr, sy, s)
+        : rows == 2 ? launch_sweeps<2, NC>(d, m, ib, gh, C, F, half_dt, om, binv, nr, sy, s)
+                    : launch_sweeps<4, NC>(d, m, ib, gh, C, F, half_dt, om, binv, nr, sy, s);
+  } else if (e == cudaSuccess) {
+    diag_sweep<0, NC>(d, m, ib, gh, C, F, half_dt, om, binv, scr, s, launches);
+    diag_sweep<1, NC>(d, m, ib, gh, C, F, half_dt, om, binv + nref, scr, s, launches);
+    diag_sweep<2, NC>(d, m, ib, gh, C, F, half_dt, om, binv + 2 * nref, scr, s, launches);
+    e = cudaGetLastError();
+  }
   note_launches(launches);
-  int gave_up[3] = {0, 0, 0};
-  for (int a = 0; a < 3 && e == cudaSuccess; ++a)
-    e = cudaMemcpyAsync(&gave_up[a], sync + a * nsync, sizeof(int), cudaMemcpyDeviceToHost, s);
+  int gave_up = 0;
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&gave_up, sync, sizeof(int), cudaMemcpyDeviceToHost, s);
   const cudaError_t es = cudaStreamSynchronize(s);
   if (e == cudaSuccess) e = es;
   {
@@ -913,7 +984,7 @@ fg_status ad_sweeps(fg_case *c, const ad::Comps<NC> &C, const ad::Faces &F, cons
     set_last_error(cudaGetErrorString(e), __FILE__, __LINE__);
     return FG_CUDA_ERROR;
   }
-  return gave_up[0] || gave_up[1] || gave_up[2] ? FG_TIMEOUT : FG_OK;
+  return gave_up ? FG_TIMEOUT : FG_OK;
 }
 
 // calc_residual_ad of NC components: resm[c] and loc[3 c ..]
