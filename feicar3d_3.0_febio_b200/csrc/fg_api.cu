@@ -531,6 +531,7 @@ struct fg_batch {
   struct Tune {
     int var[kMaxLevels][3] = {};
     double us[kMaxLevels][3] = {};
+    bool fixed[kMaxLevels] = {};  // families chosen by hand
     std::vector<int> key;
     bool nu_tuned = false;
     double solve_ms[4] = {0, 0, 0, 0};
@@ -538,13 +539,10 @@ struct fg_batch {
     int cnu1 = 0, cnu2 = 0, cfrom = 2;
     double solve_ms_coarse[2] = {0.0, 0.0};
   } tune;
-  // the small levels (k_small_cycle): from level small_L down, one block per
-  // problem whose hierarchy reaches small_L (small_L == maxdepth: none)
-  int small_L = 0;
-  int n_small = 0, small_maxgn = 0;
-  std::vector<SmallProb> h_small;
-  SmallProb *d_small = nullptr;
-  DevLevel *d_small_levs = nullptr;
+  // the levels one kernel cycles through (k_cycle): from level cyc.Lc down,
+  // for the problems whose hierarchy reaches it (cyc.Lc == maxdepth: none)
+  Cycle cyc;
+  std::vector<CycleProb> h_cyc;
   // level 0 over all problems
   DevLevel *d_lev0 = nullptr;
   int *d_off0 = nullptr, *d_offf0 = nullptr, *d_offq0 = nullptr;
@@ -639,9 +637,9 @@ static void free_batch_tables(fg_batch *b) {
     s = fg_batch::LevelSet();
   }
   fg::dev_free(b->d_lev0); fg::dev_free(b->d_off0); fg::dev_free(b->d_offf0); fg::dev_free(b->d_offq0);
-  fg::dev_free(b->d_small); fg::dev_free(b->d_small_levs);
-  b->d_small = nullptr; b->d_small_levs = nullptr; b->n_small = 0; b->small_maxgn = 0;
-  b->h_small.clear();
+  fg::dev_free(b->cyc.probs); fg::dev_free(b->cyc.levs);
+  b->cyc = Cycle();
+  b->h_cyc.clear();
   fg::dev_free(b->d_rprob); fg::dev_free(b->d_rtgt); fg::dev_free(b->d_rcell); fg::dev_free(b->d_rw);
   fg::dev_free(b->d_rc0); fg::dev_free(b->d_rd); fg::dev_free(b->d_rf); fg::dev_free(b->d_tmp);
   fg::dev_free(b->d_norm); fg::dev_free(b->d_part);
@@ -733,19 +731,23 @@ static fg_status upload_geometry(fg_batch *b) {
     FG_CUDA(cudaMemcpy(s.d_gidx, gi.data(), gi.size() * sizeof(int *), cudaMemcpyHostToDevice));
     FG_CUDA(cudaMemcpy(s.d_gn, gn.data(), gn.size() * sizeof(int), cudaMemcpyHostToDevice));
   }
-  if (b->n_small > 0) {
-    b->small_maxgn = 0;
-    int q = 0;
+  if (b->cyc.n > 0) {
+    b->cyc.maxgn = 0;
+    int q = 0, row = 0;
     for (const fg_case *c : b->cases) {
-      if (c->nlev <= b->small_L) continue;
-      SmallProb &sp = b->h_small[q++];
-      sp.G = c->d_G;
-      sp.gidx = c->d_gidx;
-      sp.gn = (int)c->gidx.size();
-      b->small_maxgn = std::max(b->small_maxgn, sp.gn);
+      const int rows = (int)c->rows.tgt.size();
+      if (c->nlev > b->cyc.Lc) {
+        CycleProb &cp = b->h_cyc[q++];
+        cp.G = c->d_G;
+        cp.gidx = c->d_gidx;
+        cp.gn = (int)c->gidx.size();
+        cp.r0 = row;
+        cp.r1 = row + rows;
+        b->cyc.maxgn = std::max(b->cyc.maxgn, cp.gn);
+      }
+      row += rows;
     }
-    FG_CUDA(cudaMemcpy(b->d_small, b->h_small.data(), b->h_small.size() * sizeof(SmallProb),
-                       cudaMemcpyHostToDevice));
+    FG_CUDA(cudaMemcpy(b->cyc.probs, b->h_cyc.data(), b->h_cyc.size() * sizeof(CycleProb), cudaMemcpyHostToDevice));
   }
   // rows (dead rows then ghost rows of each problem, problems in order)
   std::vector<int> prob;
@@ -806,10 +808,81 @@ static fg_status upload_geometry(fg_batch *b) {
 static std::vector<int> tune_key(const fg_batch *b);
 static fg_status rebuild_line_offsets(fg_batch *b, int L, int axis);
 
+// Which levels one kernel cycles through (k_cycle).  Up to CL_MAXPROBS
+// problems get a cluster each and start at the first level all of whose
+// fields have at most CL_MAXCELLS cells, level 0 included: a phase of the
+// kernel then takes 1.5-3 us where a launch takes about 5.  More problems
+// fill the GPU through the launches, each of which serves all of them; they
+// get one block each, from the first level below level 0 whose hierarchy
+// fits its shared memory.
+static fg_status build_cycle(fg_batch *b) {
+  Cycle &cy = b->cyc;
+  cy = Cycle();
+  cy.Lc = b->maxdepth;
+  const int ts = b->cfg.precision == FG_PREC_MIXED ? 4 : 8;
+  const bool cluster = (int)b->cases.size() <= CL_MAXPROBS;
+  for (int L = cluster ? 0 : 1; L < b->maxdepth; ++L) {
+    bool fits = true;
+    size_t most = 0, need = 0;
+    std::vector<CycleProb> probs;
+    std::vector<DevLevel> lv;
+    for (auto *c : b->cases) {
+      if (c->nlev <= L) continue;
+      CycleProb q{};
+      q.l0 = (int)lv.size();
+      q.nl = c->nlev - L;
+      // the first level kept in shared memory (never level 0: it has rows)
+      int ns = 0;
+      while (cluster && ns < q.nl - 1 &&
+             (L + ns == 0 || (long long)c->lev[L + ns].nx * c->lev[L + ns].ny * c->lev[L + ns].nz > SC_MAXCELLS))
+        ++ns;
+      q.ns = ns;
+      size_t sum = 0, coarsest = 0;
+      for (int l = 0; l < q.nl; ++l) {
+        const HLevel &H = c->lev[L + l];
+        const long long cells = (long long)H.nx * H.ny * H.nz;
+        sum += k::cycle_bytes(H.nx, H.ny, H.nz, ts, l >= ns);
+        coarsest = (size_t)cells * sizeof(double);
+        fits = fits && H.nx <= SC_MAXN && H.ny <= SC_MAXN && H.nz <= SC_MAXN && cells <= CL_MAXCELLS;
+        lv.push_back(H.dl);
+      }
+      fits = fits && L + ns > 0 && sum + coarsest <= SC_MAXBYTES;
+      most = std::max(most, sum);
+      need = std::max(need, sum + coarsest);
+      probs.push_back(q);
+    }
+    if (!fits || probs.empty()) continue;
+    cy.n = (int)probs.size();
+    cy.Lc = L;
+    cy.bytes = most;
+    if (cluster)
+      for (int size : {16, 8}) {
+        const int room = ts == 4 ? k::cycle_clusters<float>(size, need) : k::cycle_clusters<double>(size, need);
+        if (room >= cy.n) { cy.size = size; break; }
+        if (size == 8 && room > 0) cy.size = size;
+      }
+    b->h_cyc = probs;
+    FG_CUDA(run_launch_set_alloc((void **)&cy.levs, lv));
+    FG_CUDA(fg::dev_alloc(&cy.probs, probs.size() * sizeof(CycleProb)));
+    break;
+  }
+  return FG_OK;
+}
+
+// the first level of that kernel: later where a level's line kernels were
+// chosen by hand (fg_*_set_tuning)
+static int cycle_start(const fg_batch *b) {
+  int L = b->cyc.Lc;
+  for (int l = L; l < b->maxdepth; ++l)
+    if (b->tune.fixed[l]) L = l + 1;
+  return std::min(L, b->maxdepth);
+}
+
 static fg_status build_batch(fg_batch *b) {
   if (b->built && b->sig == batch_signature(b)) return upload_geometry(b);
   free_batch_tables(b);
   const int np = (int)b->cases.size();
+  fg_status st0;
   b->maxdepth = 0;
   for (auto *c : b->cases) b->maxdepth = std::max(b->maxdepth, c->nlev);
   for (int L = 0; L < b->maxdepth; ++L) {
@@ -861,33 +934,7 @@ static fg_status build_batch(fg_batch *b) {
       FG_CUDA(fg::dev_alloc(&s.d_gn, s.C.size() * sizeof(int)));
     }
   }
-  // the small levels: the first level below level 0 from which every level
-  // of every problem that reaches it fits one block's sweeps
-  b->small_L = b->maxdepth;
-  for (int L = 1; L < b->maxdepth; ++L) {
-    bool fits = true;
-    for (auto *c : b->cases)
-      for (int l = L; l < c->nlev && fits; ++l) {
-        const HLevel &H = c->lev[l];
-        fits = (long long)H.nx * H.ny * H.nz <= SC_MAXCELLS && H.nx <= SC_MAXN && H.ny <= SC_MAXN &&
-               H.nz <= SC_MAXN;
-      }
-    if (fits) { b->small_L = L; break; }
-  }
-  if (b->small_L < b->maxdepth) {
-    std::vector<DevLevel> lv;
-    for (auto *c : b->cases) {
-      if (c->nlev <= b->small_L) continue;
-      SmallProb q{};
-      q.l0 = (int)lv.size();
-      q.nl = c->nlev - b->small_L;
-      for (int l = b->small_L; l < c->nlev; ++l) lv.push_back(c->lev[l].dl);
-      b->h_small.push_back(q);
-    }
-    FG_CUDA(run_launch_set_alloc((void **)&b->d_small_levs, lv));
-    FG_CUDA(fg::dev_alloc(&b->d_small, b->h_small.size() * sizeof(SmallProb)));
-    b->n_small = (int)b->h_small.size();
-  }
+  if ((st0 = build_cycle(b)) != FG_OK) return st0;
   // level 0 over all problems
   {
     std::vector<DevLevel> v0;
@@ -1022,7 +1069,7 @@ template <typename T>
 static fg_status vcycle(fg_batch *b, cudaStream_t s) {
   const int corr = (b->krylov || sizeof(T) == 4) ? 1 : 0;
   fg_status st;
-  const int Ls = std::min(b->maxdepth, b->small_L);  // levels from Ls down: one block per problem
+  const int Ls = cycle_start(b);  // levels from Ls down: one kernel
   for (int L = 0; L < Ls; ++L) {
     auto &ls = b->ls[L];
     if (!ls.S.empty()) {
@@ -1031,7 +1078,6 @@ static fg_status vcycle(fg_batch *b, cudaStream_t s) {
       const size_t e0 = prof_begin(b, s);
       FG_K(k::residual_q<T>(ls.quads, s));
       FG_K(k::restrict_to<T>(ls.next, ls.d_levS, s));
-      FG_K(k::zero_x<T>(ls.next, s));
       prof_end(b, e0, FG_PROF_TRANSFER, 0.0, s);
     }
     if (!ls.C.empty()) {
@@ -1042,8 +1088,12 @@ static fg_status vcycle(fg_batch *b, cudaStream_t s) {
   }
   if (Ls < b->maxdepth) {
     const size_t e0 = prof_begin(b, s);
-    FG_K(k::small_cycle<T>(b->n_small, b->d_small, b->d_small_levs, b->small_maxgn, nu_pre(b, Ls),
-                           nu_post(b, Ls), b->cfg.omega, s));
+    CycleSteps nu;
+    for (int L = 0; L < kMaxLevels; ++L) {
+      nu.pre[L] = nu_pre(b, L);
+      nu.post[L] = nu_post(b, L);
+    }
+    FG_K(k::cycle<T>(b->cyc, Ls - b->cyc.Lc, nu, b->cfg.omega, b->rows, corr, b->d_tmp, s));
     prof_end(b, e0, FG_PROF_LINE_COARSE, 0.0, s);
   }
   for (int L = std::min(b->maxdepth - 2, Ls - 1); L >= 0; --L) {
@@ -1071,7 +1121,7 @@ static std::vector<char> vcycle_params(const fg_batch *b) {
   put(&b->rows, sizeof(DevRows));
   put(&b->d_tmp, sizeof(b->d_tmp));
   for (int L = 0; L < b->maxdepth; ++L) put(&b->ls[L].maxgn, sizeof(int));
-  put(&b->small_maxgn, sizeof(int));
+  put(&b->cyc.maxgn, sizeof(int));
   return v;
 }
 
@@ -1774,8 +1824,8 @@ static void drop_graphs(fg_batch *b) {
 // Times every kernel family that can take each level set's lines (two
 // colours, three repetitions after a warm-up, CUDA events) and keeps the
 // fastest.  The sweeps run on the levels' current arrays, which every
-// solve overwrites before reading.  Levels the one-block small cycle
-// takes have no line launches and are skipped.
+// solve overwrites before reading.  Levels that one kernel cycles through
+// have no line launches and are skipped.
 template <typename T>
 static fg_status tune_lines(fg_batch *b) {
   cudaStream_t s = b->stream;
@@ -1784,7 +1834,7 @@ static fg_status tune_lines(fg_batch *b) {
   FG_CUDA(cudaEventCreate(&e0));
   FG_CUDA(cudaEventCreate(&e1));
   fg_status st = FG_OK;
-  const int Ls = std::min(b->maxdepth, b->small_L);
+  const int Ls = cycle_start(b);
   for (int L = 0; L < Ls && st == FG_OK; ++L) {
     auto &ls = b->ls[L];
     if (ls.S.empty()) continue;
@@ -2865,7 +2915,7 @@ fg_status fg_batch_get_tuning(const fg_batch *b, fg_tuning *out) {
     for (int a = 0; a < 3; ++a) {
       const auto &ls = b->ls[L];
       const int maxn = a == 0 ? ls.maxnx : a == 1 ? ls.maxny : ls.maxnz;
-      const bool lines = !ls.S.empty() && L < std::min(b->maxdepth, b->small_L);
+      const bool lines = !ls.S.empty() && L < cycle_start(b);
       out->line_variant[L][a] = lines ? k::line_variant(a, maxn, b->tune.var[L][a]) : 0;
       out->line_us[L][a] = b->tune.us[L][a];
     }
@@ -2901,10 +2951,12 @@ fg_status fg_batch_set_tuning(fg_batch *b, const fg_tuning *t) {
   }
   for (int L = 0; L < b->maxdepth && L < FG_TUNE_MAXLEVELS; ++L) {
     if (b->ls[L].S.empty()) continue;
+    b->tune.fixed[L] = false;
     for (int a = 0; a < 3; ++a) {
       const int v = t->line_variant[L][a];
       if (v < 0 || v > (a == 0 ? k::LV_NX : k::LV_NYZ)) return FG_BAD_INPUT;
       b->tune.var[L][a] = v;  // 0 or a family that cannot take the lines: the default
+      b->tune.fixed[L] = b->tune.fixed[L] || v != 0;
       b->tune.us[L][a] = 0.0;
       fg_status s = rebuild_line_offsets(b, L, a);
       if (s != FG_OK) return s;

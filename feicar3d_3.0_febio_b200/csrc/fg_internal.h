@@ -250,17 +250,34 @@ enum : int {
   KPH_UPDATE = 4      // P += sum y_i Z_i over jlast columns
 };
 
-// A problem's small levels that one block cycles through (k_small_cycle):
-// levels [l0, l0 + nl) of a packed DevLevel table, the last one the
+// The levels of a batch that one kernel cycles through, a cluster of blocks
+// per problem (k_cycle): hierarchy levels Lc down to each problem's
+// coarsest.  A problem's levels are [l0, l0 + nl) of a packed DevLevel
+// table; the first ns of them are worked on by the whole cluster in global
+// memory, the rest by its first block in shared memory, the last one the
 // coarsest, with its generalised inverse G (gn x gn) over the cells gidx.
-constexpr int SC_THREADS = 256;           // threads of the block
-constexpr int SC_MAXN = 32;               // longest line of such a level
-constexpr long long SC_MAXCELLS = 2048;   // most cells of any such level
-struct SmallProb {
-  int l0, nl;
+// Rows [r0, r1) of the batch's interpolation rows are the problem's.
+constexpr int SC_MAXN = 128;                // longest line (4 rows per lane of a warp)
+constexpr size_t SC_MAXBYTES = 200 * 1024;  // shared memory of a block
+constexpr long long SC_MAXCELLS = 2048;   // a cluster's largest level in shared memory
+constexpr long long CL_MAXCELLS = 16384;     // a cluster's largest level in global memory
+constexpr int CL_MAXPROBS = 16;             // most problems that get a cluster of more than one block
+struct CycleProb {
+  int l0, nl, ns;
   const double *G;
   const int *gidx;
-  int gn;
+  int gn, r0, r1;
+};
+struct CycleSteps {
+  int pre[kMaxLevels], post[kMaxLevels];  // smoothing steps per hierarchy level
+};
+struct Cycle {
+  int n = 0, Lc = 0;        // problems, first hierarchy level
+  int size = 1;             // blocks per cluster
+  size_t bytes = 0;         // shared memory of the largest problem's levels
+  int maxgn = 0;
+  CycleProb *probs = nullptr;
+  DevLevel *levs = nullptr;
 };
 
 // kernel launchers (fg_mg.cu)
@@ -317,10 +334,16 @@ template <typename T>
 cudaError_t residual_q(const Launch &quads, cudaStream_t s);
 template <typename T>
 cudaError_t zero_x(const Launch &L, cudaStream_t s);
-// the V-cycle of each problem's small levels, one block per problem
+// shared memory a level of nx x ny x nz cells takes in cycle(), with or
+// without its fields
+size_t cycle_bytes(int nx, int ny, int nz, int tsize, bool fields);
+// clusters of `size` blocks with `bytes` of shared memory each that run at once
 template <typename T>
-cudaError_t small_cycle(int nprob, const SmallProb *probs, const DevLevel *levs, int maxgn, int nu1,
-                        int nu2, double omega, cudaStream_t s);
+int cycle_clusters(int size, size_t bytes);
+// the V-cycle from hierarchy level c.Lc + first down
+template <typename T>
+cudaError_t cycle(const Cycle &c, int first, const CycleSteps &nu, double omega, const DevRows &R, int corr,
+                  double *tmp, cudaStream_t s);
 template <typename T>
 cudaError_t rows_relax(const DevRows &R, const DevLevel *lev0, int correction_form,
                        double *tmp, cudaStream_t s);

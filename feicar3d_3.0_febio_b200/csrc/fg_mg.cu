@@ -2060,27 +2060,7 @@ cudaError_t residual_q(const Launch &Lq, cudaStream_t s) {
 // ------------------------------------------------------- restriction
 // coarse rhs = volume-weighted mean of the children's residuals on active
 // coarse cells (the sum of the children's finite-volume equations)
-// the restriction into coarse cell (I,J,K)
-template <typename T>
-__device__ __forceinline__ void restrict_cell(const DevLevel &C, const DevLevel &F, int I, int J, int K) {
-  auto rc = PrecOf<T>::rhs(C);
-  auto rf = PrecOf<T>::res(F);
-  const long long id = I + C.sy * J + C.sz * K;
-  if (!(glob(C.mask)[id] & 64)) { rc[id] = T(0); return; }
-  double s = 0.0, v = 0.0;
-  for (int k = glob(C.clz)[K]; k <= glob(C.chz)[K]; ++k)
-    for (int j = glob(C.cly)[J]; j <= glob(C.chy)[J]; ++j) {
-      const double wyz = glob(F.wy)[j] * glob(F.wz)[k];
-      const long long rb = F.sy * j + F.sz * k;
-      for (int i = glob(C.clx)[I]; i <= glob(C.chx)[I]; ++i) {
-        const double w = glob(F.wx)[i] * wyz;
-        s += w * (double)rf[rb + i];
-        v += w;
-      }
-    }
-  rc[id] = (T)(s / v);
-}
-
+// (and the coarse unknown starts from zero)
 template <typename T>
 __global__ void __launch_bounds__(CELL_BLOCK)
 k_restrict(const int *FG_RESTRICT off, int nent, const DevLevel *FG_RESTRICT coarse, const DevLevel *FG_RESTRICT fine) {
@@ -2088,14 +2068,15 @@ k_restrict(const int *FG_RESTRICT off, int nent, const DevLevel *FG_RESTRICT coa
   const DevLevel &C = coarse[p];
   const DevLevel &F = fine[p];
   const int lb = blockIdx.x - off[p];
-  // the arithmetic of restrict_cell with the thread's i-children and their
-  // widths kept over the block's CELL_ROWS rows (at most two children per
+  // the thread's i-children and their widths are kept over the block's
+  // CELL_ROWS rows (at most two children per
   // axis: cl = 2I-1, ch = min(2I, n))
   const int tpr = (C.nx + CELL_BLOCK - 1) / CELL_BLOCK;
   const int rb = lb / tpr;
   const int I = 1 + (lb - rb * tpr) * CELL_BLOCK + (int)threadIdx.x;
   if (I > C.nx) return;
   dptr<T> FG_RESTRICT rc = PrecOf<T>::rhs(C);
+  dptr<T> FG_RESTRICT xc = PrecOf<T>::x(C);
   dptr<const T> FG_RESTRICT rf = PrecOf<T>::res(F);
   dptr<const uint8_t> FG_RESTRICT cm = C.mask;
   const long long csy = C.sy, csz = C.sz, fsy = F.sy, fsz = F.sz;
@@ -2104,8 +2085,7 @@ k_restrict(const int *FG_RESTRICT off, int nent, const DevLevel *FG_RESTRICT coa
   const double wx0 = glob(F.wx)[il], wx1 = glob(F.wx)[ih];
   // every child's value is loaded before the coarse mask decides (the
   // children exist for every coarse cell), so the rows' loads are in
-  // flight together; the sums take the valid children in the order of
-  // restrict_cell
+  // flight together; the sums take the valid children in k, j, i order
   const int row0 = rb * CELL_ROWS;
   int J = 1 + row0 % cny, K = 1 + row0 / cny;
 #pragma unroll
@@ -2119,6 +2099,7 @@ k_restrict(const int *FG_RESTRICT off, int nent, const DevLevel *FG_RESTRICT coa
                     b11 = fsy * jh + fsz * kh;
     const T f[8] = {rf[b00 + il], rf[b00 + ih], rf[b10 + il], rf[b10 + ih],
                     rf[b01 + il], rf[b01 + ih], rf[b11 + il], rf[b11 + ih]};
+    xc[id] = T(0);
     if (!(cm[id] & 64)) { rc[id] = T(0); continue; }
     double s = 0.0, v = 0.0;
 #pragma unroll
@@ -2421,7 +2402,22 @@ cudaError_t rows_residual(const DevRows &R, const DevLevel *lev0, double *maxabs
 
 // ---------------------------------------------------- coarsest solve
 // x = G rhs over the active cells of a problem's coarsest level, G the
-// generalised inverse of the coarsest operator (FP64)
+// generalised inverse of the coarsest operator (FP64).  One warp per row
+// of G, its lanes along the row: the row is read once, coalesced (a thread
+// per row read it by single dependent loads: 147 us for 125 cells).
+template <typename V, typename S>
+__device__ __forceinline__ void dense_rows(const double *G, int n, const V &rhs, const S &store) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  for (int r = warp; r < n; r += nw) {
+    const double *gr = G + (size_t)r * n;
+    double acc = 0.0;
+    for (int c = lane; c < n; c += 32) acc += gr[c] * rhs(c);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+    if (lane == 0) store(r, acc);
+  }
+}
+
 template <typename T>
 __global__ void __launch_bounds__(256)
 k_coarsest(const DevLevel *FG_RESTRICT levs, const double *const *G, const int *const *gidx, const int *gn) {
@@ -2430,17 +2426,11 @@ k_coarsest(const DevLevel *FG_RESTRICT levs, const double *const *G, const int *
   const DevLevel &L = levs[p];
   const int n = gn[p];
   const int *idx = gidx[p];
-  const double *g = G[p];
   auto rhs = PrecOf<T>::rhs(L);
   auto x = PrecOf<T>::x(L);
   for (int c = threadIdx.x; c < n; c += blockDim.x) sr[c] = (double)rhs[idx[c]];
   __syncthreads();
-  for (int r = threadIdx.x; r < n; r += blockDim.x) {
-    double acc = 0.0;
-    const double *gr = g + (size_t)r * n;
-    for (int c = 0; c < n; ++c) acc += gr[c] * sr[c];
-    x[idx[r]] = (T)acc;
-  }
+  dense_rows(G[p], n, [&](int c) { return sr[c]; }, [&](int r, double v) { x[idx[r]] = (T)v; });
 }
 
 template <typename T>
@@ -2455,157 +2445,696 @@ cudaError_t coarsest_solve(int nprob, const DevLevel *lev, const double *const *
   return cudaGetLastError();
 }
 
-// ------------------------------------------------ small levels, one block
-// The V-cycle from the first level whose every line has at most SC_MAXN
-// cells and every level at most SC_MAXCELLS cells down to the coarsest, as
-// one block per problem.  On such levels each launch of the level-by-level
-// cycle (six line sweeps per smoothing step, residual, restriction,
-// prolongation, coarsest solve) is a few microseconds of fixed cost for a
-// few hundred cells; here they are phases of one kernel separated by
-// __syncthreads, on data that stays in the SM's L1.  The line sweeps keep
-// the line kernels' colours ((transverse index sum) & 1), rows, held rows,
-// couplings and omega, one line per thread solved by the Thomas algorithm;
-// residual, restriction, prolongation and coarsest solve use the
-// arithmetic of their kernels.
+// ------------------------------------------------ many levels, one kernel
+// The V-cycle from a level down to the coarsest as one kernel, a cluster of
+// blocks per problem.  On such levels each launch of the level-by-level
+// cycle (six line sweeps per smoothing step, rows, residual, restriction,
+// prolongation, coarsest solve) is some 5 us of fixed cost for a few
+// thousand cells; here they are phases between barriers.
+//
+// The upper levels (C.ns of them) stay in global memory (L2): the lines of a
+// colour are spread over the whole cluster, a cluster barrier ends each
+// phase.  The levels below run on the cluster's first block alone, with
+// unknowns, right-hand sides, masks and couplings in shared memory and
+// __syncthreads between the phases.  The line sweeps keep the line kernels'
+// colours ((transverse index sum) & 1), rows, held rows, couplings and
+// omega; a line is SC_M rows per lane, its chunk equations solved by cyclic
+// reduction across the lanes.  Residual (formed by the restriction as it
+// reads), restriction, prolongation, ghost/dead rows and coarsest solve use
+// the arithmetic of their kernels.
+//
+// Bound by the phases' latency: a colour of a level takes 0.7 us in shared
+// memory (1024 cells), 2.3-3 us in global memory on 16 blocks (8192 cells)
+// and 5 us (65536 cells), which is what a launch takes there.  Measured (B200,
+// solves to 1e-11): 32x16x16 cells mixed 5.11 ms by launches with one thread
+// per line on the small levels, 2.75 ms; 128x64x64 FP64 5.82 and 4.58 ms.
+constexpr int SC_M = 4;         // rows per lane
+constexpr int SC_THREADS = 512; // threads of a block: what the FP64 form's registers allow
+constexpr int SC_NW = SC_THREADS / 32;
+
+// A level: its 1-D arrays in shared memory (byte offsets, so that every
+// access is known to be a shared-memory one), and where its fields are.
 template <typename T>
-__device__ void sc_sweep(const DevLevel &L, int axis, int color, T omega) {
-  const int n = axis == 0 ? L.nx : axis == 1 ? L.ny : L.nz;
-  const int n1 = axis == 0 ? L.ny : L.nx;  // first transverse extent
-  const int n2 = axis == 2 ? L.ny : L.nz;  // second transverse extent
-  const long long ls = axis == 0 ? 1 : axis == 1 ? L.sy : L.sz;
-  auto x = PrecOf<T>::x(L);
-  auto rhs = PrecOf<T>::rhs(L);
-  auto am_ = axis == 0 ? L.amx : axis == 1 ? L.amy : L.amz;
-  auto ap_ = axis == 0 ? L.apx : axis == 1 ? L.apy : L.apz;
-  for (int line = threadIdx.x; line < n1 * n2; line += blockDim.x) {
-    const int a = 1 + line % n1, b = 1 + line / n1;  // transverse indices
-    if (((a + b) & 1) != color) continue;
-    const int i = axis == 0 ? 1 : a, j = axis == 0 ? a : axis == 1 ? 1 : b, k = axis == 2 ? 1 : b;
-    const LineCoef lc = line_coef(L, axis, i, j, k);
-    const bool iso_line = lc.tdir == 0.0 && !lc.dirm && !lc.dirp;
-    const long long base = (long long)i + L.sy * j + L.sz * k - ls;  // row r at base + ls (r + 1)
-    T cpa[SC_MAXN], dpa[SC_MAXN];
-    T cprev = T(0), dprev = T(0);
-    for (int r = 0; r < n; ++r) {
-      const long long id = base + ls * (r + 1);
-      const uint8_t m8 = glob(L.mask)[id];
-      T aa = T(0), bb = T(1), cc = T(0), dd;
-      const bool held = !(m8 & 64) || (((m8 & 63) == 0) && iso_line);
-      if (held) {
-        dd = x[id];
-      } else {
-        T acc = rhs[id];
+struct ScLevel {
+  int n[3];
+  int c[6];          // couplings to the lower and upper neighbour per axis and index (T)
+  int c64[6];        // the same in FP64 (the diagonals are summed in FP64)
+  int w[3];          // cell widths (FP64)
+  int ch[3];         // first child | last child << 16 in the next finer level
+  int pl[3], pw[3];  // prolongation: lower coarse cell, weight of the upper one
+  unsigned magic[3]; // ceil(2^32 / d) of the lines per colour and second index, per axis
+  int n1h[3];        // d: ceil(n1 / 2)
+  unsigned bc;       // bit q: Dirichlet boundary at face q
+  // fields in shared memory: offsets and pitches; element (i, j, k), 0-based,
+  // at i + sy j + sz k; x has a guard of sz elements on either side, so that
+  // the neighbour loads need no bounds
+  int x, rhs, mk, sy, sz;
+  // fields in global memory: strides; cell (0, 0, 0) at g0
+  dptr<T> gx, grhs;
+  dptr<const uint8_t> gmk;
+  int gsy, gsz, g0;
+};
+extern __shared__ __align__(16) unsigned char sc_smem[];
+template <typename V> __device__ __forceinline__ V *sc_at(int off) { return reinterpret_cast<V *>(sc_smem + off); }
+
+__host__ __device__ inline int sc_sy(int nx) { return nx | 1; }  // odd pitches: lanes along y or z on distinct banks
+__host__ __device__ inline int sc_sz(int nx, int ny) { return (sc_sy(nx) * ny) | 1; }
+__host__ __device__ inline int sc_round(int b) { return (b + 15) & ~15; }
+// lays a level's arrays out from byte `at` on, its fields too when they are
+// kept in shared memory; returns the end
+template <typename T>
+__host__ __device__ inline int sc_place(int nx, int ny, int nz, bool fields, int at, ScLevel<T> &S) {
+  constexpr int ts = (int)sizeof(T);
+  S.n[0] = nx; S.n[1] = ny; S.n[2] = nz;
+  for (int a = 0; a < 3; ++a) {
+    S.w[a] = at; at += 8 * S.n[a];
+    S.c64[2 * a] = at; S.c64[2 * a + 1] = at + 8 * S.n[a]; at += 16 * S.n[a];
+  }
+  for (int a = 0; a < 3; ++a) {
+    S.c[2 * a] = at; S.c[2 * a + 1] = at + S.n[a] * ts; S.pw[a] = at + 2 * S.n[a] * ts;
+    at += 3 * S.n[a] * ts;
+  }
+  for (int a = 0; a < 3; ++a) { S.ch[a] = at; S.pl[a] = at + 4 * S.n[a]; at += 8 * S.n[a]; }
+  at = sc_round(at);
+  S.sy = sc_sy(nx); S.sz = sc_sz(nx, ny);
+  if (!fields) return at;
+  const int cells = S.sz * nz;
+  S.x = at + S.sz * ts; at = sc_round(at + (cells + 2 * S.sz) * ts);
+  S.rhs = at; at = sc_round(at + cells * ts);
+  S.mk = at;
+  return sc_round(at + cells);
+}
+size_t cycle_bytes(int nx, int ny, int nz, int tsize, bool fields) {
+  ScLevel<float> f;
+  ScLevel<double> d;
+  return (size_t)(tsize == 4 ? sc_place<float>(nx, ny, nz, fields, 0, f) : sc_place<double>(nx, ny, nz, fields, 0, d));
+}
+
+// The fields of a level in shared memory, used by one block
+template <typename T>
+struct ScFields {
+  static constexpr bool CLUSTER = false;
+  T *xp, *rp;
+  uint8_t *mp;
+  int st[3];
+  __device__ __forceinline__ explicit ScFields(const ScLevel<T> &S)
+      : xp(sc_at<T>(S.x)), rp(sc_at<T>(S.rhs)), mp(sc_at<uint8_t>(S.mk)), st{1, S.sy, S.sz} {}
+  __device__ __forceinline__ int id(int i, int j, int k) const { return i + st[1] * j + st[2] * k; }
+  __device__ __forceinline__ T x(int e) const { return xp[e]; }
+  __device__ __forceinline__ void set_x(int e, T v) const { xp[e] = v; }
+  __device__ __forceinline__ T rhs(int e) const { return rp[e]; }
+  __device__ __forceinline__ void set_rhs(int e, T v) const { rp[e] = v; }
+  __device__ __forceinline__ unsigned mk(int e) const { return mp[e]; }
+  // rows r0 .. r0 + 3 of a line (past its end: any value)
+  template <int AXIS>
+  __device__ __forceinline__ void x4(int e0, int r0, int n, T (&v)[SC_M]) const {
 #pragma unroll
-        for (int t = 0; t < 4; ++t)
-          if ((m8 >> lc.qt[t]) & 1) acc -= (T)lc.tq[t] * x[id + lc.to[t]];
-        dd = acc;
-        row_coef<T>(m8, r, n, am_[1 + r], ap_[1 + r], lc, aa, bb, cc);
+    for (int u = 0; u < SC_M; ++u) v[u] = xp[e0 + st[AXIS] * min(r0 + u, n - 1)];
+  }
+  template <int AXIS>
+  __device__ __forceinline__ void rhs4(int e0, int r0, int n, T (&v)[SC_M]) const {
+#pragma unroll
+    for (int u = 0; u < SC_M; ++u) v[u] = rp[e0 + st[AXIS] * min(r0 + u, n - 1)];
+  }
+  template <int AXIS>
+  __device__ __forceinline__ void mk4(int e0, int r0, int n, unsigned (&v)[SC_M]) const {
+#pragma unroll
+    for (int u = 0; u < SC_M; ++u) v[u] = mp[e0 + st[AXIS] * min(r0 + u, n - 1)];
+  }
+};
+
+// The fields of a level in global memory, used by the whole cluster: what
+// other blocks write is read past L1
+template <typename T>
+struct GlFields {
+  static constexpr bool CLUSTER = true;
+  dptr<T> xp, rp;
+  dptr<const uint8_t> mp;
+  int st[3], g0;
+  __device__ __forceinline__ explicit GlFields(const ScLevel<T> &S)
+      : xp(S.gx), rp(S.grhs), mp(S.gmk), st{1, S.gsy, S.gsz}, g0(S.g0) {}
+  __device__ __forceinline__ int id(int i, int j, int k) const { return g0 + i + st[1] * j + st[2] * k; }
+  __device__ __forceinline__ T x(int e) const { return __ldcg(&xp[e]); }
+  __device__ __forceinline__ void set_x(int e, T v) const { xp[e] = v; }
+  __device__ __forceinline__ T rhs(int e) const { return __ldcg(&rp[e]); }
+  __device__ __forceinline__ void set_rhs(int e, T v) const { rp[e] = v; }
+  __device__ __forceinline__ unsigned mk(int e) const { return mp[e]; }
+  template <int AXIS>
+  __device__ __forceinline__ void run(const dptr<T> &p, int e0, int r0, int n, T (&v)[SC_M]) const {
+#ifndef FG_CHECKED
+    if constexpr (AXIS == 0) {  // cell 1 + 4 q of a row is 16-byte aligned, rows are padded
+      const uint4 *src = reinterpret_cast<const uint4 *>(&p[e0 + min(r0, (n - 1) / SC_M * SC_M)]);
+      constexpr int N = SC_M * (int)sizeof(T) / 16;
+#pragma unroll
+      for (int q = 0; q < N; ++q) {
+        const uint4 t = __ldcg(src + q);
+        memcpy(&v[q * (16 / (int)sizeof(T))], &t, 16);
       }
-      const T den = bb - aa * cprev;
-      cprev = cc / den;
-      dprev = (dd - aa * dprev) / den;
-      cpa[r] = cprev;
-      dpa[r] = dprev;
-    }
-    T xn = T(0);
-    for (int r = n - 1; r >= 0; --r) {
-      xn = dpa[r] - cpa[r] * xn;
-      const long long id = base + ls * (r + 1);
-      T v = xn;
-      if (omega != T(1)) v = x[id] + omega * (v - x[id]);
-      x[id] = v;
+    } else
+#endif
+    {
+#pragma unroll
+      for (int u = 0; u < SC_M; ++u) v[u] = __ldcg(&p[e0 + st[AXIS] * min(r0 + u, n - 1)]);
     }
   }
-  __syncthreads();
+  template <int AXIS>
+  __device__ __forceinline__ void x4(int e0, int r0, int n, T (&v)[SC_M]) const {
+    // a row's transverse neighbours start at the same alignment
+    run<AXIS>(xp, e0, r0, n, v);
+  }
+  template <int AXIS>
+  __device__ __forceinline__ void rhs4(int e0, int r0, int n, T (&v)[SC_M]) const { run<AXIS>(rp, e0, r0, n, v); }
+  template <int AXIS>
+  __device__ __forceinline__ void mk4(int e0, int r0, int n, unsigned (&v)[SC_M]) const {
+#pragma unroll
+    for (int u = 0; u < SC_M; ++u) v[u] = mp[e0 + st[AXIS] * min(r0 + u, n - 1)];
+  }
+};
+
+// the warps that share a level's work, and the barrier that ends a phase
+struct ScTeam {
+  int rank, size;  // block of the cluster
+  template <bool CLUSTER>
+  __device__ __forceinline__ int warp0() const { return CLUSTER ? (int)(threadIdx.x >> 5) * size + rank : (int)(threadIdx.x >> 5); }
+  template <bool CLUSTER>
+  __device__ __forceinline__ int warps() const { return CLUSTER ? SC_NW * size : SC_NW; }
+  template <bool CLUSTER>
+  __device__ __forceinline__ void sync() const {
+    if (CLUSTER) {
+      asm volatile("barrier.cluster.arrive;\n\tbarrier.cluster.wait;" ::: "memory");
+    } else {
+      __syncthreads();
+    }
+  }
+};
+
+// Dirichlet faces of the domain at cell (i, j, k)
+template <typename T>
+__device__ __forceinline__ unsigned sc_dirichlet(const ScLevel<T> &S, int i, int j, int k) {
+  const unsigned at = (i == 0 ? 1u : 0u) | (i == S.n[0] - 1 ? 2u : 0u) | (j == 0 ? 4u : 0u) |
+                      (j == S.n[1] - 1 ? 8u : 0u) | (k == 0 ? 16u : 0u) | (k == S.n[2] - 1 ? 32u : 0u);
+  return at & S.bc;
 }
 
+// minus the sum over the kept faces of their couplings (doubled on Dirichlet
+// boundary faces) at the indices at[axis]
 template <typename T>
-__device__ void sc_smooth(const DevLevel &L, int nu, T omega) {
-  for (int s_ = 0; s_ < nu; ++s_)
-    for (int axis = 0; axis < 3; ++axis)
-      for (int color = 0; color < 2; ++color) sc_sweep<T>(L, axis, color, omega);
+__device__ __forceinline__ double sc_diag(const ScLevel<T> &S, unsigned mk, unsigned dir, const int (&at)[3]) {
+  double d = 0.0;
+#pragma unroll
+  for (int q = 0; q < 6; ++q) {
+    const double c = sc_at<double>(S.c64[q])[at[q >> 1]];
+    d -= (mk >> q) & 1 ? c : (dir >> q) & 1 ? 2.0 * c : 0.0;
+  }
+  return d;
 }
 
-// residual of fine level F restricted into coarse level C, coarse x = 0
+// one colour of the lines along AXIS
+template <int AXIS, typename T, class V>
+__device__ __forceinline__ void sc_sweep(const ScLevel<T> &S, const V &v, const ScTeam &team, int color, T omega) {
+  constexpr int A0 = AXIS == 0 ? 1 : 0, A1 = AXIS == 2 ? 1 : 2;
+  constexpr int M = SC_M;
+  const int n = S.n[AXIS], n1 = S.n[A0], n2 = S.n[A1];
+  const int ls = v.st[AXIS], s1 = v.st[A0], s2 = v.st[A1];
+  const int sh = n <= M ? 0 : 32 - __clz((n - 1) / M);  // lanes per line: 2^sh >= n / M
+  const int W = 1 << sh;
+  const int n1h = S.n1h[AXIS], lines = n1h * n2;
+  const unsigned magic = S.magic[AXIS], bc = S.bc;
+  const int lane = threadIdx.x & 31;
+  const int step = 32 * team.template warps<V::CLUSTER>();
+  const T *const cm = sc_at<T>(S.c[2 * AXIS]), *const cp = sc_at<T>(S.c[2 * AXIS + 1]);
+  const double *const dm = sc_at<double>(S.c64[2 * AXIS]), *const dp = sc_at<double>(S.c64[2 * AXIS + 1]);
+  for (int t0 = 32 * team.template warp0<V::CLUSTER>(); t0 < lines << sh; t0 += step) {
+    const int t = t0 + lane, sl = t & (W - 1), q = t >> sh;
+    int b = n1h == 1 ? q : (int)__umulhi((unsigned)q, magic);
+    int a = 2 * (q - b * n1h) + ((b ^ color) & 1);
+    const bool ok = q < lines && a < n1;
+    if (!ok) { a = 0; b = 0; }
+    const int r0 = sl * M;
+    const int id0 = v.id(0, 0, 0) + s1 * a + s2 * b;
+    // every load of the chunk before its first use (rows past the line end
+    // repeat the last one)
+    unsigned mk[M];
+    T nb[4][M], d[M], xo[M];
+    v.template mk4<AXIS>(id0, r0, n, mk);
+    v.template x4<AXIS>(id0, r0, n, xo);
+    v.template rhs4<AXIS>(id0, r0, n, d);
+    v.template x4<AXIS>(id0 - s1, r0, n, nb[0]);
+    v.template x4<AXIS>(id0 + s1, r0, n, nb[1]);
+    v.template x4<AXIS>(id0 - s2, r0, n, nb[2]);
+    v.template x4<AXIS>(id0 + s2, r0, n, nb[3]);
+    const T tq[4] = {sc_at<T>(S.c[2 * A0])[a], sc_at<T>(S.c[2 * A0 + 1])[a], sc_at<T>(S.c[2 * A1])[b],
+                     sc_at<T>(S.c[2 * A1 + 1])[b]};
+    const double tsum = -(sc_at<double>(S.c64[2 * A0])[a] + sc_at<double>(S.c64[2 * A0 + 1])[a] +
+                          sc_at<double>(S.c64[2 * A1])[b] + sc_at<double>(S.c64[2 * A1 + 1])[b]);
+    // Dirichlet faces of the whole line
+    const unsigned dt = bc & (((a == 0) << (2 * A0)) | ((a == n1 - 1) << (2 * A0 + 1)) | ((b == 0) << (2 * A1)) |
+                              ((b == n2 - 1) << (2 * A1 + 1)));
+    const bool iso = dt == 0 && !((bc >> (2 * AXIS)) & 3);
+    T lo[M], di[M], up[M];
+#pragma unroll
+    for (int u = 0; u < M; ++u) {
+      const int r = r0 + u, rc = min(r, n - 1);
+      const bool in = ok && r < n;
+      const bool act = in && (mk[u] & 64) && !((mk[u] & 63) == 0 && iso);
+      T dv;
+      if ((mk[u] & 63) == 63) {  // every face coupled
+        dv = (T)(tsum - (dm[rc] + dp[rc]));
+      } else {
+        int at[3];
+        at[AXIS] = rc; at[A0] = a; at[A1] = b;
+        const unsigned de = ((r == 0) << (2 * AXIS)) | ((r == n - 1) << (2 * AXIS + 1));
+        dv = (T)sc_diag(S, mk[u], dt | (de & bc), at);
+      }
+      T acc = d[u];
+      acc -= (mk[u] >> (2 * A0)) & 1 ? tq[0] * nb[0][u] : T(0);
+      acc -= (mk[u] >> (2 * A0 + 1)) & 1 ? tq[1] * nb[1][u] : T(0);
+      acc -= (mk[u] >> (2 * A1)) & 1 ? tq[2] * nb[2][u] : T(0);
+      acc -= (mk[u] >> (2 * A1 + 1)) & 1 ? tq[3] * nb[3][u] : T(0);
+      d[u] = act ? acc : in ? xo[u] : T(0);
+      lo[u] = act && ((mk[u] >> (2 * AXIS)) & 1) ? cm[rc] : T(0);
+      up[u] = act && ((mk[u] >> (2 * AXIS + 1)) & 1) ? cp[rc] : T(0);
+      di[u] = act ? dv : T(1);
+    }
+    // chunk elimination (the partition method of chunk_eliminate): lo and up
+    // become the couplings to the chunk's first and last row
+    {
+      const T rr = rcp_nr(di[1]);
+      lo[1] *= rr; up[1] *= rr; d[1] *= rr;
+    }
+#pragma unroll
+    for (int u = 2; u < M; ++u) {
+      const T rr = rcp_nr(di[u] - lo[u] * up[u - 1]);
+      d[u] = (d[u] - lo[u] * d[u - 1]) * rr;
+      lo[u] = -lo[u] * lo[u - 1] * rr;
+      up[u] *= rr;
+    }
+    const T aL = lo[M - 1], cL = up[M - 1], dL = d[M - 1];
+    T pa = T(0), pb = T(-1), pd = T(0);
+#pragma unroll
+    for (int u = M - 2; u >= 1; --u) {
+      const T nd = d[u] - up[u] * pd, na = lo[u] - up[u] * pa, nv = -up[u] * pb;
+      lo[u] = na; up[u] = nv; d[u] = nd;
+      pa = na; pb = nv; pd = nd;
+    }
+    const T aF = lo[0], bF = di[0] - up[0] * pa, cF = -up[0] * pb, dF = d[0] - up[0] * pd;
+    T aLp = __shfl_up_sync(0xffffffffu, aL, 1), cLp = __shfl_up_sync(0xffffffffu, cL, 1),
+      dLp = __shfl_up_sync(0xffffffffu, dL, 1);
+    if (sl == 0) { aLp = T(0); cLp = T(0); dLp = T(0); }
+    T A = -aF * aLp, B = bF - aF * cLp - cF * aL, Cc = -cF * cL, D = dF - aF * dLp - cF * dL;
+    for (int o = 1; o < W; o <<= 1) {
+      // unit diagonals: each lane divides its own equation
+      const T ib = rcp_nr(B);
+      A *= ib; Cc *= ib; D *= ib;
+      T la = __shfl_up_sync(0xffffffffu, A, o), lc = __shfl_up_sync(0xffffffffu, Cc, o);
+      T ld = __shfl_up_sync(0xffffffffu, D, o);
+      T ra = __shfl_down_sync(0xffffffffu, A, o), rc = __shfl_down_sync(0xffffffffu, Cc, o);
+      T rd = __shfl_down_sync(0xffffffffu, D, o);
+      if (sl < o) { la = T(0); lc = T(0); ld = T(0); }
+      if (sl + o >= W) { ra = T(0); rc = T(0); rd = T(0); }
+      B = T(1) - A * lc - Cc * ra;
+      D = D - A * ld - Cc * rd;
+      A = -A * la;
+      Cc = -Cc * rc;
+    }
+    const T xF = D * rcp_nr(B);
+    const T xFn = __shfl_down_sync(0xffffffffu, xF, 1);
+    const T xL = dL - aL * xF - cL * (sl + 1 < W ? xFn : T(0));
+#pragma unroll
+    for (int u = 0; u < M; ++u) {
+      T val = u == 0 ? xF : u == M - 1 ? xL : d[u] - lo[u] * xF - up[u] * xL;
+      if (omega != T(1)) val = xo[u] + omega * (val - xo[u]);
+      if (ok && r0 + u < n) v.set_x(id0 + ls * (r0 + u), val);
+    }
+  }
+  team.template sync<V::CLUSTER>();
+}
+
+// a Jacobi pass of the problem's ghost and dead rows on the finest level
+// (k_rows and k_rows_scatter): all values first, then all targets
+struct ScRows {
+  int r0, r1, corr;
+};
 template <typename T>
-__device__ void sc_down(const DevLevel &F, const DevLevel &C) {
-  auto x = PrecOf<T>::x(F);
-  auto rhs = PrecOf<T>::rhs(F);
-  auto res = PrecOf<T>::res(F);
-  const int nf = F.nx * F.ny * F.nz;
-  for (int c = threadIdx.x; c < nf; c += blockDim.x) {
-    const int i = 1 + c % F.nx, j = 1 + (c / F.nx) % F.ny, k = 1 + c / (F.nx * F.ny);
-    const long long id = i + F.sy * j + F.sz * k;
-    const uint8_t mk = glob(F.mask)[id];
-    T r = T(0);
-    if (mk & 64) r = rhs[id] - apply_row<T>(F, id, i, j, k, mk, x);
-    res[id] = r;
+__device__ void sc_rows(const DevRows &R, const ScRows &rg, const ScLevel<T> &S, const ScTeam &team, double *tmp) {
+  if (rg.r1 <= rg.r0) return;
+  constexpr int KEEP = 2;  // rows per thread kept in registers
+  const int gt = 32 * team.warp0<true>() + (int)(threadIdx.x & 31), nt = 32 * team.warps<true>();
+  const bool keep = rg.r1 - rg.r0 <= KEEP * nt;
+  const long long sy = S.gsy, sz = S.gsz;
+  const long long o[8] = {0, sy, sy + 1, 1, sz, sz + sy, sz + sy + 1, sz + 1};
+  T mine[KEEP];
+  int u = 0;
+  for (int r = rg.r0 + gt; r < rg.r1; r += nt, ++u) {
+    const long long b = R.cell[r];
+    T xv[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) xv[q] = __ldcg(&S.gx[b + o[q]]);
+    double acc = 0.0;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) acc += R.w[8 * r + q] * (double)xv[q];
+    const double c = !rg.corr ? R.c0[r] : sizeof(T) == 4 ? (double)R.rf[r] : R.rd[r];
+    if (!keep) tmp[r] = acc + c;
+    else if (u == 0) mine[0] = (T)(acc + c);
+    else mine[KEEP - 1] = (T)(acc + c);
+  }
+  team.sync<true>();
+  u = 0;
+  for (int r = rg.r0 + gt; r < rg.r1; r += nt, ++u)
+    S.gx[R.tgt[r]] = !keep ? (T)tmp[r] : u == 0 ? mine[0] : mine[KEEP - 1];
+  team.sync<true>();
+}
+
+template <typename T, class V>
+__device__ void sc_smooth(const ScLevel<T> &S, const ScTeam &team, int nu, T omega, const DevRows *R, const ScRows &rg,
+                          double *tmp) {
+  const V v(S);
+  for (int s_ = 0; s_ < nu; ++s_) {
+#pragma unroll 1
+    for (int color = 0; color < 2; ++color) sc_sweep<0>(S, v, team, color, omega);
+    if (V::CLUSTER && R) sc_rows<T>(*R, rg, S, team, tmp);
+#pragma unroll 1
+    for (int color = 0; color < 2; ++color) sc_sweep<1>(S, v, team, color, omega);
+    if (V::CLUSTER && R) sc_rows<T>(*R, rg, S, team, tmp);
+#pragma unroll 1
+    for (int color = 0; color < 2; ++color) sc_sweep<2>(S, v, team, color, omega);
+    if (V::CLUSTER && R) sc_rows<T>(*R, rg, S, team, tmp);
+  }
+}
+
+// the residual of the fine level's active cells, in the arithmetic of
+// apply_vals, restricted into the coarse level as k_restrict does (at most
+// two children per axis, 2 I and 2 I + 1 where the axis is coarsened).  A
+// lane takes a fine column i and the up to four (j, k) of a coarse cell; the
+// two columns of a coarse cell meet by a shuffle.
+template <typename T, class VF, class VC>
+__device__ void sc_down(const ScLevel<T> &F, const ScLevel<T> &C, const ScTeam &team) {
+  const VF f(F);
+  const VC c(C);
+  const int lane = threadIdx.x & 31;
+  const bool pair = C.n[0] < F.n[0];
+  const int nwx = (F.n[0] + 31) >> 5;
+  for (int e = team.template warp0<VF::CLUSTER>(); e < nwx * C.n[1] * C.n[2]; e += team.template warps<VF::CLUSTER>()) {
+    const int row = e / nwx, i0 = 32 * (e - row * nwx) + lane;
+    const int K = row / C.n[1], J = row - K * C.n[1];
+    const int jc = sc_at<int>(C.ch[1])[J], kc = sc_at<int>(C.ch[2])[K];
+    const int i = min(i0, F.n[0] - 1);
+    const T cx0 = sc_at<T>(F.c[0])[i], cx1 = sc_at<T>(F.c[1])[i];
+    const double wx = sc_at<double>(F.w[0])[i];
+    double s = 0.0, w = 0.0;
+    unsigned mk[4];
+    T xv[4][7], rh[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {  // absent children repeat a present one
+      const int id = f.id(i, q & 1 ? jc >> 16 : jc & 0xffff, q & 2 ? kc >> 16 : kc & 0xffff);
+      mk[q] = f.mk(id);
+      rh[q] = f.rhs(id);
+      xv[q][6] = f.x(id);
+#pragma unroll
+      for (int a = 0; a < 3; ++a) { xv[q][2 * a] = f.x(id - f.st[a]); xv[q][2 * a + 1] = f.x(id + f.st[a]); }
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int j = q & 1 ? jc >> 16 : jc & 0xffff, k = q & 2 ? kc >> 16 : kc & 0xffff;
+      const bool have = !((q & 1) && (jc >> 16) == (jc & 0xffff)) && !((q & 2) && (kc >> 16) == (kc & 0xffff));
+      const T cf[6] = {cx0, cx1, sc_at<T>(F.c[2])[j], sc_at<T>(F.c[3])[j], sc_at<T>(F.c[4])[k], sc_at<T>(F.c[5])[k]};
+      T acc = T(0);
+#pragma unroll
+      for (int g = 0; g < 6; ++g) acc += (mk[q] >> g) & 1 ? cf[g] * xv[q][g] : T(0);
+      const int at[3] = {i, j, k};
+      const T dg = (T)sc_diag(F, mk[q], sc_dirichlet(F, i, j, k), at);
+      const T r = mk[q] & 64 ? rh[q] - (acc + dg * xv[q][6]) : T(0);
+      const double wt = have && i0 < F.n[0] ? wx * (sc_at<double>(F.w[1])[j] * sc_at<double>(F.w[2])[k]) : 0.0;
+      s += wt * (double)r;
+      w += wt;
+    }
+    const double s2 = __shfl_down_sync(0xffffffffu, s, 1), w2 = __shfl_down_sync(0xffffffffu, w, 1);
+    if (pair) { s += s2; w += w2; }
+    if (i0 < F.n[0] && !(pair && (i0 & 1))) {
+      const int id = c.id(pair ? i0 >> 1 : i0, J, K);
+      c.set_rhs(id, c.mk(id) & 64 ? (T)(s / w) : T(0));
+      c.set_x(id, T(0));
+    }
+  }
+  team.template sync<VF::CLUSTER>();
+}
+
+// prolong_cell
+template <typename T, class VF, class VC>
+__device__ void sc_up(const ScLevel<T> &F, const ScLevel<T> &C, const ScTeam &team) {
+  const VF f(F);
+  const VC c(C);
+  const int lane = threadIdx.x & 31;
+  const int nwx = (F.n[0] + 31) >> 5;
+  for (int e = team.template warp0<VF::CLUSTER>(); e < nwx * F.n[1] * F.n[2]; e += team.template warps<VF::CLUSTER>()) {
+    const int row = e / nwx, i = 32 * (e - row * nwx) + lane;
+    const int k = row / F.n[1], j = row - k * F.n[1];
+    if (i >= F.n[0]) continue;
+    const int j0 = sc_at<int>(F.pl[1])[j], k0 = sc_at<int>(F.pl[2])[k], i0 = sc_at<int>(F.pl[0])[i];
+    const int j1 = min(j0 + 1, C.n[1] - 1), k1 = min(k0 + 1, C.n[2] - 1), i1 = min(i0 + 1, C.n[0] - 1);
+    const int id = f.id(i, j, k);
+    const unsigned mk = f.mk(id);
+    const T xf = f.x(id);
+    T xv[8];
+    unsigned cm[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int cid = c.id(q & 1 ? i1 : i0, q & 2 ? j1 : j0, q & 4 ? k1 : k0);
+      xv[q] = c.x(cid);
+      cm[q] = c.mk(cid);
+    }
+    const T wy1 = sc_at<T>(F.pw[1])[j], wz1 = sc_at<T>(F.pw[2])[k], wx1 = sc_at<T>(F.pw[0])[i];
+    const T wx[2] = {T(1) - wx1, wx1};
+    const T wyz[4] = {(T(1) - wy1) * (T(1) - wz1), wy1 * (T(1) - wz1), (T(1) - wy1) * wz1, wy1 * wz1};
+    T s = T(0), ws = T(0);
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const T w = wx[q & 1] * wyz[q >> 1];
+      const T act = (cm[q] & 64) ? w : T(0);
+      s += act * xv[q];
+      ws += act;
+    }
+    if ((mk & 128) && ws > T(1e-12)) f.set_x(id, xf + s / ws);
+  }
+  team.template sync<VF::CLUSTER>();
+}
+
+// the levels [s0, nl) of a problem, kept in shared memory by one block: from
+// the right-hand side of level s0 to its unknown
+template <typename T>
+__device__ void sc_small(const CycleProb &P, const DevLevel *FG_RESTRICT levs, const ScLevel<T> *S, int s0,
+                         const CycleSteps &nu, int Lc, T omega) {
+  const ScTeam team = {0, 1};
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const ScRows none = {0, 0, 0};
+  constexpr int ROWS = 4;  // rows loaded together
+  for (int l = s0; l < P.nl; ++l) {
+    const ScLevel<T> &D = S[l];
+    const int ny = D.n[1], rows = ny * D.n[2], nx = D.n[0];
+    const GlFields<T> g(D);
+    const ScFields<T> d(D);
+    for (int row0 = warp; row0 < rows; row0 += SC_NW * ROWS) {
+      for (int i = lane; i < nx; i += 32) {
+        unsigned mk[ROWS];
+        T rv[ROWS];
+#pragma unroll
+        for (int u = 0; u < ROWS; ++u) {
+          const int row = min(row0 + SC_NW * u, rows - 1), k = row / ny, j = row - k * ny;
+          const int id = g.id(i, j, k);
+          mk[u] = g.mk(id);
+          rv[u] = l == s0 ? g.rhs(id) : T(0);
+        }
+#pragma unroll
+        for (int u = 0; u < ROWS; ++u) {
+          const int row = row0 + SC_NW * u;
+          if (row >= rows) continue;
+          const int k = row / ny, j = row - k * ny, id = d.id(i, j, k);
+          d.mp[id] = (uint8_t)mk[u];
+          if (l == s0) {
+            d.rp[id] = rv[u];
+            d.xp[id] = T(0);
+          }
+        }
+      }
+    }
   }
   __syncthreads();
-  auto xc = PrecOf<T>::x(C);
-  const int ncc = C.nx * C.ny * C.nz;
-  for (int c = threadIdx.x; c < ncc; c += blockDim.x) {
-    const int I = 1 + c % C.nx, J = 1 + (c / C.nx) % C.ny, K = 1 + c / (C.nx * C.ny);
-    restrict_cell<T>(C, F, I, J, K);
-    xc[I + C.sy * J + C.sz * K] = T(0);
-  }
-  __syncthreads();
-}
-
-template <typename T>
-__device__ void sc_up(const DevLevel &F, const DevLevel &C) {
-  const int nf = F.nx * F.ny * F.nz;
-  for (int c = threadIdx.x; c < nf; c += blockDim.x) {
-    const int i = 1 + c % F.nx, j = 1 + (c / F.nx) % F.ny, k = 1 + c / (F.nx * F.ny);
-    prolong_cell<T>(F, C, i, j, k);
-  }
-  __syncthreads();
-}
-
-template <typename T>
-__global__ void __launch_bounds__(SC_THREADS)
-k_small_cycle(const SmallProb *probs, const DevLevel *FG_RESTRICT levs, int nu1, int nu2, T omega) {
-  extern __shared__ double sc_sr[];  // coarsest right-hand side (gn values)
-  const SmallProb P = probs[blockIdx.x];
-  for (int l = 0; l < P.nl - 1; ++l) {
-    sc_smooth<T>(levs[P.l0 + l], nu1, omega);
-    sc_down<T>(levs[P.l0 + l], levs[P.l0 + l + 1]);
+  for (int l = s0; l < P.nl - 1; ++l) {
+    sc_smooth<T, ScFields<T>>(S[l], team, nu.pre[Lc + l], omega, nullptr, none, nullptr);
+    sc_down<T, ScFields<T>, ScFields<T>>(S[l], S[l + 1], team);
   }
   {
-    const DevLevel &L = levs[P.l0 + P.nl - 1];
-    auto rhs = PrecOf<T>::rhs(L);
-    auto x = PrecOf<T>::x(L);
-    for (int c = threadIdx.x; c < P.gn; c += blockDim.x) sc_sr[c] = (double)rhs[P.gidx[c]];
+    double *sr = sc_at<double>(0);  // coarsest right-hand side (gn values)
+    const ScLevel<T> &D = S[P.nl - 1];
+    const ScFields<T> d(D);
+    // gidx: element indices of the device layout
+    auto at = [&](int c) {
+      const int g = P.gidx[c];
+      const int k = g / D.gsz, r = g - k * D.gsz, j = r / D.gsy, i = r - j * D.gsy;
+      return d.id(i - 1, j - 1, k - 1);
+    };
+    for (int c = tid; c < P.gn; c += SC_THREADS) sr[c] = (double)d.rp[at(c)];
     __syncthreads();
-    for (int r = threadIdx.x; r < P.gn; r += blockDim.x) {
-      double acc = 0.0;
-      const double *gr = P.G + (size_t)r * P.gn;
-      for (int c = 0; c < P.gn; ++c) acc += gr[c] * sc_sr[c];
-      x[P.gidx[r]] = (T)acc;
-    }
+    dense_rows(P.G, P.gn, [&](int c) { return sr[c]; }, [&](int r, double v) { d.xp[at(r)] = (T)v; });
     __syncthreads();
   }
-  for (int l = P.nl - 2; l >= 0; --l) {
-    sc_up<T>(levs[P.l0 + l], levs[P.l0 + l + 1]);
-    sc_smooth<T>(levs[P.l0 + l], nu2, omega);
+  for (int l = P.nl - 2; l >= s0; --l) {
+    sc_up<T, ScFields<T>, ScFields<T>>(S[l], S[l + 1], team);
+    sc_smooth<T, ScFields<T>>(S[l], team, nu.post[Lc + l], omega, nullptr, none, nullptr);
+  }
+  const ScLevel<T> &D = S[s0];
+  const GlFields<T> g(D);
+  const ScFields<T> d(D);
+  for (int row = warp; row < D.n[1] * D.n[2]; row += SC_NW) {
+    const int k = row / D.n[1], j = row - k * D.n[1];
+    for (int i = lane; i < D.n[0]; i += 32) g.set_x(g.id(i, j, k), d.xp[d.id(i, j, k)]);
+  }
+}
+
+// first: the first level of the problem's table to run (Lc + first in the
+// hierarchy); the ghost and dead rows belong to hierarchy level 0
+template <typename T>
+__global__ void __launch_bounds__(SC_THREADS)
+k_cycle(const CycleProb *probs, const DevLevel *FG_RESTRICT levs, int Lc, int first, int maxgn, CycleSteps nu, T omega,
+        DevRows R, int corr, double *tmp) {
+  __shared__ __align__(16) unsigned char s_lev[kMaxLevels * sizeof(ScLevel<T>)];
+  ScLevel<T> *const S = reinterpret_cast<ScLevel<T> *>(s_lev);
+  ScTeam team;
+  {
+    unsigned r, n;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(n));
+    team.rank = (int)r;
+    team.size = (int)n;
+  }
+  const CycleProb P = probs[blockIdx.x / team.size];
+  if (first >= P.nl) return;  // this hierarchy ends above (its coarsest level has a launch of its own)
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int s0 = max(P.ns, first);  // first level in shared memory
+  if (warp == 0) {                  // lane l lays out level l
+    int mine = 0, at = sc_round(maxgn * (int)sizeof(double));
+    if (lane < P.nl) {
+      const DevLevel &L = levs[P.l0 + lane];
+      ScLevel<T> &D = S[lane];
+      mine = sc_place<T>(L.nx, L.ny, L.nz, lane >= s0, 0, D);
+      D.bc = 0;
+      for (int f = 0; f < 6; ++f) D.bc |= (L.bc[f] ? 1u : 0u) << f;
+      for (int a = 0; a < 3; ++a) {
+        D.n1h[a] = (D.n[a == 0 ? 1 : 0] + 1) >> 1;
+        D.magic[a] = D.n1h[a] > 1 ? magic_u32(D.n1h[a]) : 0u;
+      }
+      D.gx = PrecOf<T>::x(L);
+      D.grhs = PrecOf<T>::rhs(L);
+      D.gmk = L.mask;
+      D.gsy = (int)L.sy; D.gsz = (int)L.sz; D.g0 = 1 + (int)L.sy + (int)L.sz;
+    }
+    for (int l = 0; l < P.nl; ++l) {
+      const int b = __shfl_sync(0xffffffffu, mine, l);
+      if (l < lane) at += b;
+    }
+    if (lane < P.nl) {
+      ScLevel<T> &D = S[lane];
+      D.x += at; D.rhs += at; D.mk += at;
+      for (int f = 0; f < 6; ++f) { D.c[f] += at; D.c64[f] += at; }
+      for (int a = 0; a < 3; ++a) { D.w[a] += at; D.ch[a] += at; D.pl[a] += at; D.pw[a] += at; }
+    }
+  }
+  __syncthreads();
+  // the axis arrays, a warp per level and axis
+  for (int e = warp; e < 3 * P.nl; e += SC_NW) {
+    const int l = e / 3, a = e - 3 * l;
+    const DevLevel &L = levs[P.l0 + l];
+    const ScLevel<T> &D = S[l];
+    auto am = a == 0 ? L.amx : a == 1 ? L.amy : L.amz;
+    auto ap = a == 0 ? L.apx : a == 1 ? L.apy : L.apz;
+    auto w = a == 0 ? L.wx : a == 1 ? L.wy : L.wz;
+    auto cl = a == 0 ? L.clx : a == 1 ? L.cly : L.clz;
+    auto chh = a == 0 ? L.chx : a == 1 ? L.chy : L.chz;
+    auto pl = a == 0 ? L.plx : a == 1 ? L.ply : L.plz;
+    auto pw = a == 0 ? L.pwx : a == 1 ? L.pwy : L.pwz;
+    const bool child = l > 0, up = l + 1 < P.nl;  // links inside these levels
+    for (int i = lane; i < D.n[a]; i += 32) {
+      const double vm = glob(am)[1 + i], vp = glob(ap)[1 + i], vw = glob(w)[1 + i];
+      const int c0 = child ? glob(cl)[1 + i] : 1, c1 = child ? glob(chh)[1 + i] : 1;
+      const int p0 = up ? glob(pl)[1 + i] : 1;
+      const double p1 = up ? (double)glob(pw)[1 + i] : 0.0;
+      sc_at<T>(D.c[2 * a])[i] = (T)vm;
+      sc_at<T>(D.c[2 * a + 1])[i] = (T)vp;
+      sc_at<double>(D.c64[2 * a])[i] = vm;
+      sc_at<double>(D.c64[2 * a + 1])[i] = vp;
+      sc_at<double>(D.w[a])[i] = vw;
+      sc_at<int>(D.ch[a])[i] = (c0 - 1) | ((c1 - 1) << 16);
+      sc_at<int>(D.pl[a])[i] = p0 - 1;
+      sc_at<T>(D.pw[a])[i] = (T)p1;
+    }
+  }
+  __syncthreads();
+  const ScRows rg = {P.r0, P.r1, corr};
+  using G = GlFields<T>;
+  for (int l = first; l < s0; ++l) {
+    sc_smooth<T, G>(S[l], team, nu.pre[Lc + l], omega, Lc + l == 0 ? &R : nullptr, rg, tmp);
+    sc_down<T, G, G>(S[l], S[l + 1], team);
+  }
+  if (team.rank == 0) sc_small<T>(P, levs, S, s0, nu, Lc, omega);
+  if (s0 == first) return;  // a single block
+  team.sync<true>();
+  for (int l = s0 - 1; l >= first; --l) {
+    sc_up<T, G, G>(S[l], S[l + 1], team);
+    if (Lc + l == 0) sc_rows<T>(R, rg, S[l], team, tmp);
+    sc_smooth<T, G>(S[l], team, nu.post[Lc + l], omega, Lc + l == 0 ? &R : nullptr, rg, tmp);
   }
 }
 
 template <typename T>
-cudaError_t small_cycle(int nprob, const SmallProb *probs, const DevLevel *levs, int maxgn, int nu1,
-                        int nu2, double omega, cudaStream_t s) {
-  if (nprob <= 0) return cudaSuccess;
-  const size_t sm = (size_t)std::max(1, maxgn) * sizeof(double);
-  if (sm > 48 * 1024)
-    cudaFuncSetAttribute(k_small_cycle<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  k_small_cycle<T><<<nprob, SC_THREADS, sm, s>>>(probs, levs, nu1, nu2, (T)omega);
-  note_launches(1);
-  return cudaGetLastError();
+int cycle_clusters(int size, size_t bytes) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = size; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+  cfg.gridDim = dim3(size);
+  cfg.blockDim = dim3(SC_THREADS);
+  cfg.dynamicSmemBytes = bytes;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaFuncSetAttribute(k_cycle<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess ||
+      cudaFuncSetAttribute(k_cycle<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&n, k_cycle<T>, &cfg) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return 0;
+  }
+  return n;
 }
-template cudaError_t small_cycle<float>(int, const SmallProb *, const DevLevel *, int, int, int, double,
-                                        cudaStream_t);
-template cudaError_t small_cycle<double>(int, const SmallProb *, const DevLevel *, int, int, int, double,
-                                         cudaStream_t);
+template int cycle_clusters<float>(int, size_t);
+template int cycle_clusters<double>(int, size_t);
+
+template <typename T>
+cudaError_t cycle(const Cycle &c, int first, const CycleSteps &nu, double omega, const DevRows &R, int corr,
+                  double *tmp, cudaStream_t s) {
+  if (c.n <= 0) return cudaSuccess;
+  const size_t sm = c.bytes + (size_t)sc_round(c.maxgn * (int)sizeof(double));
+  cudaError_t e = cudaFuncSetAttribute(k_cycle<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  if (e == cudaSuccess && c.size > 8)
+    e = cudaFuncSetAttribute(k_cycle<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (e != cudaSuccess) return e;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = c.size; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+  cfg.gridDim = dim3(c.n * c.size);
+  cfg.blockDim = dim3(SC_THREADS);
+  cfg.dynamicSmemBytes = sm;
+  cfg.stream = s;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  e = cudaLaunchKernelEx(&cfg, k_cycle<T>, c.probs, c.levs, c.Lc, first, c.maxgn, nu, (T)omega, R, corr, tmp);
+  note_launches(1);
+  return e;
+}
+template cudaError_t cycle<float>(const Cycle &, int, const CycleSteps &, double, const DevRows &, int, double *,
+                                  cudaStream_t);
+template cudaError_t cycle<double>(const Cycle &, int, const CycleSteps &, double, const DevRows &, int, double *,
+                                   cudaStream_t);
 
 // ----------------------------------------- layout conversion (boundary)
 // reference field (0:nx+1 nodes) <-> device level-0 layout, nx ny nz cells
@@ -3782,7 +4311,6 @@ template cudaError_t prolong_add<float>(const Launch &, const DevLevel *, cudaSt
 template cudaError_t residual<float>(const Launch &, double *, double *, cudaStream_t);
 template cudaError_t restrict_to<double>(const Launch &, const DevLevel *, cudaStream_t);
 template cudaError_t restrict_to<float>(const Launch &, const DevLevel *, cudaStream_t);
-template cudaError_t zero_x<double>(const Launch &, cudaStream_t);
 template cudaError_t zero_x<float>(const Launch &, cudaStream_t);
 template cudaError_t rows_relax<double>(const DevRows &, const DevLevel *, int, double *,
                                         cudaStream_t);
