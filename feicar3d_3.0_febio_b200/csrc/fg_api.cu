@@ -573,6 +573,7 @@ struct fg_batch {
   std::vector<long long> ksig;  // level-0 sizes and partial-sum blocks they were made for
   std::vector<void *> kraw;
   KDesc *d_kd = nullptr;
+  KrySet kset() const { return {d_kd, h_kd.empty() ? KDesc{} : h_kd[0]}; }
   std::vector<KDesc> h_kd;
   double *d_kpart = nullptr, *d_kout = nullptr, *d_kcoef = nullptr;
   KCtl *d_kctl = nullptr;   // scalar FGMRES state on the device
@@ -678,7 +679,7 @@ static void free_krylov(fg_batch *b) {
 // wave: room behind the offsets for the ticket and plane counters of a
 // both-colour y/z sweep (zeroed by each such launch)
 static fg_status build_offsets(const std::vector<int> &blocks, int **d_off, Launch &Lr,
-                               const DevLevel *d_lev, bool wave = false) {
+                               const DevLevel *d_lev, const std::vector<DevLevel> &h_lev, bool wave = false) {
   std::vector<int> off(blocks.size() + 1, 0);
   for (size_t p = 0; p < blocks.size(); ++p) off[p + 1] = off[p] + blocks[p];
   const int total = off.back();
@@ -688,6 +689,7 @@ static fg_status build_offsets(const std::vector<int> &blocks, int **d_off, Laun
   Lr.blocks = total;
   Lr.off = *d_off;
   Lr.lev = d_lev;
+  if (Lr.n == 1) Lr.one = h_lev[0];
   Lr.wave = wave ? *d_off + blocks.size() + 1 : nullptr;
   return FG_OK;
 }
@@ -921,12 +923,12 @@ static fg_status build_batch(fg_batch *b) {
     FG_CUDA(run_launch_set_alloc((void **)&s.d_levC, vC));
     if (!vS.empty()) {
       fg_status st;
-      if ((st = build_offsets(bc, &s.d_off_cells, s.cells, s.d_levS)) != FG_OK) return st;
-      if ((st = build_offsets(bx, &s.d_off_x, s.xl, s.d_levS)) != FG_OK) return st;
-      if ((st = build_offsets(by, &s.d_off_y, s.yl, s.d_levS, true)) != FG_OK) return st;
-      if ((st = build_offsets(bz, &s.d_off_z, s.zl, s.d_levS, true)) != FG_OK) return st;
-      if ((st = build_offsets(bn, &s.d_off_next, s.next, s.d_levS_next)) != FG_OK) return st;
-      if ((st = build_offsets(bq, &s.d_off_quads, s.quads, s.d_levS)) != FG_OK) return st;
+      if ((st = build_offsets(bc, &s.d_off_cells, s.cells, s.d_levS, vS)) != FG_OK) return st;
+      if ((st = build_offsets(bx, &s.d_off_x, s.xl, s.d_levS, vS)) != FG_OK) return st;
+      if ((st = build_offsets(by, &s.d_off_y, s.yl, s.d_levS, vS, true)) != FG_OK) return st;
+      if ((st = build_offsets(bz, &s.d_off_z, s.zl, s.d_levS, vS, true)) != FG_OK) return st;
+      if ((st = build_offsets(bn, &s.d_off_next, s.next, s.d_levS_next, vSn)) != FG_OK) return st;
+      if ((st = build_offsets(bq, &s.d_off_quads, s.quads, s.d_levS, vS)) != FG_OK) return st;
     }
     if (!s.C.empty()) {
       FG_CUDA(fg::dev_alloc(&s.d_G, s.C.size() * sizeof(double *)));
@@ -946,11 +948,11 @@ static fg_status build_batch(fg_batch *b) {
       bq.push_back(k::blocks_quads(c->lev[0].dl));
     }
     FG_CUDA(run_launch_set_alloc((void **)&b->d_lev0, v0));
-    fg_status st = build_offsets(b0, &b->d_off0, b->all0, b->d_lev0);
+    fg_status st = build_offsets(b0, &b->d_off0, b->all0, b->d_lev0, v0);
     if (st != FG_OK) return st;
-    st = build_offsets(bf, &b->d_offf0, b->flat0, b->d_lev0);
+    st = build_offsets(bf, &b->d_offf0, b->flat0, b->d_lev0, v0);
     if (st != FG_OK) return st;
-    st = build_offsets(bq, &b->d_offq0, b->all0q, b->d_lev0);
+    st = build_offsets(bq, &b->d_offq0, b->all0q, b->d_lev0, v0);
     if (st != FG_OK) return st;
   }
   fg_status st;
@@ -1058,7 +1060,7 @@ static fg_status smooth(fg_batch *b, int L, cudaStream_t s) {
     }
     if (L == 0) {
       const size_t e0 = prof_begin(b, s);
-      FG_K(k::rows_relax<T>(b->rows, b->d_lev0, corr, b->d_tmp, s));
+      FG_K(k::rows_relax<T>(b->rows, b->all0, corr, b->d_tmp, s));
       prof_end(b, e0, FG_PROF_ROWS, 0.0, s);
     }
   }
@@ -1077,7 +1079,7 @@ static fg_status vcycle(fg_batch *b, cudaStream_t s) {
         if ((st = smooth<T>(b, L, s)) != FG_OK) return st;
       const size_t e0 = prof_begin(b, s);
       FG_K(k::residual_q<T>(ls.quads, s));
-      FG_K(k::restrict_to<T>(ls.next, ls.d_levS, s));
+      FG_K(k::restrict_to<T>(ls.next, ls.quads, s));
       prof_end(b, e0, FG_PROF_TRANSFER, 0.0, s);
     }
     if (!ls.C.empty()) {
@@ -1100,11 +1102,11 @@ static fg_status vcycle(fg_batch *b, cudaStream_t s) {
     auto &ls = b->ls[L];
     if (ls.S.empty()) continue;
     size_t e0 = prof_begin(b, s);
-    FG_K(k::prolong_add<T>(ls.cells, ls.d_levS_next, s));
+    FG_K(k::prolong_add<T>(ls.cells, ls.next, s));
     prof_end(b, e0, FG_PROF_TRANSFER, 0.0, s);
     if (L == 0) {
       e0 = prof_begin(b, s);
-      FG_K(k::rows_relax<T>(b->rows, b->d_lev0, corr, b->d_tmp, s));
+      FG_K(k::rows_relax<T>(b->rows, b->all0, corr, b->d_tmp, s));
       prof_end(b, e0, FG_PROF_ROWS, 0.0, s);
     }
     for (int q = 0; q < nu_post(b, L); ++q)
@@ -1190,7 +1192,7 @@ static fg_status batch_solve_richardson(fg_batch *b, fg_solve_stats *st) {
   if (!b->ev0) { cudaEventCreate(&b->ev0); cudaEventCreate(&b->ev1); }
   FG_CUDA(cudaEventRecord(b->ev0, s));
   // ghost / dead values consistent with the initial field
-  FG_K(k::rows_relax<double>(b->rows, b->d_lev0, 0, b->d_tmp, s));
+  FG_K(k::rows_relax<double>(b->rows, b->all0, 0, b->d_tmp, s));
   FG_CUDA(cudaMemsetAsync(b->d_norm, 0, 3 * np * sizeof(double), s));
   FG_K(k::fluid_norm(b->all0, b->d_norm + np, b->d_part, s));
   if (mixed) {
@@ -1337,7 +1339,7 @@ struct FgPieces {
   // scalar state reset
   fg_status pre(cudaStream_t s) {
     const int np = (int)b->cases.size();
-    FG_K(k::rows_relax<double>(b->rows, b->d_lev0, 0, b->d_tmp, s));
+    FG_K(k::rows_relax<double>(b->rows, b->all0, 0, b->d_tmp, s));
     FG_CUDA(cudaMemsetAsync(b->d_norm, 0, 3 * np * sizeof(double), s));
     FG_K(k::fluid_norm(b->all0, b->d_norm + np, b->d_part, s));
     for (int p = 0; p < np; ++p) {
@@ -1354,8 +1356,8 @@ struct FgPieces {
     const int np = (int)b->cases.size();
     FG_CUDA(cudaMemsetAsync(b->d_norm, 0, np * sizeof(double), s));
     const size_t e_r = prof_begin(b, s);
-    FG_K(k::kr_resid<B>(b->all0q, b->rows, b->d_lev0, b->d_kd, 0, b->d_part, b->d_norm, s));
-    FG_K(k::krd_dots<B>(b->flat0, b->d_kd, b->d_kctl, KPH_RESTART, b->d_kpart, b->d_kout, s));
+    FG_K(k::kr_resid<B>(b->all0q, b->rows, b->kset(), 0, b->d_part, b->d_norm, s));
+    FG_K(k::krd_dots<B>(b->flat0, b->kset(), b->d_kctl, KPH_RESTART, b->d_kpart, b->d_kout, s));
     prof_end(b, e_r, FG_PROF_RESIDUAL, 0.0, s);
     FG_K(k::fg_restart(b->d_kctl, b->d_kprob, b->d_kout, b->d_norm, b->d_kcoef, use_cond, ho, hb, hi, s));
     return FG_OK;
@@ -1363,7 +1365,7 @@ struct FgPieces {
   // V_0 / beta, staged as the first preconditioner input
   fg_status stage(cudaStream_t s) {
     const size_t e0 = prof_begin(b, s);
-    FG_K((k::krd_vaxpy<B, T>(b->flat0, b->rows, b->d_lev0, b->d_kd, b->d_kctl, KPH_RESTART, b->d_kcoef, s)));
+    FG_K((k::krd_vaxpy<B, T>(b->flat0, b->rows, b->kset(), b->d_kctl, KPH_RESTART, b->d_kcoef, s)));
     prof_end(b, e0, FG_PROF_RESIDUAL, 0.0, s);
     return FG_OK;
   }
@@ -1372,8 +1374,8 @@ struct FgPieces {
     fg_status r = graph ? vcycle<T>(b, s) : run_vcycle<T>(b, s);
     if (r != FG_OK) return r;
     const size_t e0 = prof_begin(b, s);
-    FG_K((k::krd_apply<B, T>(b->all0q, b->rows, b->d_lev0, b->d_kd, b->d_kctl, s)));
-    FG_K(k::krd_dots<B>(b->flat0, b->d_kd, b->d_kctl, KPH_APPLY, b->d_kpart, b->d_kout, s));
+    FG_K((k::krd_apply<B, T>(b->all0q, b->rows, b->kset(), b->d_kctl, s)));
+    FG_K(k::krd_dots<B>(b->flat0, b->kset(), b->d_kctl, KPH_APPLY, b->d_kpart, b->d_kout, s));
     prof_end(b, e0, FG_PROF_RESIDUAL, 0.0, s);
     FG_K(k::fg_reorth_test(b->d_kctl, b->d_kprob, b->d_kout, b->d_kcoef, use_cond, hr, s));
     return FG_OK;
@@ -1381,8 +1383,8 @@ struct FgPieces {
   // the second Gram-Schmidt pass
   fg_status reorth(cudaStream_t s) {
     const size_t e0 = prof_begin(b, s);
-    FG_K((k::krd_vaxpy<B, T>(b->flat0, b->rows, b->d_lev0, b->d_kd, b->d_kctl, KPH_REORTH, b->d_kcoef, s)));
-    FG_K(k::krd_dots<B>(b->flat0, b->d_kd, b->d_kctl, KPH_APPLY, b->d_kpart, b->d_kout, s));
+    FG_K((k::krd_vaxpy<B, T>(b->flat0, b->rows, b->kset(), b->d_kctl, KPH_REORTH, b->d_kcoef, s)));
+    FG_K(k::krd_dots<B>(b->flat0, b->kset(), b->d_kctl, KPH_APPLY, b->d_kpart, b->d_kout, s));
     prof_end(b, e0, FG_PROF_RESIDUAL, 0.0, s);
     return FG_OK;
   }
@@ -1390,7 +1392,7 @@ struct FgPieces {
   fg_status step_b(cudaStream_t s, int use_cond, unsigned long long hi) {
     FG_K(k::fg_arnoldi(b->d_kctl, b->d_kprob, b->d_kout, b->d_kcoef, use_cond, hi, s));
     const size_t e0 = prof_begin(b, s);
-    FG_K((k::krd_vaxpy<B, T>(b->flat0, b->rows, b->d_lev0, b->d_kd, b->d_kctl, KPH_NORMALIZE, b->d_kcoef,
+    FG_K((k::krd_vaxpy<B, T>(b->flat0, b->rows, b->kset(), b->d_kctl, KPH_NORMALIZE, b->d_kcoef,
                              s)));
     prof_end(b, e0, FG_PROF_RESIDUAL, 0.0, s);
     return FG_OK;
@@ -1399,7 +1401,7 @@ struct FgPieces {
   fg_status finish_cycle(cudaStream_t s) {
     FG_K(k::fg_lsq(b->d_kctl, b->d_kprob, b->d_kcoef, s));
     const size_t e0 = prof_begin(b, s);
-    FG_K(k::krd_update<B>(b->flat0, b->d_kd, b->d_kctl, b->d_kcoef, s));
+    FG_K(k::krd_update<B>(b->flat0, b->kset(), b->d_kctl, b->d_kcoef, s));
     prof_end(b, e0, FG_PROF_RESIDUAL, 0.0, s);
     return FG_OK;
   }
@@ -1558,6 +1560,7 @@ static std::vector<char> solve_params(const fg_batch *b) {
   std::vector<char> v = vcycle_params(b);
   auto put = [&](const void *p, size_t n) { v.insert(v.end(), (const char *)p, (const char *)p + n); };
   put(&b->d_kd, sizeof(b->d_kd));
+  put(b->h_kd.data(), b->h_kd.size() * sizeof(KDesc));  // a lone problem's is a launch argument
   put(&b->d_kctl, sizeof(b->d_kctl));
   put(&b->km, sizeof(b->km));
   put(&b->cfg.max_cycles, sizeof(int));
@@ -1689,7 +1692,7 @@ static fg_status batch_solve_lsor(fg_batch *b, fg_solve_stats *st) {
   if (b->ls[0].S.empty()) return FG_BAD_INPUT;  // a single-level grid has no line launches
   if (!b->ev0) { cudaEventCreate(&b->ev0); cudaEventCreate(&b->ev1); }
   FG_CUDA(cudaEventRecord(b->ev0, s));
-  FG_K(k::rows_relax<double>(b->rows, b->d_lev0, 0, b->d_tmp, s));
+  FG_K(k::rows_relax<double>(b->rows, b->all0, 0, b->d_tmp, s));
   FG_CUDA(cudaMemsetAsync(b->d_norm, 0, 3 * np * sizeof(double), s));
   FG_K(k::fluid_norm(b->all0, b->d_norm + np, b->d_part, s));
   b->history.clear();
@@ -1798,8 +1801,10 @@ static std::vector<int> tune_key(const fg_batch *b) {
 static fg_status rebuild_line_offsets(fg_batch *b, int L, int axis) {
   auto &s = b->ls[L];
   std::vector<int> blocks;
+  std::vector<DevLevel> lev;
   for (int p : s.S) {
     const DevLevel &d = b->cases[p]->lev[L].dl;
+    lev.push_back(d);
     blocks.push_back(axis == 0 ? k::blocks_xline(d, s.maxnx, b->tune.var[L][0])
                                : k::blocks_tile(d, axis, axis == 1 ? s.maxny : s.maxnz, b->tune.var[L][axis]));
   }
@@ -1807,7 +1812,7 @@ static fg_status rebuild_line_offsets(fg_batch *b, int L, int axis) {
   Launch &Lr = axis == 0 ? s.xl : axis == 1 ? s.yl : s.zl;
   fg::dev_free(*off);
   *off = nullptr;
-  return build_offsets(blocks, off, Lr, s.d_levS, axis != 0);
+  return build_offsets(blocks, off, Lr, s.d_levS, lev, axis != 0);
 }
 
 // the captured V-cycle and solve graphs hold the old launch shapes
@@ -2782,7 +2787,7 @@ fg_status fg_ghostcell_pressure(fg_case *c, double *p, const double *p_old, int 
   FG_CUDA(cudaMemcpyAsync(c->d_pin, p, nref * sizeof(double), cudaMemcpyHostToDevice, c->stream));
   FG_K(k::copy_in(L0.d_x64 ? L0.d_x64 : nullptr, c->d_pin, L0.nx, L0.ny, L0.nz, L0.sy, L0.sz, c->stream));
   for (int it = 0; it < iterations; ++it)
-    FG_K(k::rows_relax<double>(c->solo->rows, c->solo->d_lev0, 0, c->solo->d_tmp, c->stream));
+    FG_K(k::rows_relax<double>(c->solo->rows, c->solo->all0, 0, c->solo->d_tmp, c->stream));
   FG_K(k::copy_out(c->d_pin, L0.d_x64, L0.nx, L0.ny, L0.nz, L0.sy, L0.sz, c->stream));
   FG_CUDA(cudaMemcpyAsync(p, c->d_pin, nref * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   FG_CUDA(cudaStreamSynchronize(c->stream));

@@ -147,6 +147,7 @@ struct Launch {
   const int *off = nullptr;
   const DevLevel *lev = nullptr;
   int *wave = nullptr;  // y/z sweeps: ticket and plane counters (blocks + 2 ints)
+  DevLevel one{};       // n == 1: the problem's level, passed to the kernels by value
   bool empty() const { return n == 0 || blocks == 0; }
 };
 
@@ -206,6 +207,12 @@ struct KDesc {
   long long n;       // elements of one vector (the level's ntot)
   long long stride;  // elements from one vector to the next
 };
+// the Krylov vectors of a batch: one descriptor per problem on the device,
+// and the first problem's by value
+struct KrySet {
+  const KDesc *kd = nullptr;
+  KDesc one{};
+};
 constexpr int KR_MAXV = 16;  // most vectors one dot-product pass reads
 constexpr int KR_CS = KR_MAXV + 2;  // stride of the per-problem dot results and coefficients
 
@@ -260,7 +267,7 @@ enum : int {
 constexpr int SC_MAXN = 128;                // longest line (4 rows per lane of a warp)
 constexpr size_t SC_MAXBYTES = 200 * 1024;  // shared memory of a block
 constexpr long long SC_MAXCELLS = 2048;   // a cluster's largest level in shared memory
-constexpr long long CL_MAXCELLS = 16384;     // a cluster's largest level in global memory
+constexpr long long CL_MAXCELLS = 32768;     // a cluster's largest level in global memory
 constexpr int CL_MAXPROBS = 16;             // most problems that get a cluster of more than one block
 struct CycleProb {
   int l0, nl, ns;
@@ -324,10 +331,9 @@ cudaError_t line_sweep(const Launch &L, int axis, int color, double omega, int m
 template <typename T>
 cudaError_t residual(const Launch &L, double *norm2, double *part, cudaStream_t s);
 template <typename T>
-cudaError_t restrict_to(const Launch &fine_cells_of_coarse, const DevLevel *fine,
-                        cudaStream_t s);
+cudaError_t restrict_to(const Launch &coarse_cells, const Launch &fine, cudaStream_t s);
 template <typename T>
-cudaError_t prolong_add(const Launch &fine, const DevLevel *coarse, cudaStream_t s);
+cudaError_t prolong_add(const Launch &fine, const Launch &coarse, cudaStream_t s);
 // the residual (no norm) with quads: Launch over the level's quads
 // (blocks_quads)
 template <typename T>
@@ -345,8 +351,7 @@ template <typename T>
 cudaError_t cycle(const Cycle &c, int first, const CycleSteps &nu, double omega, const DevRows &R, int corr,
                   double *tmp, cudaStream_t s);
 template <typename T>
-cudaError_t rows_relax(const DevRows &R, const DevLevel *lev0, int correction_form,
-                       double *tmp, cudaStream_t s);
+cudaError_t rows_relax(const DevRows &R, const Launch &L0, int correction_form, double *tmp, cudaStream_t s);
 cudaError_t rows_residual(const DevRows &R, const DevLevel *lev0, double *maxabs,
                           cudaStream_t s);
 template <typename T>
@@ -418,33 +423,33 @@ cudaError_t finish_field(double *ref, const DevLevel *lev0, int nx, int ny, int 
 //             active rows (0 elsewhere), x_T = 0, row constants = V_vd
 //  kr_update: P += sum_{i<ns} c_{1+i} Z_i
 template <typename B>
-cudaError_t kr_resid(const Launch &cells, const DevRows &R, const DevLevel *lev0, const KDesc *kd, int vd,
+cudaError_t kr_resid(const Launch &cells, const DevRows &R, const KrySet &kd, int vd,
                      double *part, double *norm2, cudaStream_t s);
 template <typename B, typename T>
-cudaError_t kr_apply(const Launch &cells, const DevRows &R, const DevLevel *lev0, const KDesc *kd, int vz,
+cudaError_t kr_apply(const Launch &cells, const DevRows &R, const KrySet &kd, int vz,
                      int vw, cudaStream_t s);
 template <typename B>
-cudaError_t kr_dots(const Launch &flat, const KDesc *kd, int vw, int nv, double *part, double *out,
+cudaError_t kr_dots(const Launch &flat, const KrySet &kd, int vw, int nv, double *part, double *out,
                     int ostride, cudaStream_t s);
 template <typename B, typename T>
-cudaError_t kr_vaxpy(const Launch &flat, const DevRows &R, const DevLevel *lev0, const KDesc *kd, int vd,
+cudaError_t kr_vaxpy(const Launch &flat, const DevRows &R, const KrySet &kd, int vd,
                      int s0, int ns, const double *coef, int cs, bool stage, cudaStream_t s);
 template <typename B>
-cudaError_t kr_update(const Launch &flat, const KDesc *kd, int ns, const double *coef, int cs,
+cudaError_t kr_update(const Launch &flat, const KrySet &kd, int ns, const double *coef, int cs,
                       cudaStream_t s);
 // The same vector passes with their vector indices taken on the device from
 // ctl (phase KPH_*), so one captured launch serves every step of a loop.
 template <typename B, typename T>
-cudaError_t krd_apply(const Launch &quads, const DevRows &R, const DevLevel *lev0, const KDesc *kd,
+cudaError_t krd_apply(const Launch &quads, const DevRows &R, const KrySet &kd,
                       const KCtl *ctl, cudaStream_t s);
 template <typename B>
-cudaError_t krd_dots(const Launch &flat, const KDesc *kd, const KCtl *ctl, int phase, double *part,
+cudaError_t krd_dots(const Launch &flat, const KrySet &kd, const KCtl *ctl, int phase, double *part,
                      double *out, cudaStream_t s);
 template <typename B, typename T>
-cudaError_t krd_vaxpy(const Launch &flat, const DevRows &R, const DevLevel *lev0, const KDesc *kd,
+cudaError_t krd_vaxpy(const Launch &flat, const DevRows &R, const KrySet &kd,
                       const KCtl *ctl, int phase, const double *coef, cudaStream_t s);
 template <typename B>
-cudaError_t krd_update(const Launch &flat, const KDesc *kd, const KCtl *ctl, const double *coef,
+cudaError_t krd_update(const Launch &flat, const KrySet &kd, const KCtl *ctl, const double *coef,
                        cudaStream_t s);
 // scalar FGMRES steps (one block over all problems); with use_cond the
 // decisions are also written to the CUDA graph conditional handles

@@ -66,6 +66,57 @@ __device__ __forceinline__ int find_entry(const int *off, int n, int b) {
   return lo;
 }
 
+// What a launch over a set of problems works on.  With one problem its
+// level descriptor (and Krylov vectors) is the kernel argument itself, read
+// from constant memory; with several, a block finds its problem and reads
+// the descriptor from global memory.  The two or three dependent reads this
+// saves are a large part of a small launch (y/z lines of 32 rows in FP64: 8.6
+// -> 6.1 us under ncu) and shorten the larger ones too, by the descriptor's
+// re-reads (512x256x256 mixed solve: 91.4 -> 85.9 ms with the rows below).
+template <bool ONE> struct Lev;
+template <> struct Lev<false> {
+  const int *off;
+  int n;
+  const DevLevel *levs;
+};
+template <> struct Lev<true> {
+  DevLevel one;
+};
+template <bool ONE> struct Kry;
+template <> struct Kry<false> {
+  const KDesc *kd;
+};
+template <> struct Kry<true> {
+  KDesc one;
+};
+// the block's problem p, its block lb within the problem, and its level
+__device__ __forceinline__ const DevLevel &entry(const Lev<true> &a, int &p, int &lb) {
+  p = 0;
+  lb = blockIdx.x;
+  return a.one;
+}
+__device__ __forceinline__ const DevLevel &entry(const Lev<false> &a, int &p, int &lb) {
+  p = find_entry(a.off, a.n, blockIdx.x);
+  lb = blockIdx.x - a.off[p];
+  return a.levs[p];
+}
+__device__ __forceinline__ const DevLevel &level(const Lev<true> &a, int) { return a.one; }
+__device__ __forceinline__ const DevLevel &level(const Lev<false> &a, int p) { return a.levs[p]; }
+__device__ __forceinline__ const KDesc &krylov(const Kry<true> &a, int) { return a.one; }
+__device__ __forceinline__ const KDesc &krylov(const Kry<false> &a, int p) { return a.kd[p]; }
+template <bool ONE> Lev<ONE> lev_of(const Launch &L);
+template <> inline Lev<true> lev_of<true>(const Launch &L) { return {L.one}; }
+template <> inline Lev<false> lev_of<false>(const Launch &L) { return {L.off, L.n, L.lev}; }
+template <bool ONE> Kry<ONE> kry_of(const KrySet &K);
+template <> inline Kry<true> kry_of<true>(const KrySet &K) { return {K.one}; }
+template <> inline Kry<false> kry_of<false>(const KrySet &K) { return {K.kd}; }
+// calls f with the launch's form as a compile-time constant
+template <class F>
+static void by_form(const Launch &L, F f) {
+  if (L.n == 1) f(std::true_type{});
+  else f(std::false_type{});
+}
+
 // 1 = coupled neighbour, 2 = Dirichlet boundary face (diagonal doubled,
 // CORE_SET_OUTER_BC.F90:901-904 with :1093), 0 = face dropped (Neumann
 // boundary, CORE_SET_OUTER_BC.F90:907-911 with pgrad = 0, or OFF cell)
@@ -667,12 +718,11 @@ __device__ __forceinline__ void chunk_eliminate_smem(int r0, int n, const uint8_
 // chunk-first unknowns are solved by PCR across the line's lanes.  One
 // pass over rhs, mask, the line's own values and its four neighbour
 // lines; no shared memory.
-template <typename T, int M, int W>
+template <typename T, int M, int W, bool ONE>
 __global__ void __launch_bounds__(XL_WARPS * 32, 1)
-k_xline_reg(const int *FG_RESTRICT off, int nent, const DevLevel *FG_RESTRICT levs, int color, T omega) {
-  const int p = find_entry(off, nent, blockIdx.x);
-  const DevLevel &L = levs[p];
-  const int lb = blockIdx.x - off[p];
+k_xline_reg(const __grid_constant__ Lev<ONE> A, int color, T omega) {
+  int p, lb;
+  const DevLevel &L = entry(A, p, lb);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int sl = lane % W;
   const int nyh = (L.ny + 1) >> 1;
@@ -808,9 +858,9 @@ __device__ __forceinline__ bool xs_line(const DevLevel &L, int lb, int warp, int
   return j <= L.ny;
 }
 
-template <typename T, int M>
+template <typename T, int M, bool ONE>
 __global__ void __launch_bounds__(XS_WARPS * 32)
-k_xline_smem(const int *FG_RESTRICT off, int nent, const DevLevel *FG_RESTRICT levs, int color, T omega) {
+k_xline_smem(const __grid_constant__ Lev<ONE> A, int color, T omega) {
   using LY = XsLayout<T, M>;
   using LC = LineCoefT<T, 0>;
   constexpr int P = XS_PIECE;
@@ -819,9 +869,8 @@ k_xline_smem(const int *FG_RESTRICT off, int nent, const DevLevel *FG_RESTRICT l
   // chunk starts at l (M + 1), so the lanes' reads fall in distinct banks
   __shared__ T s_am[32 * (M + 1)], s_ap[32 * (M + 1)];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int p = find_entry(off, nent, blockIdx.x);
-  const DevLevel &L = levs[p];
-  const int lb = blockIdx.x - off[p];
+  int p, lb;
+  const DevLevel &L = entry(A, p, lb);
   const int n = L.nx;
   for (int r = threadIdx.x; r < n; r += XS_WARPS * 32) {
     s_am[r + r / M] = (T)glob(L.amx)[1 + r];
@@ -923,9 +972,9 @@ struct ChunkEq { T a, b, c, d; };
 template <typename T>
 struct Eq3 { T a, c, d; };  // a x_prev + x + c x_next = d
 
-template <typename T, int M, int CH, int AXIS>
+template <typename T, int M, int CH, int AXIS, bool ONE>
 __global__ void __launch_bounds__(CH * 32, (sizeof(T) == 4 && CH == 16) ? (M <= 8 ? 3 : 2) : 1)
-k_yzline_reg(const int *FG_RESTRICT off, int nent, const DevLevel *FG_RESTRICT levs, int color, T omega) {
+k_yzline_reg(const __grid_constant__ Lev<ONE> A, int color, T omega) {
   using LC = LineCoefT<T, AXIS>;
   __shared__ ChunkEq<T> s_eq[CH][32];
   __shared__ T s_f[CH + 1][32];   // chunk-first unknowns
@@ -936,9 +985,8 @@ k_yzline_reg(const int *FG_RESTRICT off, int nent, const DevLevel *FG_RESTRICT l
   T *s_al = s_d + M * NT;
   T *s_ga = s_al + M * NT;
   const int tid = threadIdx.x;
-  const int p = find_entry(off, nent, blockIdx.x);
-  const DevLevel &L = levs[p];
-  const int lb = blockIdx.x - off[p];
+  int p, lb;
+  const DevLevel &L = entry(A, p, lb);
   const int ntx = (L.nx + 63) >> 6;
   const int ti = lb % ntx;
   const int o = 1 + lb / ntx;  // k for AXIS 1, j for AXIS 2
@@ -1269,7 +1317,9 @@ static cudaError_t launch_line(const Launch &Lr, int axis, int color, double ome
 // maxn: the longest line of this launch along `axis`
 template <typename T, int M, int W>
 static cudaError_t launch_xreg(const Launch &Lr, int color, double omega, cudaStream_t s) {
-  k_xline_reg<T, M, W><<<Lr.blocks, XL_WARPS * 32, 0, s>>>(Lr.off, Lr.n, Lr.lev, color, (T)omega);
+  by_form(Lr, [&](auto one) {
+    k_xline_reg<T, M, W, one.value><<<Lr.blocks, XL_WARPS * 32, 0, s>>>(lev_of<one.value>(Lr), color, (T)omega);
+  });
   note_launches(1);
   return cudaGetLastError();
 }
@@ -1512,12 +1562,11 @@ struct YpBound {
 // one colour of a sweep: block -> (problem, tile, plane); a colour-1
 // launch walks the planes backward, so its first blocks meet the planes
 // the colour-0 launch left in L2
-template <typename T, int M, int CH, int AXIS, int NB>
+template <typename T, int M, int CH, int AXIS, int NB, bool ONE>
 __global__ void __launch_bounds__(CH * YP_LINES, YpBound<T, CH, NB>::v)
-k_yzline_pcr(const int *FG_RESTRICT off, int nent, const DevLevel *FG_RESTRICT levs, int color, T omega) {
-  const int p = find_entry(off, nent, blockIdx.x);
-  const int lb = blockIdx.x - off[p];
-  const DevLevel &L = levs[p];
+k_yzline_pcr(const __grid_constant__ Lev<ONE> A, int color, T omega) {
+  int p, lb;
+  const DevLevel &L = entry(A, p, lb);
   const int ntx = (L.nx + 2 * YP_LINES - 1) / (2 * YP_LINES);
   const int ti = lb % ntx;
   const int o = color == 1 ? (AXIS == 1 ? L.nz : L.ny) - lb / ntx : 1 + lb / ntx;
@@ -1595,9 +1644,11 @@ k_yzline_wave(const int *FG_RESTRICT off, int nent, const DevLevel *FG_RESTRICT 
 template <typename T, int M>
 static cudaError_t launch_xsmem(const Launch &Lr, int color, double omega, cudaStream_t s) {
   const size_t sm = (size_t)XS_WARPS * XsLayout<T, M>::PER_WARP;
-  auto kern = k_xline_smem<T, M>;
-  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  kern<<<Lr.blocks, XS_WARPS * 32, sm, s>>>(Lr.off, Lr.n, Lr.lev, color, (T)omega);
+  by_form(Lr, [&](auto one) {
+    auto kern = k_xline_smem<T, M, one.value>;
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    kern<<<Lr.blocks, XS_WARPS * 32, sm, s>>>(lev_of<one.value>(Lr), color, (T)omega);
+  });
   note_launches(1);
   return cudaGetLastError();
 }
@@ -1605,15 +1656,11 @@ static cudaError_t launch_xsmem(const Launch &Lr, int color, double omega, cudaS
 template <typename T, int M, int CH, int NB = 0>
 static cudaError_t launch_yzpcr(const Launch &Lr, int axis, int color, double omega, cudaStream_t s) {
   const size_t sm = (size_t)2 * CH * YP_LINES * sizeof(Eq3<T>);
-  if (axis == 1) {
-    auto kern = k_yzline_pcr<T, M, CH, 1, NB>;
+  by_form(Lr, [&](auto one) {
+    auto kern = axis == 1 ? k_yzline_pcr<T, M, CH, 1, NB, one.value> : k_yzline_pcr<T, M, CH, 2, NB, one.value>;
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    kern<<<Lr.blocks, CH * YP_LINES, sm, s>>>(Lr.off, Lr.n, Lr.lev, color, (T)omega);
-  } else {
-    auto kern = k_yzline_pcr<T, M, CH, 2, NB>;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    kern<<<Lr.blocks, CH * YP_LINES, sm, s>>>(Lr.off, Lr.n, Lr.lev, color, (T)omega);
-  }
+    kern<<<Lr.blocks, CH * YP_LINES, sm, s>>>(lev_of<one.value>(Lr), color, (T)omega);
+  });
   note_launches(1);
   return cudaGetLastError();
 }
@@ -1692,15 +1739,11 @@ bool line_both_colours(int axis, int maxn, int variant) {
 template <typename T, int M, int CH>
 static cudaError_t launch_yzreg(const Launch &Lr, int axis, int color, double omega, cudaStream_t s) {
   const size_t sm = (size_t)3 * M * CH * 32 * sizeof(T);  // row state: d, al, ga
-  if (axis == 1) {
-    auto kern = k_yzline_reg<T, M, CH, 1>;
+  by_form(Lr, [&](auto one) {
+    auto kern = axis == 1 ? k_yzline_reg<T, M, CH, 1, one.value> : k_yzline_reg<T, M, CH, 2, one.value>;
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    kern<<<Lr.blocks, CH * 32, sm, s>>>(Lr.off, Lr.n, Lr.lev, color, (T)omega);
-  } else {
-    auto kern = k_yzline_reg<T, M, CH, 2>;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    kern<<<Lr.blocks, CH * 32, sm, s>>>(Lr.off, Lr.n, Lr.lev, color, (T)omega);
-  }
+    kern<<<Lr.blocks, CH * 32, sm, s>>>(lev_of<one.value>(Lr), color, (T)omega);
+  });
   note_launches(1);
   return cudaGetLastError();
 }
@@ -2011,12 +2054,11 @@ struct QuadVals {
 
 // r = f - A x on active cells, 0 on the other interior cells (the V-cycle's
 // restriction input); the arithmetic of k_residual, per quad
-template <typename T>
+template <typename T, bool ONE>
 __global__ void __launch_bounds__(QBLOCK)
-k_residual_q(const int *FG_RESTRICT off, int nent, const DevLevel *FG_RESTRICT levs) {
-  const int p = find_entry(off, nent, blockIdx.x);
-  const DevLevel &L = levs[p];
-  const int lb = blockIdx.x - off[p];
+k_residual_q(const __grid_constant__ Lev<ONE> A) {
+  int p, lb;
+  const DevLevel &L = entry(A, p, lb);
   auto x = PrecOf<T>::x(L);
   auto rhs = PrecOf<T>::rhs(L);
   auto res = PrecOf<T>::res(L);
@@ -2052,7 +2094,7 @@ k_residual_q(const int *FG_RESTRICT off, int nent, const DevLevel *FG_RESTRICT l
 template <typename T>
 cudaError_t residual_q(const Launch &Lq, cudaStream_t s) {
   if (Lq.empty()) return cudaSuccess;
-  k_residual_q<T><<<Lq.blocks, QBLOCK, 0, s>>>(Lq.off, Lq.n, Lq.lev);
+  by_form(Lq, [&](auto one) { k_residual_q<T, one.value><<<Lq.blocks, QBLOCK, 0, s>>>(lev_of<one.value>(Lq)); });
   note_launches(1);
   return cudaGetLastError();
 }
@@ -2061,13 +2103,12 @@ cudaError_t residual_q(const Launch &Lq, cudaStream_t s) {
 // coarse rhs = volume-weighted mean of the children's residuals on active
 // coarse cells (the sum of the children's finite-volume equations)
 // (and the coarse unknown starts from zero)
-template <typename T>
+template <typename T, bool ONE>
 __global__ void __launch_bounds__(CELL_BLOCK)
-k_restrict(const int *FG_RESTRICT off, int nent, const DevLevel *FG_RESTRICT coarse, const DevLevel *FG_RESTRICT fine) {
-  const int p = find_entry(off, nent, blockIdx.x);
-  const DevLevel &C = coarse[p];
-  const DevLevel &F = fine[p];
-  const int lb = blockIdx.x - off[p];
+k_restrict(const __grid_constant__ Lev<ONE> A, const __grid_constant__ Lev<ONE> FA) {
+  int p, lb;
+  const DevLevel &C = entry(A, p, lb);
+  const DevLevel &F = level(FA, p);
   // the thread's i-children and their widths are kept over the block's
   // CELL_ROWS rows (at most two children per
   // axis: cl = 2I-1, ch = min(2I, n))
@@ -2127,9 +2168,11 @@ k_restrict(const int *FG_RESTRICT off, int nent, const DevLevel *FG_RESTRICT coa
 }
 
 template <typename T>
-cudaError_t restrict_to(const Launch &Lc, const DevLevel *fine, cudaStream_t s) {
+cudaError_t restrict_to(const Launch &Lc, const Launch &Lf, cudaStream_t s) {
   if (Lc.empty()) return cudaSuccess;
-  k_restrict<T><<<Lc.blocks, CELL_BLOCK, 0, s>>>(Lc.off, Lc.n, Lc.lev, fine);
+  by_form(Lc, [&](auto one) {
+    k_restrict<T, one.value><<<Lc.blocks, CELL_BLOCK, 0, s>>>(lev_of<one.value>(Lc), lev_of<one.value>(Lf));
+  });
   note_launches(1);
   return cudaGetLastError();
 }
@@ -2189,17 +2232,16 @@ __device__ __forceinline__ void cp_async_wait_all() {
   asm volatile("cp.async.wait_group 0;\n" ::: "memory");
 }
 
-template <typename T>
+template <typename T, bool ONE>
 __global__ void __launch_bounds__(PT_I)
-k_prolong(const int *FG_RESTRICT off, int nent, const DevLevel *FG_RESTRICT fine, const DevLevel *FG_RESTRICT coarse) {
+k_prolong(const __grid_constant__ Lev<ONE> A, const __grid_constant__ Lev<ONE> CA) {
   __shared__ T sv[2 * PT_CJ * PT_CI];
   __shared__ uint32_t smw[2 * PT_CJ * PT_MW];
   __shared__ T swy[PT_J];
   __shared__ int sr0[PT_J], sr1[PT_J];
-  const int p = find_entry(off, nent, blockIdx.x);
-  const DevLevel &F = fine[p];
-  const DevLevel &C = coarse[p];
-  const int lb = blockIdx.x - off[p];
+  int p, lb;
+  const DevLevel &F = entry(A, p, lb);
+  const DevLevel &C = level(CA, p);
   const int nti = (F.nx + PT_I - 1) / PT_I, ntj = (F.ny + PT_J - 1) / PT_J;
   const int ti = lb % nti, rest = lb / nti, tj = rest % ntj, k = 1 + rest / ntj;
   const int ia = 1 + ti * PT_I, ib = min(F.nx, ia + PT_I - 1);
@@ -2281,9 +2323,11 @@ k_prolong(const int *FG_RESTRICT off, int nent, const DevLevel *FG_RESTRICT fine
 }
 
 template <typename T>
-cudaError_t prolong_add(const Launch &Lf, const DevLevel *coarse, cudaStream_t s) {
+cudaError_t prolong_add(const Launch &Lf, const Launch &Lc, cudaStream_t s) {
   if (Lf.empty()) return cudaSuccess;
-  k_prolong<T><<<Lf.blocks, CELL_BLOCK, 0, s>>>(Lf.off, Lf.n, Lf.lev, coarse);
+  by_form(Lf, [&](auto one) {
+    k_prolong<T, one.value><<<Lf.blocks, CELL_BLOCK, 0, s>>>(lev_of<one.value>(Lf), lev_of<one.value>(Lc));
+  });
   note_launches(1);
   return cudaGetLastError();
 }
@@ -2315,12 +2359,12 @@ cudaError_t zero_x(const Launch &Lr, cudaStream_t s) {
 // (solution form) or the row residual (correction form).  Rows read other
 // rows' targets, so the update is a Jacobi step: all new values are formed
 // from the current field first (k_rows), then written (k_rows_scatter).
-template <typename T>
+template <typename T, bool ONE>
 __global__ void __launch_bounds__(CELL_BLOCK)
-k_rows(DevRows R, const DevLevel *lev0, int corr, double *tmp) {
+k_rows(DevRows R, const __grid_constant__ Lev<ONE> A, int corr, double *tmp) {
   const int r = blockIdx.x * CELL_BLOCK + threadIdx.x;
   if (r >= R.n) return;
-  const DevLevel &L = lev0[R.prob[r]];
+  const DevLevel &L = level(A, ONE ? 0 : R.prob[r]);
   auto x = PrecOf<T>::x(L);
   const long long b = R.cell[r], sy = L.sy, sz = L.sz;
   const long long o[8] = {0, sy, sy + 1, 1, sz, sz + sy, sz + sy + 1, sz + 1};
@@ -2333,24 +2377,68 @@ k_rows(DevRows R, const DevLevel *lev0, int corr, double *tmp) {
   tmp[r] = acc + c;
 }
 
-template <typename T>
+template <typename T, bool ONE>
 __global__ void __launch_bounds__(CELL_BLOCK)
-k_rows_scatter(DevRows R, const DevLevel *lev0, const double *tmp) {
+k_rows_scatter(DevRows R, const __grid_constant__ Lev<ONE> A, const double *tmp) {
   const int r = blockIdx.x * CELL_BLOCK + threadIdx.x;
   if (r >= R.n) return;
-  const DevLevel &L = lev0[R.prob[r]];
+  const DevLevel &L = level(A, ONE ? 0 : R.prob[r]);
   PrecOf<T>::x(L)[R.tgt[r]] = (T)tmp[r];
 }
 
+// Both steps of up to RC_MAX rows in one launch: one cluster of blocks forms
+// the values of all rows in registers, meets at the cluster barrier and
+// writes them.  The two launches each cost their start and a chain of
+// dependent reads for a few thousand rows: 4.4 + 3.1 us under ncu for 1376
+// rows in FP64, 4.8 us for this one.
+constexpr int RC_BLOCKS = 8, RC_THREADS = 512, RC_KEEP = 4;
+constexpr int RC_MAX = RC_BLOCKS * RC_THREADS * RC_KEEP;
+template <typename T, bool ONE>
+__global__ void __cluster_dims__(RC_BLOCKS, 1, 1) __launch_bounds__(RC_THREADS)
+k_rows_cluster(DevRows R, const __grid_constant__ Lev<ONE> A, int corr) {
+  T v[RC_KEEP];
+  long long t[RC_KEEP];
+  int pr[RC_KEEP];
+#pragma unroll
+  for (int u = 0; u < RC_KEEP; ++u) {
+    const int r = (u * RC_BLOCKS + (int)blockIdx.x) * RC_THREADS + (int)threadIdx.x;
+    if (r >= R.n) continue;
+    pr[u] = ONE ? 0 : R.prob[r];
+    const DevLevel &L = level(A, pr[u]);
+    auto x = PrecOf<T>::x(L);
+    const long long b = R.cell[r], sy = L.sy, sz = L.sz;
+    const long long o[8] = {0, sy, sy + 1, 1, sz, sz + sy, sz + sy + 1, sz + 1};
+    double acc = 0.0;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) acc += R.w[8 * r + q] * (double)x[b + o[q]];
+    const double c = !corr ? R.c0[r] : sizeof(T) == 4 ? (double)R.rf[r] : R.rd[r];
+    v[u] = (T)(acc + c);
+    t[u] = R.tgt[r];
+  }
+  asm volatile("barrier.cluster.arrive;\n\tbarrier.cluster.wait;" ::: "memory");
+#pragma unroll
+  for (int u = 0; u < RC_KEEP; ++u) {
+    const int r = (u * RC_BLOCKS + (int)blockIdx.x) * RC_THREADS + (int)threadIdx.x;
+    if (r < R.n) PrecOf<T>::x(level(A, pr[u]))[t[u]] = v[u];
+  }
+}
+
 template <typename T>
-cudaError_t rows_relax(const DevRows &R, const DevLevel *lev0, int corr, double *tmp,
-                       cudaStream_t s) {
+cudaError_t rows_relax(const DevRows &R, const Launch &L0, int corr, double *tmp, cudaStream_t s) {
   if (R.n <= 0) return cudaSuccess;
+  if (R.n <= RC_MAX) {
+    by_form(L0, [&](auto one) {
+      k_rows_cluster<T, one.value><<<RC_BLOCKS, RC_THREADS, 0, s>>>(R, lev_of<one.value>(L0), corr);
+    });
+    note_launches(1);
+    return cudaGetLastError();
+  }
   const int nb = (R.n + CELL_BLOCK - 1) / CELL_BLOCK;
-  k_rows<T><<<nb, CELL_BLOCK, 0, s>>>(R, lev0, corr, tmp);
-  note_launches(1);
-  k_rows_scatter<T><<<nb, CELL_BLOCK, 0, s>>>(R, lev0, tmp);
-  note_launches(1);
+  by_form(L0, [&](auto one) {
+    k_rows<T, one.value><<<nb, CELL_BLOCK, 0, s>>>(R, lev_of<one.value>(L0), corr, tmp);
+    k_rows_scatter<T, one.value><<<nb, CELL_BLOCK, 0, s>>>(R, lev_of<one.value>(L0), tmp);
+  });
+  note_launches(2);
   return cudaGetLastError();
 }
 
@@ -3544,13 +3632,12 @@ __device__ __forceinline__ KSel kidx(const KCtl *ctl, int ph, KSel s) {
 // V_vd = F - A P on active rows, 0 on every other interior cell; part[b] =
 // block sum of the squared active-row residuals (fluid-row norm).  Per quad
 // (4 cells of a row per thread, vector loads), FP64 arithmetic.
-template <typename B>
+template <typename B, bool ONE>
 __global__ void __launch_bounds__(QBLOCK)
-k_kr_resid(const int *FG_RESTRICT off, int nent, const DevLevel *FG_RESTRICT levs, const KDesc *kd, int vd, double *part) {
-  const int p = find_entry(off, nent, blockIdx.x);
-  const DevLevel &L = levs[p];
-  const int lb = blockIdx.x - off[p];
-  const KDesc &d = kd[p];
+k_kr_resid(const __grid_constant__ Lev<ONE> A, const __grid_constant__ Kry<ONE> K, int vd, double *part) {
+  int p, lb;
+  const DevLevel &L = entry(A, p, lb);
+  const KDesc &d = krylov(K, p);
   auto P = glob(mkptr<const double>(d.P, d.n, K_X));
   auto F = glob(mkptr<const double>(d.F, d.n, K_RHS));
   auto D = kvec<B>(d, d.V, vd);
@@ -3592,15 +3679,14 @@ k_kr_resid(const int *FG_RESTRICT off, int nent, const DevLevel *FG_RESTRICT lev
 // cells of a row per thread, vector loads), in the FP64 arithmetic of
 // apply_row_d.  x_T is zero on the pure-solid cells an active row may
 // couple to (they are held at the staged zero), so A x_T equals A Z_vz.
-template <typename B, typename T>
+template <typename B, typename T, bool ONE>
 __global__ void __launch_bounds__(QBLOCK)
-k_kr_apply_q(const int *FG_RESTRICT off, int nent, const DevLevel *FG_RESTRICT levs, const KDesc *kd, int vz, int vw,
+k_kr_apply_q(const __grid_constant__ Lev<ONE> A, const __grid_constant__ Kry<ONE> K, int vz, int vw,
              const KCtl *ctl) {
   if (ctl) { vz = ctl->j; vw = ctl->j + 1; }
-  const int p = find_entry(off, nent, blockIdx.x);
-  const DevLevel &L = levs[p];
-  const int lb = blockIdx.x - off[p];
-  const KDesc &d = kd[p];
+  int p, lb;
+  const DevLevel &L = entry(A, p, lb);
+  const KDesc &d = krylov(K, p);
   auto x = PrecOf<T>::x(L);
   auto Z = kvec<B>(d, d.Z, vz);
   auto W = kvec<B>(d, d.V, vw);
@@ -3647,9 +3733,9 @@ k_kr_apply_q(const int *FG_RESTRICT off, int nent, const DevLevel *FG_RESTRICT l
 // row's residual in solution form), mode 1 -> V_vd[t] = Z_vs[t] - sum w
 // Z_vs[corner] (the row of A), mode 2 -> correction constants of the
 // preconditioner: rd = rf = V_vs[t]
-template <typename B>
+template <typename B, bool ONE>
 __global__ void __launch_bounds__(CELL_BLOCK)
-k_kr_rows(DevRows R, const DevLevel *lev0, const KDesc *kd, int mode, int vs, int vd, const KCtl *ctl,
+k_kr_rows(DevRows R, const __grid_constant__ Lev<ONE> A, const __grid_constant__ Kry<ONE> K, int mode, int vs, int vd, const KCtl *ctl,
           int ph) {
   if (ctl) {
     if (mode == 1) { vs = ctl->j; vd = ctl->j + 1; }
@@ -3660,9 +3746,9 @@ k_kr_rows(DevRows R, const DevLevel *lev0, const KDesc *kd, int mode, int vs, in
   }
   const int r = blockIdx.x * CELL_BLOCK + threadIdx.x;
   if (r >= R.n) return;
-  const int p = R.prob[r];
-  const DevLevel &L = lev0[p];
-  const KDesc &d = kd[p];
+  const int p = ONE ? 0 : R.prob[r];
+  const DevLevel &L = level(A, p);
+  const KDesc &d = krylov(K, p);
   const long long t = R.tgt[r];
   if (mode == 2) {
     const B v = kvec<B>(d, d.V, vs)[t];
@@ -3705,18 +3791,18 @@ __device__ __forceinline__ long long flat_end(long long n) { return 1 + 4 * ((n 
 
 // block partials of (V_vw, V_i) for i < nv and of (V_vw, V_vw):
 // part[i * nblk + b], part[nv * nblk + b]
-template <typename B>
+template <typename B, bool ONE>
 __global__ void __launch_bounds__(FLAT_THREADS)
-k_kr_dots(const int *off, int nent, const KDesc *kd, int vw, int nv, int nblk, double *part,
+k_kr_dots(const __grid_constant__ Lev<ONE> A, const __grid_constant__ Kry<ONE> K, int vw, int nv, int nblk, double *part,
           const KCtl *ctl, int ph) {
   {
     const KSel ks = kidx(ctl, ph, KSel{0, vw, nv, 0, 0, 0, 0});
     vw = ks.vw;
     nv = ks.nv;
   }
-  const int p = find_entry(off, nent, blockIdx.x);
-  const int lb = blockIdx.x - off[p];
-  const KDesc &d = kd[p];
+  int p, lb;
+  entry(A, p, lb);
+  const KDesc &d = krylov(K, p);
   const long long lim = flat_end(d.n);
   B w[FLAT_PPT][4];
   bool ok[FLAT_PPT];
@@ -3801,17 +3887,17 @@ k_kr_reduce(const int *off, const double *part, int nblk, double *out, int ostri
 
 // V_vd = c0 V_vd + sum_{i<ns} c_{1+i} V_{s0+i} (FP64 arithmetic); with
 // stage, rhs_T = V_vd on active rows (0 elsewhere) and x_T = 0
-template <typename B, typename T>
+template <typename B, typename T, bool ONE>
 __global__ void __launch_bounds__(FLAT_THREADS)
-k_kr_vaxpy(const int *FG_RESTRICT off, int nent, const DevLevel *FG_RESTRICT levs, const KDesc *kd, int vd, int s0, int ns,
+k_kr_vaxpy(const __grid_constant__ Lev<ONE> A, const __grid_constant__ Kry<ONE> K, int vd, int s0, int ns,
            const double *coef, int cs, int stage, const KCtl *ctl, int ph) {
   {
     const KSel ks = kidx(ctl, ph, KSel{0, 0, 0, vd, s0, ns, stage});
     vd = ks.vd; s0 = ks.s0; ns = ks.ns; stage = ks.stage;
   }
-  const int p = find_entry(off, nent, blockIdx.x);
-  const int lb = blockIdx.x - off[p];
-  const KDesc &d = kd[p];
+  int p, lb;
+  const DevLevel &L = entry(A, p, lb);
+  const KDesc &d = krylov(K, p);
   const long long lim = flat_end(d.n);
   const double *cf = coef + (size_t)p * cs;
   auto D = kvec<B>(d, d.V, vd);
@@ -3845,7 +3931,6 @@ k_kr_vaxpy(const int *FG_RESTRICT off, int nent, const DevLevel *FG_RESTRICT lev
 #pragma unroll
       for (int q = 0; q < 4; ++q) acc[u][q] += ci * (double)v[u][q];
   }
-  const DevLevel &L = levs[p];
 #pragma unroll
   for (int u = 0; u < FLAT_PPT; ++u) {
     if (!ok[u]) continue;
@@ -3867,15 +3952,15 @@ k_kr_vaxpy(const int *FG_RESTRICT off, int nent, const DevLevel *FG_RESTRICT lev
 }
 
 // P += sum_{i<ns} c_{1+i} Z_i (c_0 is 1)
-template <typename B>
+template <typename B, bool ONE>
 __global__ void __launch_bounds__(FLAT_THREADS)
-k_kr_update(const int *off, int nent, const KDesc *kd, int ns, const double *coef, int cs,
+k_kr_update(const __grid_constant__ Lev<ONE> A, const __grid_constant__ Kry<ONE> K, int ns, const double *coef, int cs,
             const KCtl *ctl) {
   if (ctl) ns = ctl->jlast;
   if (ns == 0) return;
-  const int p = find_entry(off, nent, blockIdx.x);
-  const int lb = blockIdx.x - off[p];
-  const KDesc &d = kd[p];
+  int p, lb;
+  entry(A, p, lb);
+  const KDesc &d = krylov(K, p);
   const long long lim = flat_end(d.n);
   const double *cf = coef + (size_t)p * cs;
   auto P = glob(mkptr<double>(d.P, d.n, K_X));
@@ -3904,155 +3989,172 @@ k_kr_update(const int *off, int nent, const KDesc *kd, int ns, const double *coe
     if (ok[u]) store_run<double, 4>(P, flat_elem(lb, u), acc[u], 4);
 }
 
-static int rows_blocks(const DevRows &R) { return (R.n + CELL_BLOCK - 1) / CELL_BLOCK; }
+template <typename B>
+static void kr_rows(const Launch &L, const DevRows &R, const KrySet &kd, int mode, int vs, int vd, const KCtl *ctl, int ph,
+                    cudaStream_t s) {
+  const int nb = (R.n + CELL_BLOCK - 1) / CELL_BLOCK;
+  by_form(L, [&](auto one) {
+    k_kr_rows<B, one.value><<<nb, CELL_BLOCK, 0, s>>>(R, lev_of<one.value>(L), kry_of<one.value>(kd), mode, vs, vd, ctl, ph);
+  });
+}
 
 template <typename B>
-cudaError_t kr_resid(const Launch &quads, const DevRows &R, const DevLevel *lev0, const KDesc *kd, int vd,
+cudaError_t kr_resid(const Launch &quads, const DevRows &R, const KrySet &kd, int vd,
                      double *part, double *norm2, cudaStream_t s) {
   if (quads.empty()) return cudaSuccess;
-  k_kr_resid<B><<<quads.blocks, QBLOCK, 0, s>>>(quads.off, quads.n, quads.lev, kd, vd, part);
+  by_form(quads, [&](auto one) {
+    k_kr_resid<B, one.value><<<quads.blocks, QBLOCK, 0, s>>>(lev_of<one.value>(quads), kry_of<one.value>(kd), vd, part);
+  });
   k_reduce_parts<<<quads.n, 1024, 0, s>>>(quads.off, part, norm2);
   note_launches(2);
   if (R.n > 0) {
-    k_kr_rows<B><<<rows_blocks(R), CELL_BLOCK, 0, s>>>(R, lev0, kd, 0, 0, vd, nullptr, 0);
+    kr_rows<B>(quads, R, kd, 0, 0, vd, nullptr, 0, s);
     note_launches(1);
   }
   return cudaGetLastError();
 }
 
 template <typename B, typename T>
-cudaError_t kr_apply(const Launch &quads, const DevRows &R, const DevLevel *lev0, const KDesc *kd, int vz,
+cudaError_t kr_apply(const Launch &quads, const DevRows &R, const KrySet &kd, int vz,
                      int vw, cudaStream_t s) {
   if (quads.empty()) return cudaSuccess;
-  k_kr_apply_q<B, T><<<quads.blocks, QBLOCK, 0, s>>>(quads.off, quads.n, quads.lev, kd, vz, vw, nullptr);
+  by_form(quads, [&](auto one) {
+    k_kr_apply_q<B, T, one.value><<<quads.blocks, QBLOCK, 0, s>>>(lev_of<one.value>(quads), kry_of<one.value>(kd), vz, vw, nullptr);
+  });
   note_launches(1);
   if (R.n > 0) {
-    k_kr_rows<B><<<rows_blocks(R), CELL_BLOCK, 0, s>>>(R, lev0, kd, 1, vz, vw, nullptr, 0);
+    kr_rows<B>(quads, R, kd, 1, vz, vw, nullptr, 0, s);
     note_launches(1);
   }
   return cudaGetLastError();
 }
 
 template <typename B>
-cudaError_t kr_dots(const Launch &flat, const KDesc *kd, int vw, int nv, double *part, double *out,
+cudaError_t kr_dots(const Launch &flat, const KrySet &kd, int vw, int nv, double *part, double *out,
                     int ostride, cudaStream_t s) {
   if (flat.empty()) return cudaSuccess;
   if (nv > KR_MAXV) return cudaErrorInvalidValue;
-  k_kr_dots<B><<<flat.blocks, FLAT_THREADS, 0, s>>>(flat.off, flat.n, kd, vw, nv, flat.blocks, part,
-                                                    nullptr, 0);
+  by_form(flat, [&](auto one) {
+    k_kr_dots<B, one.value><<<flat.blocks, FLAT_THREADS, 0, s>>>(lev_of<one.value>(flat), kry_of<one.value>(kd), vw, nv, flat.blocks, part, nullptr, 0);
+  });
   k_kr_reduce<<<dim3(flat.n, nv + 1), 256, 0, s>>>(flat.off, part, flat.blocks, out, ostride, nullptr, 0);
   note_launches(2);
   return cudaGetLastError();
 }
 
 template <typename B, typename T>
-cudaError_t kr_vaxpy(const Launch &flat, const DevRows &R, const DevLevel *lev0, const KDesc *kd, int vd,
+cudaError_t kr_vaxpy(const Launch &flat, const DevRows &R, const KrySet &kd, int vd,
                      int s0, int ns, const double *coef, int cs, bool stage, cudaStream_t s) {
   if (flat.empty()) return cudaSuccess;
   if (ns > KR_MAXV) return cudaErrorInvalidValue;
-  k_kr_vaxpy<B, T><<<flat.blocks, FLAT_THREADS, 0, s>>>(flat.off, flat.n, flat.lev, kd, vd, s0, ns, coef,
-                                                        cs, stage ? 1 : 0, nullptr, 0);
+  by_form(flat, [&](auto one) {
+    k_kr_vaxpy<B, T, one.value><<<flat.blocks, FLAT_THREADS, 0, s>>>(lev_of<one.value>(flat), kry_of<one.value>(kd), vd, s0, ns, coef, cs, stage ? 1 : 0, nullptr, 0);
+  });
   note_launches(1);
   if (stage && R.n > 0) {
-    k_kr_rows<B><<<rows_blocks(R), CELL_BLOCK, 0, s>>>(R, lev0, kd, 2, vd, vd, nullptr, 0);
+    kr_rows<B>(flat, R, kd, 2, vd, vd, nullptr, 0, s);
     note_launches(1);
   }
   return cudaGetLastError();
 }
 
 template <typename B>
-cudaError_t kr_update(const Launch &flat, const KDesc *kd, int ns, const double *coef, int cs,
+cudaError_t kr_update(const Launch &flat, const KrySet &kd, int ns, const double *coef, int cs,
                       cudaStream_t s) {
   if (flat.empty() || ns == 0) return cudaSuccess;
   if (ns > KR_MAXV) return cudaErrorInvalidValue;
-  k_kr_update<B><<<flat.blocks, FLAT_THREADS, 0, s>>>(flat.off, flat.n, kd, ns, coef, cs, nullptr);
+  by_form(flat, [&](auto one) {
+    k_kr_update<B, one.value><<<flat.blocks, FLAT_THREADS, 0, s>>>(lev_of<one.value>(flat), kry_of<one.value>(kd), ns, coef, cs, nullptr);
+  });
   note_launches(1);
   return cudaGetLastError();
 }
 
-template cudaError_t kr_resid<float>(const Launch &, const DevRows &, const DevLevel *, const KDesc *, int,
+template cudaError_t kr_resid<float>(const Launch &, const DevRows &, const KrySet &, int,
                                      double *, double *, cudaStream_t);
-template cudaError_t kr_resid<double>(const Launch &, const DevRows &, const DevLevel *, const KDesc *, int,
+template cudaError_t kr_resid<double>(const Launch &, const DevRows &, const KrySet &, int,
                                       double *, double *, cudaStream_t);
-template cudaError_t kr_apply<float, float>(const Launch &, const DevRows &, const DevLevel *, const KDesc *,
+template cudaError_t kr_apply<float, float>(const Launch &, const DevRows &, const KrySet &,
                                             int, int, cudaStream_t);
-template cudaError_t kr_apply<double, double>(const Launch &, const DevRows &, const DevLevel *,
-                                              const KDesc *, int, int, cudaStream_t);
-template cudaError_t kr_dots<float>(const Launch &, const KDesc *, int, int, double *, double *, int,
+template cudaError_t kr_apply<double, double>(const Launch &, const DevRows &, const KrySet &, int, int, cudaStream_t);
+template cudaError_t kr_dots<float>(const Launch &, const KrySet &, int, int, double *, double *, int,
                                     cudaStream_t);
-template cudaError_t kr_dots<double>(const Launch &, const KDesc *, int, int, double *, double *, int,
+template cudaError_t kr_dots<double>(const Launch &, const KrySet &, int, int, double *, double *, int,
                                      cudaStream_t);
-template cudaError_t kr_vaxpy<float, float>(const Launch &, const DevRows &, const DevLevel *, const KDesc *,
+template cudaError_t kr_vaxpy<float, float>(const Launch &, const DevRows &, const KrySet &,
                                             int, int, int, const double *, int, bool, cudaStream_t);
-template cudaError_t kr_vaxpy<double, double>(const Launch &, const DevRows &, const DevLevel *,
-                                              const KDesc *, int, int, int, const double *, int, bool,
+template cudaError_t kr_vaxpy<double, double>(const Launch &, const DevRows &, const KrySet &, int, int, int, const double *, int, bool,
                                               cudaStream_t);
-template cudaError_t kr_update<float>(const Launch &, const KDesc *, int, const double *, int, cudaStream_t);
-template cudaError_t kr_update<double>(const Launch &, const KDesc *, int, const double *, int, cudaStream_t);
+template cudaError_t kr_update<float>(const Launch &, const KrySet &, int, const double *, int, cudaStream_t);
+template cudaError_t kr_update<double>(const Launch &, const KrySet &, int, const double *, int, cudaStream_t);
 
 // ---- the same passes with their indices read on the device (phase KPH_*)
 template <typename B, typename T>
-cudaError_t krd_apply(const Launch &quads, const DevRows &R, const DevLevel *lev0, const KDesc *kd,
+cudaError_t krd_apply(const Launch &quads, const DevRows &R, const KrySet &kd,
                       const KCtl *ctl, cudaStream_t s) {
   if (quads.empty()) return cudaSuccess;
-  k_kr_apply_q<B, T><<<quads.blocks, QBLOCK, 0, s>>>(quads.off, quads.n, quads.lev, kd, 0, 0, ctl);
+  by_form(quads, [&](auto one) {
+    k_kr_apply_q<B, T, one.value><<<quads.blocks, QBLOCK, 0, s>>>(lev_of<one.value>(quads), kry_of<one.value>(kd), 0, 0, ctl);
+  });
   note_launches(1);
   if (R.n > 0) {
-    k_kr_rows<B><<<rows_blocks(R), CELL_BLOCK, 0, s>>>(R, lev0, kd, 1, 0, 0, ctl, KPH_APPLY);
+    kr_rows<B>(quads, R, kd, 1, 0, 0, ctl, KPH_APPLY, s);
     note_launches(1);
   }
   return cudaGetLastError();
 }
 
 template <typename B>
-cudaError_t krd_dots(const Launch &flat, const KDesc *kd, const KCtl *ctl, int phase, double *part,
+cudaError_t krd_dots(const Launch &flat, const KrySet &kd, const KCtl *ctl, int phase, double *part,
                      double *out, cudaStream_t s) {
   if (flat.empty()) return cudaSuccess;
-  k_kr_dots<B><<<flat.blocks, FLAT_THREADS, 0, s>>>(flat.off, flat.n, kd, 0, 0, flat.blocks, part, ctl,
-                                                    phase);
+  by_form(flat, [&](auto one) {
+    k_kr_dots<B, one.value><<<flat.blocks, FLAT_THREADS, 0, s>>>(lev_of<one.value>(flat), kry_of<one.value>(kd), 0, 0, flat.blocks, part, ctl, phase);
+  });
   k_kr_reduce<<<dim3(flat.n, KR_MAXV + 1), 256, 0, s>>>(flat.off, part, flat.blocks, out, KR_CS, ctl, phase);
   note_launches(2);
   return cudaGetLastError();
 }
 
 template <typename B, typename T>
-cudaError_t krd_vaxpy(const Launch &flat, const DevRows &R, const DevLevel *lev0, const KDesc *kd,
+cudaError_t krd_vaxpy(const Launch &flat, const DevRows &R, const KrySet &kd,
                       const KCtl *ctl, int phase, const double *coef, cudaStream_t s) {
   if (flat.empty()) return cudaSuccess;
-  k_kr_vaxpy<B, T><<<flat.blocks, FLAT_THREADS, 0, s>>>(flat.off, flat.n, flat.lev, kd, 0, 0, 0, coef, KR_CS,
-                                                        0, ctl, phase);
+  by_form(flat, [&](auto one) {
+    k_kr_vaxpy<B, T, one.value><<<flat.blocks, FLAT_THREADS, 0, s>>>(lev_of<one.value>(flat), kry_of<one.value>(kd), 0, 0, 0, coef, KR_CS, 0, ctl, phase);
+  });
   note_launches(1);
   if (phase != KPH_REORTH && R.n > 0) {  // staged row constants (skipped on the device when not staged)
-    k_kr_rows<B><<<rows_blocks(R), CELL_BLOCK, 0, s>>>(R, lev0, kd, 2, 0, 0, ctl, phase);
+    kr_rows<B>(flat, R, kd, 2, 0, 0, ctl, phase, s);
     note_launches(1);
   }
   return cudaGetLastError();
 }
 
 template <typename B>
-cudaError_t krd_update(const Launch &flat, const KDesc *kd, const KCtl *ctl, const double *coef,
+cudaError_t krd_update(const Launch &flat, const KrySet &kd, const KCtl *ctl, const double *coef,
                        cudaStream_t s) {
   if (flat.empty()) return cudaSuccess;
-  k_kr_update<B><<<flat.blocks, FLAT_THREADS, 0, s>>>(flat.off, flat.n, kd, 0, coef, KR_CS, ctl);
+  by_form(flat, [&](auto one) {
+    k_kr_update<B, one.value><<<flat.blocks, FLAT_THREADS, 0, s>>>(lev_of<one.value>(flat), kry_of<one.value>(kd), 0, coef, KR_CS, ctl);
+  });
   note_launches(1);
   return cudaGetLastError();
 }
 
-template cudaError_t krd_apply<float, float>(const Launch &, const DevRows &, const DevLevel *, const KDesc *,
+template cudaError_t krd_apply<float, float>(const Launch &, const DevRows &, const KrySet &,
                                              const KCtl *, cudaStream_t);
-template cudaError_t krd_apply<double, double>(const Launch &, const DevRows &, const DevLevel *,
-                                               const KDesc *, const KCtl *, cudaStream_t);
-template cudaError_t krd_dots<float>(const Launch &, const KDesc *, const KCtl *, int, double *, double *,
+template cudaError_t krd_apply<double, double>(const Launch &, const DevRows &, const KrySet &, const KCtl *, cudaStream_t);
+template cudaError_t krd_dots<float>(const Launch &, const KrySet &, const KCtl *, int, double *, double *,
                                      cudaStream_t);
-template cudaError_t krd_dots<double>(const Launch &, const KDesc *, const KCtl *, int, double *, double *,
+template cudaError_t krd_dots<double>(const Launch &, const KrySet &, const KCtl *, int, double *, double *,
                                       cudaStream_t);
-template cudaError_t krd_vaxpy<float, float>(const Launch &, const DevRows &, const DevLevel *, const KDesc *,
+template cudaError_t krd_vaxpy<float, float>(const Launch &, const DevRows &, const KrySet &,
                                              const KCtl *, int, const double *, cudaStream_t);
-template cudaError_t krd_vaxpy<double, double>(const Launch &, const DevRows &, const DevLevel *,
-                                               const KDesc *, const KCtl *, int, const double *, cudaStream_t);
-template cudaError_t krd_update<float>(const Launch &, const KDesc *, const KCtl *, const double *,
+template cudaError_t krd_vaxpy<double, double>(const Launch &, const DevRows &, const KrySet &, const KCtl *, int, const double *, cudaStream_t);
+template cudaError_t krd_update<float>(const Launch &, const KrySet &, const KCtl *, const double *,
                                        cudaStream_t);
-template cudaError_t krd_update<double>(const Launch &, const KDesc *, const KCtl *, const double *,
+template cudaError_t krd_update<double>(const Launch &, const KrySet &, const KCtl *, const double *,
                                         cudaStream_t);
 
 // ---- scalar FGMRES steps: one block, problem p on thread p (mod 256)
@@ -4306,15 +4408,15 @@ template cudaError_t line_sweep<float>(const Launch &, int, int, double, int, in
 template cudaError_t residual<double>(const Launch &, double *, double *, cudaStream_t);
 template cudaError_t residual_q<double>(const Launch &, cudaStream_t);
 template cudaError_t residual_q<float>(const Launch &, cudaStream_t);
-template cudaError_t prolong_add<double>(const Launch &, const DevLevel *, cudaStream_t);
-template cudaError_t prolong_add<float>(const Launch &, const DevLevel *, cudaStream_t);
+template cudaError_t prolong_add<double>(const Launch &, const Launch &, cudaStream_t);
+template cudaError_t prolong_add<float>(const Launch &, const Launch &, cudaStream_t);
 template cudaError_t residual<float>(const Launch &, double *, double *, cudaStream_t);
-template cudaError_t restrict_to<double>(const Launch &, const DevLevel *, cudaStream_t);
-template cudaError_t restrict_to<float>(const Launch &, const DevLevel *, cudaStream_t);
+template cudaError_t restrict_to<double>(const Launch &, const Launch &, cudaStream_t);
+template cudaError_t restrict_to<float>(const Launch &, const Launch &, cudaStream_t);
 template cudaError_t zero_x<float>(const Launch &, cudaStream_t);
-template cudaError_t rows_relax<double>(const DevRows &, const DevLevel *, int, double *,
+template cudaError_t rows_relax<double>(const DevRows &, const Launch &, int, double *,
                                         cudaStream_t);
-template cudaError_t rows_relax<float>(const DevRows &, const DevLevel *, int, double *,
+template cudaError_t rows_relax<float>(const DevRows &, const Launch &, int, double *,
                                        cudaStream_t);
 template cudaError_t coarsest_solve<double>(int, const DevLevel *, const double *const *,
                                             const int *const *, const int *, int, cudaStream_t);
