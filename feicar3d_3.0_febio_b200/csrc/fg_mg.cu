@@ -1242,8 +1242,10 @@ int blocks_cells(const DevLevel &L) {
 int xline_lanes(int maxn) { return maxn <= 16 ? 4 : maxn <= 32 ? 8 : maxn <= 64 ? 16 : 32; }
 // The line kernel family a level set's sweep along `axis` takes (LV_*):
 // the requested one when it can take lines of maxn cells, else the
-// default (the family measured fastest for that line length on the
-// 512x256x256 case).
+// default: the family measured fastest for that line length.  Short y/z lines
+// take the block-PCR tiles too (per sweep against the register tiles, B200:
+// 64 rows of 128x64x64 cells FP32 14.4 and 16.7 us, 49 rows of 101x49x38 12.6
+// and 15.3, the 56-row levels of 16 cubes 20.8 and 37.1, in FP64 29.0 and 50.2).
 int line_variant(int axis, int maxn, int v) {
   if (axis == 0) {
     if (v == LV_XREG && maxn > 128) v = LV_DEFAULT;
@@ -1256,7 +1258,7 @@ int line_variant(int axis, int maxn, int v) {
   if ((v == LV_YREG || pcr) && maxn > YZ_MAXROWS) v = LV_DEFAULT;
   if (pcr && v != LV_YPCR && v != LV_YWAVE && maxn < YP_MINROWS) v = LV_DEFAULT;
   if (v != LV_YREG && v != LV_YWARP && !pcr)
-    v = (maxn >= YP_MINROWS && maxn <= YZ_MAXROWS) ? LV_YPCR : maxn <= YZ_MAXROWS ? LV_YREG : LV_YWARP;
+    v = maxn <= YZ_MAXROWS ? LV_YPCR : LV_YWARP;
   return v;
 }
 int blocks_xline(const DevLevel &L, int maxn, int variant) {
@@ -1770,7 +1772,7 @@ cudaError_t line_sweep(const Launch &Lr, int axis, int color, double omega, int 
     if (maxn <= 1024) return launch_xsmem<T, 32>(Lr, color, omega, s);
     return cudaErrorInvalidValue;  // lines longer than 1024 cells
   }
-  if (v == LV_YPCR) {  // lines shorter than YP_MINROWS only when chosen (autotuner)
+  if (v == LV_YPCR) {
     if (maxn <= 32) return launch_yzpcr<T, 4, 8>(Lr, axis, color, omega, s);
     if (maxn <= 64) return launch_yzpcr<T, 4, 16>(Lr, axis, color, omega, s);
     if (maxn <= 128) return launch_yzpcr<T, 8, 16>(Lr, axis, color, omega, s);
