@@ -516,8 +516,8 @@ struct fg_batch {
     DevLevel *d_levS_next = nullptr;  // level L+1 of S
     DevLevel *d_levC = nullptr;       // level L of C
     int *d_off_cells = nullptr, *d_off_x = nullptr, *d_off_y = nullptr, *d_off_z = nullptr,
-        *d_off_next = nullptr, *d_off_quads = nullptr;
-    Launch cells, xl, yl, zl, next, quads;
+        *d_off_next = nullptr, *d_off_pairs = nullptr, *d_off_quads = nullptr;
+    Launch cells, xl, yl, zl, next, quads, pairs;
     int maxnx = 0, maxny = 0, maxnz = 0;
     double ncells = 0.0;  // cells of level L summed over S
     const double **d_G = nullptr;
@@ -634,7 +634,7 @@ static void free_batch_tables(fg_batch *b) {
     auto &s = b->ls[L];
     fg::dev_free(s.d_levS); fg::dev_free(s.d_levS_next); fg::dev_free(s.d_levC);
     fg::dev_free(s.d_off_cells); fg::dev_free(s.d_off_x); fg::dev_free(s.d_off_y); fg::dev_free(s.d_off_z);
-    fg::dev_free(s.d_off_next); fg::dev_free(s.d_off_quads); fg::dev_free(s.d_G); fg::dev_free(s.d_gidx); fg::dev_free(s.d_gn);
+    fg::dev_free(s.d_off_next); fg::dev_free(s.d_off_quads); fg::dev_free(s.d_off_pairs); fg::dev_free(s.d_G); fg::dev_free(s.d_gidx); fg::dev_free(s.d_gn);
     s = fg_batch::LevelSet();
   }
   fg::dev_free(b->d_lev0); fg::dev_free(b->d_off0); fg::dev_free(b->d_offf0); fg::dev_free(b->d_offq0);
@@ -890,7 +890,8 @@ static fg_status build_batch(fg_batch *b) {
   for (int L = 0; L < b->maxdepth; ++L) {
     auto &s = b->ls[L];
     std::vector<DevLevel> vS, vSn, vC;
-    std::vector<int> bc, bx, by, bz, bn, bq;
+    std::vector<int> bc, bx, by, bz, bn, bq, br;
+    bool halved = true;
     for (int p = 0; p < np; ++p) {
       const fg_case *c = b->cases[p];
       if (L < c->nlev - 1) {
@@ -912,6 +913,8 @@ static fg_status build_batch(fg_batch *b) {
         bz.push_back(k::blocks_tile(d, 2, s.maxnz, b->tune.var[L][2]));
         bn.push_back(k::blocks_cells(c->lev[L + 1].dl));
         bq.push_back(k::blocks_quads(d));
+        br.push_back(k::blocks_restrict(d, c->lev[L + 1].dl));
+        halved = halved && k::restrict_fits(d, c->lev[L + 1].dl);
         s.ncells += (double)d.nx * d.ny * d.nz;
       } else if (L == c->nlev - 1) {
         s.C.push_back(p);
@@ -929,6 +932,7 @@ static fg_status build_batch(fg_batch *b) {
       if ((st = build_offsets(bz, &s.d_off_z, s.zl, s.d_levS, vS, true)) != FG_OK) return st;
       if ((st = build_offsets(bn, &s.d_off_next, s.next, s.d_levS_next, vSn)) != FG_OK) return st;
       if ((st = build_offsets(bq, &s.d_off_quads, s.quads, s.d_levS, vS)) != FG_OK) return st;
+      if (halved && (st = build_offsets(br, &s.d_off_pairs, s.pairs, s.d_levS, vS)) != FG_OK) return st;
     }
     if (!s.C.empty()) {
       FG_CUDA(fg::dev_alloc(&s.d_G, s.C.size() * sizeof(double *)));
@@ -1078,8 +1082,7 @@ static fg_status vcycle(fg_batch *b, cudaStream_t s) {
       for (int q = 0; q < nu_pre(b, L); ++q)
         if ((st = smooth<T>(b, L, s)) != FG_OK) return st;
       const size_t e0 = prof_begin(b, s);
-      FG_K(k::residual_q<T>(ls.quads, s));
-      FG_K(k::restrict_to<T>(ls.next, ls.quads, s));
+      FG_K(k::restrict_to<T>(ls.pairs, ls.quads, ls.next, s));
       prof_end(b, e0, FG_PROF_TRANSFER, 0.0, s);
     }
     if (!ls.C.empty()) {

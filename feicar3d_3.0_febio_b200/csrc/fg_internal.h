@@ -330,14 +330,16 @@ cudaError_t line_sweep(const Launch &L, int axis, int color, double omega, int m
 // norm2[p] += ||r||^2 of entry p when norm2 != null (part: one double per block)
 template <typename T>
 cudaError_t residual(const Launch &L, double *norm2, double *part, cudaStream_t s);
+// residual and restriction: one pass over the pairs of the coarse rows (Lr,
+// blocks_restrict) where every problem's level was halved along every axis
+// (restrict_fits); with Lr empty two passes, over the fine quads (Lq) and the
+// coarse cells (Lc).  The coarse unknown is cleared.
+int blocks_restrict(const DevLevel &F, const DevLevel &C);
+bool restrict_fits(const DevLevel &F, const DevLevel &C);
 template <typename T>
-cudaError_t restrict_to(const Launch &coarse_cells, const Launch &fine, cudaStream_t s);
+cudaError_t restrict_to(const Launch &Lr, const Launch &Lq, const Launch &Lc, cudaStream_t s);
 template <typename T>
 cudaError_t prolong_add(const Launch &fine, const Launch &coarse, cudaStream_t s);
-// the residual (no norm) with quads: Launch over the level's quads
-// (blocks_quads)
-template <typename T>
-cudaError_t residual_q(const Launch &quads, cudaStream_t s);
 template <typename T>
 cudaError_t zero_x(const Launch &L, cudaStream_t s);
 // shared memory a level of nx x ny x nz cells takes in cycle(), with or

@@ -2054,6 +2054,150 @@ struct QuadVals {
   }
 };
 
+// Four cells of i in two neighbouring rows j, j + 1 of a plane (the second
+// row may be missing at the level's end): the values of x there and around
+// them, each loaded once.
+template <typename T>
+struct PairVals {
+  T c[2][4], ym[4], yp[4], zm[2][4], zp[2][4], xl[2], xr[2];
+  bool two;
+  template <typename P>
+  __device__ __forceinline__ void load(const DevLevel &L, const P &x, int i0, int j, int k) {
+    const long long sy = L.sy, sz = L.sz, id = i0 + sy * j + sz * k;
+    two = j < L.ny;
+    const long long d = two ? sy : 0;
+    load_run<T, 4>(ym, x, id - sy);
+    load_run<T, 4>(c[0], x, id);
+    load_run<T, 4>(c[1], x, id + d);
+    load_run<T, 4>(yp, x, id + d + sy);
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      load_run<T, 4>(zm[r], x, id + r * d - sz);
+      load_run<T, 4>(zp[r], x, id + r * d + sz);
+      xl[r] = x[id + r * d - 1];
+      xr[r] = x[id + r * d + 4];
+    }
+  }
+  // neighbours of cell v of row r (faces -x,+x,-y,+y,-z,+z)
+  __device__ __forceinline__ void nbrs(int r, int v, T (&xn)[6]) const {
+    xn[0] = v == 0 ? xl[r] : c[r][v - 1];
+    xn[1] = v == 3 ? xr[r] : c[r][v + 1];
+    xn[2] = r == 0 ? ym[v] : c[0][v];
+    xn[3] = r == 0 && two ? c[1][v] : yp[v];
+    xn[4] = zm[r][v];
+    xn[5] = zp[r][v];
+  }
+};
+__device__ __forceinline__ bool all_coupled(const uint8_t (&m)[4]) {
+  uint32_t w;
+  memcpy(&w, m, 4);
+  return (w & 0x7f7f7f7fu) == 0x7f7f7f7fu;  // active, all six faces
+}
+
+// Blocks of 32 quads of i by PAIR_J row pairs of a plane: the pairs share
+// their neighbouring rows in L1
+constexpr int PAIR_J = QBLOCK / 32;
+struct PairIdx { int i0, pj, k; bool ok; };
+__device__ __forceinline__ PairIdx pair_of(int nx, int pairs, int nk, int lb) {
+  const int nseg = (nx + 127) / 128, npj = (pairs + PAIR_J - 1) / PAIR_J;
+  const int t = threadIdx.x, row = lb / nseg;
+  PairIdx p;
+  p.i0 = 1 + 4 * ((lb - row * nseg) * 32 + (t & 31));
+  p.k = 1 + row / npj;
+  p.pj = (row - (p.k - 1) * npj) * PAIR_J + (t >> 5);
+  p.ok = p.i0 <= nx && p.pj < pairs && p.k <= nk;
+  return p;
+}
+static int pair_blocks(int nx, int pairs, int nk) {
+  return (nx + 127) / 128 * ((pairs + PAIR_J - 1) / PAIR_J) * nk;
+}
+int blocks_restrict(const DevLevel &F, const DevLevel &C) { return pair_blocks(F.nx, C.ny, C.nz); }
+static bool halved(int nc, int nf) { return nc == (nf + 1) / 2 && nc < nf; }
+bool restrict_fits(const DevLevel &F, const DevLevel &C) {
+  return halved(C.nx, F.nx) && halved(C.ny, F.ny) && halved(C.nz, F.nz);
+}
+
+// Residual and restriction in one pass: coarse rhs = volume-weighted mean of
+// the children's residuals f - A x on active coarse cells (the sum of the
+// children's finite-volume equations; 0 on inactive children and coarse
+// cells), coarse x = 0.  For levels all of whose axes were halved (children 2 I
+// - 1 and min(2 I, n)): a thread takes two coarse cells, four fine cells of i
+// by two of j by two of k, and keeps their residuals in registers.  Bound by
+// the latency of its loads at 125 registers (43 % issue-active, 22 % of DRAM);
+// 512x256x256 FP32: 187 us, as two passes with the residual stored between
+// them 160 + 58.
+template <typename T, bool ONE>
+__global__ void __launch_bounds__(QBLOCK)
+k_res_restrict(const __grid_constant__ Lev<ONE> A, const __grid_constant__ Lev<ONE> CA) {
+  int p, lb;
+  const DevLevel &F = entry(A, p, lb);
+  const DevLevel &C = level(CA, p);
+  const PairIdx q = pair_of(F.nx, C.ny, C.nz, lb);
+  if (!q.ok) return;
+  const int J = 1 + q.pj, K = q.k, j = 2 * J - 1;
+  auto x = PrecOf<T>::x(F);
+  auto rhs = PrecOf<T>::rhs(F);
+  auto mask = glob(F.mask);
+  double wx[4], ax0[4], ax1[4], s[2] = {0.0, 0.0}, w[2] = {0.0, 0.0};
+#pragma unroll
+  for (int v = 0; v < 4; ++v) {
+    const int i = min(q.i0 + v, F.nx);
+    wx[v] = q.i0 + v <= F.nx ? glob(F.wx)[i] : 0.0;
+    ax0[v] = glob(F.amx)[i];
+    ax1[v] = glob(F.apx)[i];
+  }
+#pragma unroll
+  for (int kk = 0; kk < 2; ++kk) {
+    const int k = 2 * K - 1 + kk;
+    if (k > F.nz) break;
+    PairVals<T> xv;
+    xv.load(F, x, q.i0, j, k);
+    const long long id = q.i0 + F.sy * j + F.sz * k, d = xv.two ? F.sy : 0;
+    T f[2][4];
+    uint8_t m4[2][4];
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      load_run<T, 4>(f[r], rhs, id + r * d);
+      load_run<uint8_t, 4>(m4[r], mask, id + r * d);
+    }
+    const double az0 = glob(F.amz)[k], az1 = glob(F.apz)[k], wz = glob(F.wz)[k];
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      if (r == 1 && !xv.two) break;
+      const double ay0 = glob(F.amy)[j + r], ay1 = glob(F.apy)[j + r], wyz = glob(F.wy)[j + r] * wz;
+      const bool reg = all_coupled(m4[r]) && q.i0 + 3 <= F.nx;
+      const double dyz = -(ay0 + ay1 + az0 + az1);
+#pragma unroll
+      for (int v = 0; v < 4; ++v) {
+        T xn[6];
+        xv.nbrs(r, v, xn);
+        T rv = T(0);
+        if (reg) {
+          const T acc = (T)ax0[v] * xn[0] + (T)ax1[v] * xn[1] + (T)ay0 * xn[2] + (T)ay1 * xn[3] + (T)az0 * xn[4] +
+                        (T)az1 * xn[5];
+          rv = f[r][v] - (acc + (T)(dyz - (ax0[v] + ax1[v])) * xv.c[r][v]);
+        } else if (m4[r][v] & 64) {
+          const double a[6] = {ax0[v], ax1[v], ay0, ay1, az0, az1};
+          rv = f[r][v] - apply_vals<T>(F, q.i0 + v, j + r, k, m4[r][v], xv.c[r][v], xn, a);
+        }
+        const double wt = wx[v] * wyz;
+        s[v >> 1] += wt * (double)(q.i0 + v <= F.nx ? rv : T(0));
+        w[v >> 1] += wt;
+      }
+    }
+  }
+  auto rc = PrecOf<T>::rhs(C);
+  auto xc = PrecOf<T>::x(C);
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int I = (q.i0 + 1) / 2 + h;
+    if (I > C.nx) break;
+    const long long id = I + C.sy * J + C.sz * K;
+    rc[id] = glob(C.mask)[id] & 64 ? (T)(s[h] / w[h]) : T(0);
+    xc[id] = T(0);
+  }
+}
+
 // r = f - A x on active cells, 0 on the other interior cells (the V-cycle's
 // restriction input); the arithmetic of k_residual, per quad
 template <typename T, bool ONE>
@@ -2091,14 +2235,6 @@ k_residual_q(const __grid_constant__ Lev<ONE> A) {
     }
     store_run<T, 4>(res, id, out, L.nx - q.i0 + 1);
   }
-}
-
-template <typename T>
-cudaError_t residual_q(const Launch &Lq, cudaStream_t s) {
-  if (Lq.empty()) return cudaSuccess;
-  by_form(Lq, [&](auto one) { k_residual_q<T, one.value><<<Lq.blocks, QBLOCK, 0, s>>>(lev_of<one.value>(Lq)); });
-  note_launches(1);
-  return cudaGetLastError();
 }
 
 // ------------------------------------------------------- restriction
@@ -2170,12 +2306,20 @@ k_restrict(const __grid_constant__ Lev<ONE> A, const __grid_constant__ Lev<ONE> 
 }
 
 template <typename T>
-cudaError_t restrict_to(const Launch &Lc, const Launch &Lf, cudaStream_t s) {
-  if (Lc.empty()) return cudaSuccess;
-  by_form(Lc, [&](auto one) {
-    k_restrict<T, one.value><<<Lc.blocks, CELL_BLOCK, 0, s>>>(lev_of<one.value>(Lc), lev_of<one.value>(Lf));
+cudaError_t restrict_to(const Launch &Lr, const Launch &Lq, const Launch &Lc, cudaStream_t s) {
+  if (!Lr.empty()) {
+    by_form(Lr, [&](auto one) {
+      k_res_restrict<T, one.value><<<Lr.blocks, QBLOCK, 0, s>>>(lev_of<one.value>(Lr), lev_of<one.value>(Lc));
+    });
+    note_launches(1);
+    return cudaGetLastError();
+  }
+  if (Lq.empty()) return cudaSuccess;
+  by_form(Lq, [&](auto one) {
+    k_residual_q<T, one.value><<<Lq.blocks, QBLOCK, 0, s>>>(lev_of<one.value>(Lq));
+    k_restrict<T, one.value><<<Lc.blocks, CELL_BLOCK, 0, s>>>(lev_of<one.value>(Lc), lev_of<one.value>(Lq));
   });
-  note_launches(1);
+  note_launches(2);
   return cudaGetLastError();
 }
 
@@ -2296,14 +2440,50 @@ k_prolong(const __grid_constant__ Lev<ONE> A, const __grid_constant__ Lev<ONE> C
     sr1[threadIdx.x] = (cj0 < C.ny ? cj0 + 1 : cj0) - da;
     swy[threadIdx.x] = (T)glob(F.pwy)[j];
   }
+  const int ic = min(i, ib), ci0 = glob(F.plx)[ic];
+  const int i0 = ci0 - ca, i1 = (ci0 < C.nx ? ci0 + 1 : ci0) - ca;
+  const T wx1 = (T)glob(F.pwx)[ic], wz1 = (T)glob(F.pwz)[k];
+  const T wx[2] = {T(1) - wx1, wx1};
   cp_async_wait_all();
   __syncthreads();
+  // every coarse cell of the box active and every fine cell taking the
+  // correction: the weights sum to one and the eight corners factor into an
+  // x-z blend per coarse row, shared by the two fine rows next to it, and a
+  // y blend per fine row (512x256x256 FP32 in one level: 206 -> 159 us)
+  bool plain = true;
+  for (int e = threadIdx.x; e < 2 * nj * nw; e += PT_I) {
+    const int r = e / nw, w = e - r * nw, kk = r >= nj ? 1 : 0;
+    uint32_t in = 0u;  // bytes of the word inside the box
+#pragma unroll
+    for (int b = 0; b < 4; ++b)
+      if (4 * w + b >= sh && 4 * w + b < sh + ni) in |= 0x40u << (8 * b);
+    plain = plain && (smw[(kk * PT_CJ + r - kk * nj) * PT_MW + w] & in) == in;
+  }
+  if (i <= ib)
+#pragma unroll
+    for (int jj = 0; jj < PT_J; ++jj)
+      if (ja + jj <= jb) plain = plain && ((mp[jj >> 2] >> (8 * (jj & 3))) & 128);
+  plain = __syncthreads_and(plain);
   if (i > ib) return;
+  if (plain) {
+    auto blend = [&](int r) {
+      const T *u = sv + r * PT_CI, *v = sv + (PT_CJ + r) * PT_CI;
+      return (T(1) - wz1) * (wx[0] * u[i0] + wx1 * u[i1]) + wz1 * (wx[0] * v[i0] + wx1 * v[i1]);
+    };
+    int ra = sr0[0], rb = sr1[0];
+    T a0 = blend(ra), a1 = blend(rb);
+#pragma unroll
+    for (int jj = 0; jj < PT_J; ++jj) {
+      if (ja + jj > jb) break;
+      const int r0 = sr0[jj], r1 = sr1[jj];
+      if (r0 != ra) { a0 = r0 == rb ? a1 : blend(r0); ra = r0; }
+      if (r1 != rb) { a1 = blend(r1); rb = r1; }
+      const T wy1 = swy[jj];
+      x[id0 + fsy * jj] = xf[jj] + ((T(1) - wy1) * a0 + wy1 * a1);
+    }
+    return;
+  }
   const uint8_t *smb = reinterpret_cast<const uint8_t *>(smw);
-  const int ci0 = glob(F.plx)[i];
-  const int i0 = ci0 - ca, i1 = (ci0 < C.nx ? ci0 + 1 : ci0) - ca;
-  const T wx1 = (T)glob(F.pwx)[i], wz1 = (T)glob(F.pwz)[k];
-  const T wx[2] = {T(1) - wx1, wx1};
 #pragma unroll
   for (int jj = 0; jj < PT_J; ++jj) {
     if (ja + jj > jb) break;
@@ -2393,7 +2573,7 @@ k_rows_scatter(DevRows R, const __grid_constant__ Lev<ONE> A, const double *tmp)
 // writes them.  The two launches each cost their start and a chain of
 // dependent reads for a few thousand rows: 4.4 + 3.1 us under ncu for 1376
 // rows in FP64, 4.8 us for this one.
-constexpr int RC_BLOCKS = 8, RC_THREADS = 512, RC_KEEP = 4;
+constexpr int RC_BLOCKS = 8, RC_THREADS = 512, RC_KEEP = 2;
 constexpr int RC_MAX = RC_BLOCKS * RC_THREADS * RC_KEEP;
 template <typename T, bool ONE>
 __global__ void __cluster_dims__(RC_BLOCKS, 1, 1) __launch_bounds__(RC_THREADS)
@@ -4408,13 +4588,11 @@ extern "C" fg_status fg_debug_check(long long *out) {
 template cudaError_t line_sweep<double>(const Launch &, int, int, double, int, int, cudaStream_t);
 template cudaError_t line_sweep<float>(const Launch &, int, int, double, int, int, cudaStream_t);
 template cudaError_t residual<double>(const Launch &, double *, double *, cudaStream_t);
-template cudaError_t residual_q<double>(const Launch &, cudaStream_t);
-template cudaError_t residual_q<float>(const Launch &, cudaStream_t);
 template cudaError_t prolong_add<double>(const Launch &, const Launch &, cudaStream_t);
 template cudaError_t prolong_add<float>(const Launch &, const Launch &, cudaStream_t);
 template cudaError_t residual<float>(const Launch &, double *, double *, cudaStream_t);
-template cudaError_t restrict_to<double>(const Launch &, const Launch &, cudaStream_t);
-template cudaError_t restrict_to<float>(const Launch &, const Launch &, cudaStream_t);
+template cudaError_t restrict_to<double>(const Launch &, const Launch &, const Launch &, cudaStream_t);
+template cudaError_t restrict_to<float>(const Launch &, const Launch &, const Launch &, cudaStream_t);
 template cudaError_t zero_x<float>(const Launch &, cudaStream_t);
 template cudaError_t rows_relax<double>(const DevRows &, const Launch &, int, double *,
                                         cudaStream_t);
