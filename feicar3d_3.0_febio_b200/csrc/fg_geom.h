@@ -72,6 +72,9 @@ struct Geom {
   std::vector<double> g_coefD, g_bi, g_ip, g_probe, g_alpha, d_coefD, d_bi, d_probe;
   std::vector<int32_t> g_closest, d_closest;
   pinned_vector<char> h_stage;  // page-locked landing area of device -> host copies
+  // the masks' copies beside the row kernels (made at the first tagging)
+  cudaStream_t side = nullptr;
+  cudaEvent_t marked = nullptr, copied[3] = {};
   bool tagged = false;
 };
 
