@@ -39,7 +39,7 @@ struct Dims {
 // L1, and nothing divides by a runtime extent.  On 512x256x256 cells (each
 // thread one cell found by 64-bit divisions, the interpolation factors
 // divided out per cell, before): face velocities 587 -> 319 us, divergence
-// with the flux 251 + 362 -> 258 us, correction 739 -> 489 us; a plain
+// with the flux 251 + 362 -> 258 us, correction 739 -> 337 us; a plain
 // copy's rate would take 254, 180 and 300 us.
 constexpr int PJ_I = 64, PJ_J = 4, PJ_K = 8;
 struct Col {
@@ -300,7 +300,11 @@ __global__ void k_massflux_apply(Dims d, int vzg, const double *cv, double *bcxu
 }
 
 // correct_vel / calc_pres_grad: the face-interpolated gradient of p' on
-// the non-iblank cells; u -= dt grad p' and/or the gradient stored
+// the non-iblank cells; u -= dt grad p' and/or the gradient stored.  The
+// loads of CR_K planes come before their stores: a store to u may not be
+// passed by the next plane's load of u, which left one plane's loads in
+// flight per thread (512x256x256: 489 us plane by plane, 337 us so).
+constexpr int CR_K = 4;
 __global__ void __launch_bounds__(PJ_I * PJ_J)
 k_correct(Dims d, Met m, int kspan, const int8_t *__restrict__ ib, const double *__restrict__ pp, double dt,
           double *__restrict__ u, double *__restrict__ v, double *__restrict__ w, double *__restrict__ gx,
@@ -311,27 +315,43 @@ k_correct(Dims d, Met m, int kspan, const int8_t *__restrict__ ib, const double 
   const long long sy = d.NX, sz = d.NX * d.NY;
   const double fx1 = m.fx[i + 1], fx0 = m.fx[i], fy1 = m.fy[j + 1], fy0 = m.fy[j], dxi = m.dxi[i], dyi = m.dyi[j];
   double pm = pp[d.id(i, j, c.k0 - 1)], pc = pp[d.id(i, j, c.k0)];
-#pragma unroll 4
-  for (int k = c.k0; k < c.k1; ++k) {
-    const long long id = d.id(i, j, k);
-    const double pk = pp[id + sz], fz1 = m.fz[k + 1], fz0 = m.fz[k];
-    const double pe = fx1 * pp[id + 1] + (1.0 - fx1) * pc, pw = fx0 * pc + (1.0 - fx0) * pp[id - 1];
-    const double pn = fy1 * pp[id + sy] + (1.0 - fy1) * pc, ps = fy0 * pc + (1.0 - fy0) * pp[id - sy];
-    const double pf = fz1 * pk + (1.0 - fz1) * pc, pb = fz0 * pc + (1.0 - fz0) * pm;
-    const double pgx = (pe - pw) * dxi, pgy = (pn - ps) * dyi, pgz = (pf - pb) * m.dzi[k];
-    const double flag = 1.0 - (double)ib[id];
-    if (u) {
-      u[id] = u[id] - dt * pgx * flag;
-      v[id] = v[id] - dt * pgy * flag;
-      w[id] = w[id] - dt * pgz * flag;
+  for (int kb = c.k0; kb < c.k1; kb += CR_K) {
+    double pk[CR_K], px1[CR_K], px0[CR_K], py1[CR_K], py0[CR_K], vel[CR_K][3];
+    int8_t solid[CR_K];
+#pragma unroll
+    for (int q = 0; q < CR_K; ++q) {
+      if (kb + q >= c.k1) break;
+      const long long id = d.id(i, j, kb + q);
+      pk[q] = pp[id + sz];
+      px1[q] = pp[id + 1], px0[q] = pp[id - 1];
+      py1[q] = pp[id + sy], py0[q] = pp[id - sy];
+      solid[q] = ib[id];
+      if (u) vel[q][0] = u[id], vel[q][1] = v[id], vel[q][2] = w[id];
     }
-    if (gx) {
-      gx[id] = pgx * flag;
-      gy[id] = pgy * flag;
-      gz[id] = pgz * flag;
+#pragma unroll
+    for (int q = 0; q < CR_K; ++q) {
+      const int k = kb + q;
+      if (k >= c.k1) break;
+      const long long id = d.id(i, j, k);
+      const double fz1 = m.fz[k + 1], fz0 = m.fz[k];
+      const double pe = fx1 * px1[q] + (1.0 - fx1) * pc, pw = fx0 * pc + (1.0 - fx0) * px0[q];
+      const double pn = fy1 * py1[q] + (1.0 - fy1) * pc, ps = fy0 * pc + (1.0 - fy0) * py0[q];
+      const double pf = fz1 * pk[q] + (1.0 - fz1) * pc, pb = fz0 * pc + (1.0 - fz0) * pm;
+      const double pgx = (pe - pw) * dxi, pgy = (pn - ps) * dyi, pgz = (pf - pb) * m.dzi[k];
+      const double flag = 1.0 - (double)solid[q];
+      if (u) {
+        u[id] = vel[q][0] - dt * pgx * flag;
+        v[id] = vel[q][1] - dt * pgy * flag;
+        w[id] = vel[q][2] - dt * pgz * flag;
+      }
+      if (gx) {
+        gx[id] = pgx * flag;
+        gy[id] = pgy * flag;
+        gz[id] = pgz * flag;
+      }
+      pm = pc;
+      pc = pk[q];
     }
-    pm = pc;
-    pc = pk;
   }
 }
 
@@ -340,24 +360,39 @@ k_correct(Dims d, Met m, int kspan, const int8_t *__restrict__ ib, const double 
 // 0..nx on j in {0, ny} and j = 0..ny+1 on i in {0, nx}, each in the planes
 // 0, nz, nz+1, and the four k lines at (i, j) in {0, nx} x {0, ny}; then p =
 // p' when p is not null.  One pass; a block takes PU_I x PU_J entries of
-// planes z, z + gridDim.z, ...
-constexpr int PU_I = 128, PU_J = 2;
+// planes z, z + gridDim.z, ..., the loads of PU_K of them before their
+// stores (as above; 512x256x256: 164 us plane by plane, 110 us so).
+constexpr int PU_I = 128, PU_J = 2, PU_K = 4;
 __global__ void __launch_bounds__(PU_I * PU_J)
 k_update(Dims d, const int8_t *__restrict__ ib, const int8_t *__restrict__ dead, double *__restrict__ pp,
          double *__restrict__ p) {
   const int i = blockIdx.x * PU_I + threadIdx.x, j = blockIdx.y * PU_J + threadIdx.y;
   if (i >= d.NX || j >= d.NY) return;
   const bool ci = i == 0 || i == d.nx, cj = j == 0 || j == d.ny;
-#pragma unroll 4
-  for (int k = blockIdx.z; k < d.nz + 2; k += gridDim.z) {
-    const long long id = d.id(i, j, k);
-    const bool solid = i <= d.nx && ib[id] != 0 && dead[id] != -1;
-    const bool plane = k == 0 || k >= d.nz;
-    const bool edge = (plane && ((cj && i <= d.nx) || ci)) || (ci && cj);
-    const bool zero = solid || edge;
-    const double v = p ? pp[id] : 0.0;
-    if (zero) pp[id] = 0.0;
-    if (p) p[id] = zero ? 0.0 : v;
+  for (int kb = blockIdx.z; kb < d.nz + 2; kb += PU_K * gridDim.z) {
+    double v[PU_K];
+    int8_t in[PU_K], dd[PU_K];
+#pragma unroll
+    for (int q = 0; q < PU_K; ++q) {
+      const int k = kb + q * gridDim.z;
+      if (k >= d.nz + 2) break;
+      const long long id = d.id(i, j, k);
+      v[q] = p ? pp[id] : 0.0;
+      in[q] = ib[id];
+      dd[q] = dead[id];
+    }
+#pragma unroll
+    for (int q = 0; q < PU_K; ++q) {
+      const int k = kb + q * gridDim.z;
+      if (k >= d.nz + 2) break;
+      const long long id = d.id(i, j, k);
+      const bool solid = i <= d.nx && in[q] != 0 && dd[q] != -1;
+      const bool plane = k == 0 || k >= d.nz;
+      const bool edge = (plane && ((cj && i <= d.nx) || ci)) || (ci && cj);
+      const bool zero = solid || edge;
+      if (zero) pp[id] = 0.0;
+      if (p) p[id] = zero ? 0.0 : v[q];
+    }
   }
 }
 
