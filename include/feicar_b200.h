@@ -283,8 +283,8 @@ fg_status fg_ghostcell_velocity_device(fg_case *c, double *u, double *v, double 
  * from face_u/v/w when crank_nicolson (advec_scheme == CRANK_NICOLSON2;
  * central for 25 <= i <= 375, first-order upwind elsewhere, as the
  * reference), relaxation omega_ad.  The lines of each direction are
- * solved one anti-diagonal at a time, which gives the reference's
- * lexicographic Gauss-Seidel sweep bit for bit.  The ghost-cell
+ * solved as a wavefront, which gives the reference's lexicographic
+ * Gauss-Seidel sweep bit for bit.  The ghost-cell
  * coefficients the z sweep stores (ghostNScoeff) are not kept: the
  * velocity ghost-cell update stays with the caller. */
 typedef struct fg_ad_params {
@@ -379,7 +379,8 @@ enum {
   FG_PROF_LINE_X0 = 0,     /* finest-level x line sweeps (one colour each) */
   FG_PROF_LINE_Y0 = 1,     /* finest-level y line sweeps                   */
   FG_PROF_LINE_Z0 = 2,     /* finest-level z line sweeps                   */
-  FG_PROF_LINE_COARSE = 3, /* line sweeps of the coarse levels             */
+  FG_PROF_LINE_COARSE = 3, /* line sweeps of the coarse levels, and the    */
+                           /* levels that run as one kernel whole        */
   FG_PROF_RESIDUAL = 4,    /* finest residual / correction / norms         */
   FG_PROF_TRANSFER = 5,    /* residual, restriction, prolongation (coarse) */
   FG_PROF_ROWS = 6,        /* ghost / dead row relaxation                  */
