@@ -2307,7 +2307,10 @@ k_restrict(const __grid_constant__ Lev<ONE> A, const __grid_constant__ Lev<ONE> 
 
 template <typename T>
 cudaError_t restrict_to(const Launch &Lr, const Launch &Lq, const Launch &Lc, cudaStream_t s) {
-  if (!Lr.empty()) {
+  // FP64 batches keep the two passes: the fused one's registers leave too few
+  // blocks for their many small levels (64 problems, per batch solve: FP64
+  // 145.1 ms fused, 143.8 ms as two passes; mixed 117 ms either way)
+  if (!Lr.empty() && (sizeof(T) == 4 || Lr.n == 1)) {
     by_form(Lr, [&](auto one) {
       k_res_restrict<T, one.value><<<Lr.blocks, QBLOCK, 0, s>>>(lev_of<one.value>(Lr), lev_of<one.value>(Lc));
     });
