@@ -899,7 +899,7 @@ cudaError_t launch_sweeps(const ad::Dims &d, const ad::Met &m, const int8_t *ib,
   const size_t sm = (size_t)(n + 1) * (3 + 2 * NC) * sizeof(double);
   auto kern = ad::k_ad_sweeps<R, NC>;
   if (sm > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    const cudaError_t e = allow_smem(kern);
     if (e != cudaSuccess) return e;
   }
   kern<<<2 * (d.nz - 1) + d.ny - 1, ad::SW_ROLES + rows, sm, s>>>(d, m, ib, gh, C, F, half_dt, omega, binv, nref, sync);

@@ -162,6 +162,29 @@ void dev_free(void *p) {
   if (cur != o.first) cudaSetDevice(cur);
 }
 
+cudaError_t allow_smem_raw(const void *kern) {
+  static std::mutex mu;
+  static std::map<std::pair<int, const void *>, int> most;  // (device, kernel)
+  int dev = 0, bytes = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  {
+    std::lock_guard<std::mutex> lk(mu);
+    int &m = most[{dev, kern}];
+    if (m == 0) {
+      cudaFuncAttributes a;
+      if ((e = cudaFuncGetAttributes(&a, kern)) != cudaSuccess ||
+          (e = cudaDeviceGetAttribute(&m, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) != cudaSuccess) {
+        m = 0;
+        return e;
+      }
+      m -= (int)a.sharedSizeBytes;
+    }
+    bytes = m;
+  }
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+}
+
 void *pinned_get(size_t bytes) {
   if (bytes == 0) bytes = 1;
   PinnedPool &P = pinned_pool();

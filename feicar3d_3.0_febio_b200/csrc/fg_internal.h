@@ -181,6 +181,18 @@ inline cudaError_t dev_alloc(T **p, size_t bytes) {
   return dev_alloc_raw(reinterpret_cast<void **>(p), bytes);
 }
 
+// Lets a kernel be launched with any dynamic shared memory the current
+// device has.  The limit belongs to the function in the context, not to a
+// launch: a limit of a launch's own size could be lowered by another
+// thread's smaller launch of the same kernel before this one's launch or
+// graph instantiation.  So every caller sets the one value no launch
+// exceeds, the device's largest less the kernel's static part.
+cudaError_t allow_smem_raw(const void *kern);
+template <class... A>
+inline cudaError_t allow_smem(void (*kern)(A...)) {
+  return allow_smem_raw(reinterpret_cast<const void *>(kern));
+}
+
 // kernels launched by this process (every launch site adds its count)
 void note_launches(long long n);
 long long launches_so_far();

@@ -1293,22 +1293,23 @@ template <typename T, int MAXM>
 static cudaError_t launch_line(const Launch &Lr, int axis, int color, double omega, int maxn,
                                cudaStream_t s) {
   const T om = (T)omega;
+  cudaError_t e;
   if (axis == 0) {
     const size_t sm = smem_line(maxn, sizeof(T), 0);
     auto kern = k_xline<T, MAXM>;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if ((e = allow_smem(kern)) != cudaSuccess) return e;
     kern<<<Lr.blocks, XL_WARPS * 32, sm, s>>>(Lr.off, Lr.n, Lr.lev, color, om);
     note_launches(1);
   } else {
     const size_t sm = smem_line(maxn, sizeof(T), axis);
     if (axis == 1) {
       auto kern = k_yzline<T, MAXM, 1>;
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+      if ((e = allow_smem(kern)) != cudaSuccess) return e;
       kern<<<Lr.blocks, YZ_WARPS * 32, sm, s>>>(Lr.off, Lr.n, Lr.lev, color, om);
       note_launches(1);
     } else {
       auto kern = k_yzline<T, MAXM, 2>;
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+      if ((e = allow_smem(kern)) != cudaSuccess) return e;
       kern<<<Lr.blocks, YZ_WARPS * 32, sm, s>>>(Lr.off, Lr.n, Lr.lev, color, om);
       note_launches(1);
     }
@@ -2711,8 +2712,10 @@ cudaError_t coarsest_solve(int nprob, const DevLevel *lev, const double *const *
                            const int *const *gidx, const int *gn, int maxn, cudaStream_t s) {
   if (nprob <= 0) return cudaSuccess;
   const size_t sm = (size_t)maxn * sizeof(double);
-  if (sm > 48 * 1024)
-    cudaFuncSetAttribute(k_coarsest<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  if (sm > 48 * 1024) {
+    const cudaError_t e = allow_smem(k_coarsest<T>);
+    if (e != cudaSuccess) return e;
+  }
   k_coarsest<T><<<nprob, 256, sm, s>>>(lev, G, gidx, gn);
   note_launches(1);
   return cudaGetLastError();
@@ -3370,7 +3373,7 @@ int cycle_clusters(int size, size_t bytes) {
   cfg.attrs = at;
   cfg.numAttrs = 1;
   int n = 0;
-  if (cudaFuncSetAttribute(k_cycle<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess ||
+  if (allow_smem(k_cycle<T>) != cudaSuccess ||
       cudaFuncSetAttribute(k_cycle<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
       cudaOccupancyMaxActiveClusters(&n, k_cycle<T>, &cfg) != cudaSuccess) {
     (void)cudaGetLastError();
@@ -3386,7 +3389,7 @@ cudaError_t cycle(const Cycle &c, int first, const CycleSteps &nu, double omega,
                   double *tmp, cudaStream_t s) {
   if (c.n <= 0) return cudaSuccess;
   const size_t sm = c.bytes + (size_t)sc_round(c.maxgn * (int)sizeof(double));
-  cudaError_t e = cudaFuncSetAttribute(k_cycle<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  cudaError_t e = allow_smem(k_cycle<T>);
   if (e == cudaSuccess && c.size > 8)
     e = cudaFuncSetAttribute(k_cycle<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   if (e != cudaSuccess) return e;
