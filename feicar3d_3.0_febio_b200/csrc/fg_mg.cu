@@ -77,7 +77,6 @@ template <bool ONE> struct Lev;
 template <> struct Lev<false> {
   const int *off;
   int n;
-  const DevLevel *levs;
 };
 template <> struct Lev<true> {
   DevLevel one;
@@ -89,24 +88,26 @@ template <> struct Kry<false> {
 template <> struct Kry<true> {
   KDesc one;
 };
-// the block's problem p, its block lb within the problem, and its level
-__device__ __forceinline__ const DevLevel &entry(const Lev<true> &a, int &p, int &lb) {
+// the block's problem p and its block lb within the problem, and a problem's
+// level: from the array `levs`, which each kernel takes as a restrict-qualified
+// argument of its own.  As a member of Lev it cannot be qualified to any
+// effect, so a kernel read the descriptor again after every store (64 FP64
+// problems, untuned: basis updates 1.64 ms of a solve, residuals 0.52 ms).
+__device__ __forceinline__ void problem(const Lev<true> &, int &p, int &lb) {
   p = 0;
   lb = blockIdx.x;
-  return a.one;
 }
-__device__ __forceinline__ const DevLevel &entry(const Lev<false> &a, int &p, int &lb) {
+__device__ __forceinline__ void problem(const Lev<false> &a, int &p, int &lb) {
   p = find_entry(a.off, a.n, blockIdx.x);
   lb = blockIdx.x - a.off[p];
-  return a.levs[p];
 }
-__device__ __forceinline__ const DevLevel &level(const Lev<true> &a, int) { return a.one; }
-__device__ __forceinline__ const DevLevel &level(const Lev<false> &a, int p) { return a.levs[p]; }
+__device__ __forceinline__ const DevLevel &level(const Lev<true> &a, const DevLevel *, int) { return a.one; }
+__device__ __forceinline__ const DevLevel &level(const Lev<false> &, const DevLevel *levs, int p) { return levs[p]; }
 __device__ __forceinline__ const KDesc &krylov(const Kry<true> &a, int) { return a.one; }
 __device__ __forceinline__ const KDesc &krylov(const Kry<false> &a, int p) { return a.kd[p]; }
 template <bool ONE> Lev<ONE> lev_of(const Launch &L);
 template <> inline Lev<true> lev_of<true>(const Launch &L) { return {L.one}; }
-template <> inline Lev<false> lev_of<false>(const Launch &L) { return {L.off, L.n, L.lev}; }
+template <> inline Lev<false> lev_of<false>(const Launch &L) { return {L.off, L.n}; }
 template <bool ONE> Kry<ONE> kry_of(const KrySet &K);
 template <> inline Kry<true> kry_of<true>(const KrySet &K) { return {K.one}; }
 template <> inline Kry<false> kry_of<false>(const KrySet &K) { return {K.kd}; }
@@ -720,9 +721,10 @@ __device__ __forceinline__ void chunk_eliminate_smem(int r0, int n, const uint8_
 // lines; no shared memory.
 template <typename T, int M, int W, bool ONE>
 __global__ void __launch_bounds__(XL_WARPS * 32, 1)
-k_xline_reg(const __grid_constant__ Lev<ONE> A, int color, T omega) {
+k_xline_reg(const __grid_constant__ Lev<ONE> A, const DevLevel *FG_RESTRICT levs, int color, T omega) {
   int p, lb;
-  const DevLevel &L = entry(A, p, lb);
+  problem(A, p, lb);
+  const DevLevel &L = level(A, levs, p);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int sl = lane % W;
   const int nyh = (L.ny + 1) >> 1;
@@ -860,7 +862,7 @@ __device__ __forceinline__ bool xs_line(const DevLevel &L, int lb, int warp, int
 
 template <typename T, int M, bool ONE>
 __global__ void __launch_bounds__(XS_WARPS * 32)
-k_xline_smem(const __grid_constant__ Lev<ONE> A, int color, T omega) {
+k_xline_smem(const __grid_constant__ Lev<ONE> A, const DevLevel *FG_RESTRICT levs, int color, T omega) {
   using LY = XsLayout<T, M>;
   using LC = LineCoefT<T, 0>;
   constexpr int P = XS_PIECE;
@@ -870,7 +872,8 @@ k_xline_smem(const __grid_constant__ Lev<ONE> A, int color, T omega) {
   __shared__ T s_am[32 * (M + 1)], s_ap[32 * (M + 1)];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   int p, lb;
-  const DevLevel &L = entry(A, p, lb);
+  problem(A, p, lb);
+  const DevLevel &L = level(A, levs, p);
   const int n = L.nx;
   for (int r = threadIdx.x; r < n; r += XS_WARPS * 32) {
     s_am[r + r / M] = (T)glob(L.amx)[1 + r];
@@ -974,7 +977,7 @@ struct Eq3 { T a, c, d; };  // a x_prev + x + c x_next = d
 
 template <typename T, int M, int CH, int AXIS, bool ONE>
 __global__ void __launch_bounds__(CH * 32, (sizeof(T) == 4 && CH == 16) ? (M <= 8 ? 3 : 2) : 1)
-k_yzline_reg(const __grid_constant__ Lev<ONE> A, int color, T omega) {
+k_yzline_reg(const __grid_constant__ Lev<ONE> A, const DevLevel *FG_RESTRICT levs, int color, T omega) {
   using LC = LineCoefT<T, AXIS>;
   __shared__ ChunkEq<T> s_eq[CH][32];
   __shared__ T s_f[CH + 1][32];   // chunk-first unknowns
@@ -986,7 +989,8 @@ k_yzline_reg(const __grid_constant__ Lev<ONE> A, int color, T omega) {
   T *s_ga = s_al + M * NT;
   const int tid = threadIdx.x;
   int p, lb;
-  const DevLevel &L = entry(A, p, lb);
+  problem(A, p, lb);
+  const DevLevel &L = level(A, levs, p);
   const int ntx = (L.nx + 63) >> 6;
   const int ti = lb % ntx;
   const int o = 1 + lb / ntx;  // k for AXIS 1, j for AXIS 2
@@ -1321,7 +1325,7 @@ static cudaError_t launch_line(const Launch &Lr, int axis, int color, double ome
 template <typename T, int M, int W>
 static cudaError_t launch_xreg(const Launch &Lr, int color, double omega, cudaStream_t s) {
   by_form(Lr, [&](auto one) {
-    k_xline_reg<T, M, W, one.value><<<Lr.blocks, XL_WARPS * 32, 0, s>>>(lev_of<one.value>(Lr), color, (T)omega);
+    k_xline_reg<T, M, W, one.value><<<Lr.blocks, XL_WARPS * 32, 0, s>>>(lev_of<one.value>(Lr), Lr.lev, color, (T)omega);
   });
   note_launches(1);
   return cudaGetLastError();
@@ -1567,9 +1571,10 @@ struct YpBound {
 // the colour-0 launch left in L2
 template <typename T, int M, int CH, int AXIS, int NB, bool ONE>
 __global__ void __launch_bounds__(CH * YP_LINES, YpBound<T, CH, NB>::v)
-k_yzline_pcr(const __grid_constant__ Lev<ONE> A, int color, T omega) {
+k_yzline_pcr(const __grid_constant__ Lev<ONE> A, const DevLevel *FG_RESTRICT levs, int color, T omega) {
   int p, lb;
-  const DevLevel &L = entry(A, p, lb);
+  problem(A, p, lb);
+  const DevLevel &L = level(A, levs, p);
   const int ntx = (L.nx + 2 * YP_LINES - 1) / (2 * YP_LINES);
   const int ti = lb % ntx;
   const int o = color == 1 ? (AXIS == 1 ? L.nz : L.ny) - lb / ntx : 1 + lb / ntx;
@@ -1650,7 +1655,7 @@ static cudaError_t launch_xsmem(const Launch &Lr, int color, double omega, cudaS
   by_form(Lr, [&](auto one) {
     auto kern = k_xline_smem<T, M, one.value>;
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    kern<<<Lr.blocks, XS_WARPS * 32, sm, s>>>(lev_of<one.value>(Lr), color, (T)omega);
+    kern<<<Lr.blocks, XS_WARPS * 32, sm, s>>>(lev_of<one.value>(Lr), Lr.lev, color, (T)omega);
   });
   note_launches(1);
   return cudaGetLastError();
@@ -1662,7 +1667,7 @@ static cudaError_t launch_yzpcr(const Launch &Lr, int axis, int color, double om
   by_form(Lr, [&](auto one) {
     auto kern = axis == 1 ? k_yzline_pcr<T, M, CH, 1, NB, one.value> : k_yzline_pcr<T, M, CH, 2, NB, one.value>;
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    kern<<<Lr.blocks, CH * YP_LINES, sm, s>>>(lev_of<one.value>(Lr), color, (T)omega);
+    kern<<<Lr.blocks, CH * YP_LINES, sm, s>>>(lev_of<one.value>(Lr), Lr.lev, color, (T)omega);
   });
   note_launches(1);
   return cudaGetLastError();
@@ -1745,7 +1750,7 @@ static cudaError_t launch_yzreg(const Launch &Lr, int axis, int color, double om
   by_form(Lr, [&](auto one) {
     auto kern = axis == 1 ? k_yzline_reg<T, M, CH, 1, one.value> : k_yzline_reg<T, M, CH, 2, one.value>;
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    kern<<<Lr.blocks, CH * 32, sm, s>>>(lev_of<one.value>(Lr), color, (T)omega);
+    kern<<<Lr.blocks, CH * 32, sm, s>>>(lev_of<one.value>(Lr), Lr.lev, color, (T)omega);
   });
   note_launches(1);
   return cudaGetLastError();
@@ -2129,10 +2134,12 @@ bool restrict_fits(const DevLevel &F, const DevLevel &C) {
 // them 160 + 58.
 template <typename T, bool ONE>
 __global__ void __launch_bounds__(QBLOCK)
-k_res_restrict(const __grid_constant__ Lev<ONE> A, const __grid_constant__ Lev<ONE> CA) {
+k_res_restrict(const __grid_constant__ Lev<ONE> A, const DevLevel *FG_RESTRICT fine,
+               const __grid_constant__ Lev<ONE> CA, const DevLevel *FG_RESTRICT coarse) {
   int p, lb;
-  const DevLevel &F = entry(A, p, lb);
-  const DevLevel &C = level(CA, p);
+  problem(A, p, lb);
+  const DevLevel &F = level(A, fine, p);
+  const DevLevel &C = level(CA, coarse, p);
   const PairIdx q = pair_of(F.nx, C.ny, C.nz, lb);
   if (!q.ok) return;
   const int J = 1 + q.pj, K = q.k, j = 2 * J - 1;
@@ -2203,9 +2210,10 @@ k_res_restrict(const __grid_constant__ Lev<ONE> A, const __grid_constant__ Lev<O
 // restriction input); the arithmetic of k_residual, per quad
 template <typename T, bool ONE>
 __global__ void __launch_bounds__(QBLOCK)
-k_residual_q(const __grid_constant__ Lev<ONE> A) {
+k_residual_q(const __grid_constant__ Lev<ONE> A, const DevLevel *FG_RESTRICT levs) {
   int p, lb;
-  const DevLevel &L = entry(A, p, lb);
+  problem(A, p, lb);
+  const DevLevel &L = level(A, levs, p);
   auto x = PrecOf<T>::x(L);
   auto rhs = PrecOf<T>::rhs(L);
   auto res = PrecOf<T>::res(L);
@@ -2244,10 +2252,12 @@ k_residual_q(const __grid_constant__ Lev<ONE> A) {
 // (and the coarse unknown starts from zero)
 template <typename T, bool ONE>
 __global__ void __launch_bounds__(CELL_BLOCK)
-k_restrict(const __grid_constant__ Lev<ONE> A, const __grid_constant__ Lev<ONE> FA) {
+k_restrict(const __grid_constant__ Lev<ONE> A, const DevLevel *FG_RESTRICT coarse,
+           const __grid_constant__ Lev<ONE> FA, const DevLevel *FG_RESTRICT fine) {
   int p, lb;
-  const DevLevel &C = entry(A, p, lb);
-  const DevLevel &F = level(FA, p);
+  problem(A, p, lb);
+  const DevLevel &C = level(A, coarse, p);
+  const DevLevel &F = level(FA, fine, p);
   // the thread's i-children and their widths are kept over the block's
   // CELL_ROWS rows (at most two children per
   // axis: cl = 2I-1, ch = min(2I, n))
@@ -2313,15 +2323,17 @@ cudaError_t restrict_to(const Launch &Lr, const Launch &Lq, const Launch &Lc, cu
   // 145.1 ms fused, 143.8 ms as two passes; mixed 117 ms either way)
   if (!Lr.empty() && (sizeof(T) == 4 || Lr.n == 1)) {
     by_form(Lr, [&](auto one) {
-      k_res_restrict<T, one.value><<<Lr.blocks, QBLOCK, 0, s>>>(lev_of<one.value>(Lr), lev_of<one.value>(Lc));
+      k_res_restrict<T, one.value><<<Lr.blocks, QBLOCK, 0, s>>>(
+          lev_of<one.value>(Lr), Lr.lev, lev_of<one.value>(Lc), Lc.lev);
     });
     note_launches(1);
     return cudaGetLastError();
   }
   if (Lq.empty()) return cudaSuccess;
   by_form(Lq, [&](auto one) {
-    k_residual_q<T, one.value><<<Lq.blocks, QBLOCK, 0, s>>>(lev_of<one.value>(Lq));
-    k_restrict<T, one.value><<<Lc.blocks, CELL_BLOCK, 0, s>>>(lev_of<one.value>(Lc), lev_of<one.value>(Lq));
+    k_residual_q<T, one.value><<<Lq.blocks, QBLOCK, 0, s>>>(lev_of<one.value>(Lq), Lq.lev);
+    k_restrict<T, one.value><<<Lc.blocks, CELL_BLOCK, 0, s>>>(
+        lev_of<one.value>(Lc), Lc.lev, lev_of<one.value>(Lq), Lq.lev);
   });
   note_launches(2);
   return cudaGetLastError();
@@ -2384,14 +2396,16 @@ __device__ __forceinline__ void cp_async_wait_all() {
 
 template <typename T, bool ONE>
 __global__ void __launch_bounds__(PT_I)
-k_prolong(const __grid_constant__ Lev<ONE> A, const __grid_constant__ Lev<ONE> CA) {
+k_prolong(const __grid_constant__ Lev<ONE> A, const DevLevel *FG_RESTRICT fine,
+          const __grid_constant__ Lev<ONE> CA, const DevLevel *FG_RESTRICT coarse) {
   __shared__ T sv[2 * PT_CJ * PT_CI];
   __shared__ uint32_t smw[2 * PT_CJ * PT_MW];
   __shared__ T swy[PT_J];
   __shared__ int sr0[PT_J], sr1[PT_J];
   int p, lb;
-  const DevLevel &F = entry(A, p, lb);
-  const DevLevel &C = level(CA, p);
+  problem(A, p, lb);
+  const DevLevel &F = level(A, fine, p);
+  const DevLevel &C = level(CA, coarse, p);
   const int nti = (F.nx + PT_I - 1) / PT_I, ntj = (F.ny + PT_J - 1) / PT_J;
   const int ti = lb % nti, rest = lb / nti, tj = rest % ntj, k = 1 + rest / ntj;
   const int ia = 1 + ti * PT_I, ib = min(F.nx, ia + PT_I - 1);
@@ -2512,7 +2526,8 @@ template <typename T>
 cudaError_t prolong_add(const Launch &Lf, const Launch &Lc, cudaStream_t s) {
   if (Lf.empty()) return cudaSuccess;
   by_form(Lf, [&](auto one) {
-    k_prolong<T, one.value><<<Lf.blocks, CELL_BLOCK, 0, s>>>(lev_of<one.value>(Lf), lev_of<one.value>(Lc));
+    k_prolong<T, one.value><<<Lf.blocks, CELL_BLOCK, 0, s>>>(
+        lev_of<one.value>(Lf), Lf.lev, lev_of<one.value>(Lc), Lc.lev);
   });
   note_launches(1);
   return cudaGetLastError();
@@ -2547,10 +2562,10 @@ cudaError_t zero_x(const Launch &Lr, cudaStream_t s) {
 // from the current field first (k_rows), then written (k_rows_scatter).
 template <typename T, bool ONE>
 __global__ void __launch_bounds__(CELL_BLOCK)
-k_rows(DevRows R, const __grid_constant__ Lev<ONE> A, int corr, double *tmp) {
+k_rows(DevRows R, const __grid_constant__ Lev<ONE> A, const DevLevel *levs, int corr, double *tmp) {
   const int r = blockIdx.x * CELL_BLOCK + threadIdx.x;
   if (r >= R.n) return;
-  const DevLevel &L = level(A, ONE ? 0 : R.prob[r]);
+  const DevLevel &L = level(A, levs, ONE ? 0 : R.prob[r]);
   auto x = PrecOf<T>::x(L);
   const long long b = R.cell[r], sy = L.sy, sz = L.sz;
   const long long o[8] = {0, sy, sy + 1, 1, sz, sz + sy, sz + sy + 1, sz + 1};
@@ -2565,10 +2580,10 @@ k_rows(DevRows R, const __grid_constant__ Lev<ONE> A, int corr, double *tmp) {
 
 template <typename T, bool ONE>
 __global__ void __launch_bounds__(CELL_BLOCK)
-k_rows_scatter(DevRows R, const __grid_constant__ Lev<ONE> A, const double *tmp) {
+k_rows_scatter(DevRows R, const __grid_constant__ Lev<ONE> A, const DevLevel *levs, const double *tmp) {
   const int r = blockIdx.x * CELL_BLOCK + threadIdx.x;
   if (r >= R.n) return;
-  const DevLevel &L = level(A, ONE ? 0 : R.prob[r]);
+  const DevLevel &L = level(A, levs, ONE ? 0 : R.prob[r]);
   PrecOf<T>::x(L)[R.tgt[r]] = (T)tmp[r];
 }
 
@@ -2581,7 +2596,7 @@ constexpr int RC_BLOCKS = 8, RC_THREADS = 512, RC_KEEP = 2;
 constexpr int RC_MAX = RC_BLOCKS * RC_THREADS * RC_KEEP;
 template <typename T, bool ONE>
 __global__ void __cluster_dims__(RC_BLOCKS, 1, 1) __launch_bounds__(RC_THREADS)
-k_rows_cluster(DevRows R, const __grid_constant__ Lev<ONE> A, int corr) {
+k_rows_cluster(DevRows R, const __grid_constant__ Lev<ONE> A, const DevLevel *levs, int corr) {
   T v[RC_KEEP];
   long long t[RC_KEEP];
   int pr[RC_KEEP];
@@ -2590,7 +2605,7 @@ k_rows_cluster(DevRows R, const __grid_constant__ Lev<ONE> A, int corr) {
     const int r = (u * RC_BLOCKS + (int)blockIdx.x) * RC_THREADS + (int)threadIdx.x;
     if (r >= R.n) continue;
     pr[u] = ONE ? 0 : R.prob[r];
-    const DevLevel &L = level(A, pr[u]);
+    const DevLevel &L = level(A, levs, pr[u]);
     auto x = PrecOf<T>::x(L);
     const long long b = R.cell[r], sy = L.sy, sz = L.sz;
     const long long o[8] = {0, sy, sy + 1, 1, sz, sz + sy, sz + sy + 1, sz + 1};
@@ -2605,7 +2620,7 @@ k_rows_cluster(DevRows R, const __grid_constant__ Lev<ONE> A, int corr) {
 #pragma unroll
   for (int u = 0; u < RC_KEEP; ++u) {
     const int r = (u * RC_BLOCKS + (int)blockIdx.x) * RC_THREADS + (int)threadIdx.x;
-    if (r < R.n) PrecOf<T>::x(level(A, pr[u]))[t[u]] = v[u];
+    if (r < R.n) PrecOf<T>::x(level(A, levs, pr[u]))[t[u]] = v[u];
   }
 }
 
@@ -2614,15 +2629,15 @@ cudaError_t rows_relax(const DevRows &R, const Launch &L0, int corr, double *tmp
   if (R.n <= 0) return cudaSuccess;
   if (R.n <= RC_MAX) {
     by_form(L0, [&](auto one) {
-      k_rows_cluster<T, one.value><<<RC_BLOCKS, RC_THREADS, 0, s>>>(R, lev_of<one.value>(L0), corr);
+      k_rows_cluster<T, one.value><<<RC_BLOCKS, RC_THREADS, 0, s>>>(R, lev_of<one.value>(L0), L0.lev, corr);
     });
     note_launches(1);
     return cudaGetLastError();
   }
   const int nb = (R.n + CELL_BLOCK - 1) / CELL_BLOCK;
   by_form(L0, [&](auto one) {
-    k_rows<T, one.value><<<nb, CELL_BLOCK, 0, s>>>(R, lev_of<one.value>(L0), corr, tmp);
-    k_rows_scatter<T, one.value><<<nb, CELL_BLOCK, 0, s>>>(R, lev_of<one.value>(L0), tmp);
+    k_rows<T, one.value><<<nb, CELL_BLOCK, 0, s>>>(R, lev_of<one.value>(L0), L0.lev, corr, tmp);
+    k_rows_scatter<T, one.value><<<nb, CELL_BLOCK, 0, s>>>(R, lev_of<one.value>(L0), L0.lev, tmp);
   });
   note_launches(2);
   return cudaGetLastError();
@@ -3822,9 +3837,11 @@ __device__ __forceinline__ KSel kidx(const KCtl *ctl, int ph, KSel s) {
 // (4 cells of a row per thread, vector loads), FP64 arithmetic.
 template <typename B, bool ONE>
 __global__ void __launch_bounds__(QBLOCK)
-k_kr_resid(const __grid_constant__ Lev<ONE> A, const __grid_constant__ Kry<ONE> K, int vd, double *part) {
+k_kr_resid(const __grid_constant__ Lev<ONE> A, const DevLevel *FG_RESTRICT levs, const __grid_constant__ Kry<ONE> K,
+           int vd, double *part) {
   int p, lb;
-  const DevLevel &L = entry(A, p, lb);
+  problem(A, p, lb);
+  const DevLevel &L = level(A, levs, p);
   const KDesc &d = krylov(K, p);
   auto P = glob(mkptr<const double>(d.P, d.n, K_X));
   auto F = glob(mkptr<const double>(d.F, d.n, K_RHS));
@@ -3869,11 +3886,12 @@ k_kr_resid(const __grid_constant__ Lev<ONE> A, const __grid_constant__ Kry<ONE> 
 // couple to (they are held at the staged zero), so A x_T equals A Z_vz.
 template <typename B, typename T, bool ONE>
 __global__ void __launch_bounds__(QBLOCK)
-k_kr_apply_q(const __grid_constant__ Lev<ONE> A, const __grid_constant__ Kry<ONE> K, int vz, int vw,
-             const KCtl *ctl) {
+k_kr_apply_q(const __grid_constant__ Lev<ONE> A, const DevLevel *FG_RESTRICT levs, const __grid_constant__ Kry<ONE> K,
+             int vz, int vw, const KCtl *ctl) {
   if (ctl) { vz = ctl->j; vw = ctl->j + 1; }
   int p, lb;
-  const DevLevel &L = entry(A, p, lb);
+  problem(A, p, lb);
+  const DevLevel &L = level(A, levs, p);
   const KDesc &d = krylov(K, p);
   auto x = PrecOf<T>::x(L);
   auto Z = kvec<B>(d, d.Z, vz);
@@ -3923,8 +3941,8 @@ k_kr_apply_q(const __grid_constant__ Lev<ONE> A, const __grid_constant__ Kry<ONE
 // preconditioner: rd = rf = V_vs[t]
 template <typename B, bool ONE>
 __global__ void __launch_bounds__(CELL_BLOCK)
-k_kr_rows(DevRows R, const __grid_constant__ Lev<ONE> A, const __grid_constant__ Kry<ONE> K, int mode, int vs, int vd, const KCtl *ctl,
-          int ph) {
+k_kr_rows(DevRows R, const __grid_constant__ Lev<ONE> A, const DevLevel *levs, const __grid_constant__ Kry<ONE> K,
+          int mode, int vs, int vd, const KCtl *ctl, int ph) {
   if (ctl) {
     if (mode == 1) { vs = ctl->j; vd = ctl->j + 1; }
     if (mode == 2) {
@@ -3935,7 +3953,7 @@ k_kr_rows(DevRows R, const __grid_constant__ Lev<ONE> A, const __grid_constant__
   const int r = blockIdx.x * CELL_BLOCK + threadIdx.x;
   if (r >= R.n) return;
   const int p = ONE ? 0 : R.prob[r];
-  const DevLevel &L = level(A, p);
+  const DevLevel &L = level(A, levs, p);
   const KDesc &d = krylov(K, p);
   const long long t = R.tgt[r];
   if (mode == 2) {
@@ -3989,7 +4007,7 @@ k_kr_dots(const __grid_constant__ Lev<ONE> A, const __grid_constant__ Kry<ONE> K
     nv = ks.nv;
   }
   int p, lb;
-  entry(A, p, lb);
+  problem(A, p, lb);
   const KDesc &d = krylov(K, p);
   const long long lim = flat_end(d.n);
   B w[FLAT_PPT][4];
@@ -4077,14 +4095,14 @@ k_kr_reduce(const int *off, const double *part, int nblk, double *out, int ostri
 // stage, rhs_T = V_vd on active rows (0 elsewhere) and x_T = 0
 template <typename B, typename T, bool ONE>
 __global__ void __launch_bounds__(FLAT_THREADS)
-k_kr_vaxpy(const __grid_constant__ Lev<ONE> A, const __grid_constant__ Kry<ONE> K, int vd, int s0, int ns,
-           const double *coef, int cs, int stage, const KCtl *ctl, int ph) {
+k_kr_vaxpy(const __grid_constant__ Lev<ONE> A, const DevLevel *FG_RESTRICT levs, const __grid_constant__ Kry<ONE> K,
+           int vd, int s0, int ns, const double *coef, int cs, int stage, const KCtl *ctl, int ph) {
   {
     const KSel ks = kidx(ctl, ph, KSel{0, 0, 0, vd, s0, ns, stage});
     vd = ks.vd; s0 = ks.s0; ns = ks.ns; stage = ks.stage;
   }
   int p, lb;
-  const DevLevel &L = entry(A, p, lb);
+  problem(A, p, lb);
   const KDesc &d = krylov(K, p);
   const long long lim = flat_end(d.n);
   const double *cf = coef + (size_t)p * cs;
@@ -4119,6 +4137,7 @@ k_kr_vaxpy(const __grid_constant__ Lev<ONE> A, const __grid_constant__ Kry<ONE> 
 #pragma unroll
       for (int q = 0; q < 4; ++q) acc[u][q] += ci * (double)v[u][q];
   }
+  const DevLevel &L = level(A, levs, p);
 #pragma unroll
   for (int u = 0; u < FLAT_PPT; ++u) {
     if (!ok[u]) continue;
@@ -4147,7 +4166,7 @@ k_kr_update(const __grid_constant__ Lev<ONE> A, const __grid_constant__ Kry<ONE>
   if (ctl) ns = ctl->jlast;
   if (ns == 0) return;
   int p, lb;
-  entry(A, p, lb);
+  problem(A, p, lb);
   const KDesc &d = krylov(K, p);
   const long long lim = flat_end(d.n);
   const double *cf = coef + (size_t)p * cs;
@@ -4182,7 +4201,8 @@ static void kr_rows(const Launch &L, const DevRows &R, const KrySet &kd, int mod
                     cudaStream_t s) {
   const int nb = (R.n + CELL_BLOCK - 1) / CELL_BLOCK;
   by_form(L, [&](auto one) {
-    k_kr_rows<B, one.value><<<nb, CELL_BLOCK, 0, s>>>(R, lev_of<one.value>(L), kry_of<one.value>(kd), mode, vs, vd, ctl, ph);
+    k_kr_rows<B, one.value><<<nb, CELL_BLOCK, 0, s>>>(
+        R, lev_of<one.value>(L), L.lev, kry_of<one.value>(kd), mode, vs, vd, ctl, ph);
   });
 }
 
@@ -4191,7 +4211,8 @@ cudaError_t kr_resid(const Launch &quads, const DevRows &R, const KrySet &kd, in
                      double *part, double *norm2, cudaStream_t s) {
   if (quads.empty()) return cudaSuccess;
   by_form(quads, [&](auto one) {
-    k_kr_resid<B, one.value><<<quads.blocks, QBLOCK, 0, s>>>(lev_of<one.value>(quads), kry_of<one.value>(kd), vd, part);
+    k_kr_resid<B, one.value><<<quads.blocks, QBLOCK, 0, s>>>(
+        lev_of<one.value>(quads), quads.lev, kry_of<one.value>(kd), vd, part);
   });
   k_reduce_parts<<<quads.n, 1024, 0, s>>>(quads.off, part, norm2);
   note_launches(2);
@@ -4207,7 +4228,8 @@ cudaError_t kr_apply(const Launch &quads, const DevRows &R, const KrySet &kd, in
                      int vw, cudaStream_t s) {
   if (quads.empty()) return cudaSuccess;
   by_form(quads, [&](auto one) {
-    k_kr_apply_q<B, T, one.value><<<quads.blocks, QBLOCK, 0, s>>>(lev_of<one.value>(quads), kry_of<one.value>(kd), vz, vw, nullptr);
+    k_kr_apply_q<B, T, one.value><<<quads.blocks, QBLOCK, 0, s>>>(
+        lev_of<one.value>(quads), quads.lev, kry_of<one.value>(kd), vz, vw, nullptr);
   });
   note_launches(1);
   if (R.n > 0) {
@@ -4223,7 +4245,8 @@ cudaError_t kr_dots(const Launch &flat, const KrySet &kd, int vw, int nv, double
   if (flat.empty()) return cudaSuccess;
   if (nv > KR_MAXV) return cudaErrorInvalidValue;
   by_form(flat, [&](auto one) {
-    k_kr_dots<B, one.value><<<flat.blocks, FLAT_THREADS, 0, s>>>(lev_of<one.value>(flat), kry_of<one.value>(kd), vw, nv, flat.blocks, part, nullptr, 0);
+    k_kr_dots<B, one.value><<<flat.blocks, FLAT_THREADS, 0, s>>>(
+        lev_of<one.value>(flat), kry_of<one.value>(kd), vw, nv, flat.blocks, part, nullptr, 0);
   });
   k_kr_reduce<<<dim3(flat.n, nv + 1), 256, 0, s>>>(flat.off, part, flat.blocks, out, ostride, nullptr, 0);
   note_launches(2);
@@ -4236,7 +4259,8 @@ cudaError_t kr_vaxpy(const Launch &flat, const DevRows &R, const KrySet &kd, int
   if (flat.empty()) return cudaSuccess;
   if (ns > KR_MAXV) return cudaErrorInvalidValue;
   by_form(flat, [&](auto one) {
-    k_kr_vaxpy<B, T, one.value><<<flat.blocks, FLAT_THREADS, 0, s>>>(lev_of<one.value>(flat), kry_of<one.value>(kd), vd, s0, ns, coef, cs, stage ? 1 : 0, nullptr, 0);
+    k_kr_vaxpy<B, T, one.value><<<flat.blocks, FLAT_THREADS, 0, s>>>(
+        lev_of<one.value>(flat), flat.lev, kry_of<one.value>(kd), vd, s0, ns, coef, cs, stage ? 1 : 0, nullptr, 0);
   });
   note_launches(1);
   if (stage && R.n > 0) {
@@ -4252,7 +4276,8 @@ cudaError_t kr_update(const Launch &flat, const KrySet &kd, int ns, const double
   if (flat.empty() || ns == 0) return cudaSuccess;
   if (ns > KR_MAXV) return cudaErrorInvalidValue;
   by_form(flat, [&](auto one) {
-    k_kr_update<B, one.value><<<flat.blocks, FLAT_THREADS, 0, s>>>(lev_of<one.value>(flat), kry_of<one.value>(kd), ns, coef, cs, nullptr);
+    k_kr_update<B, one.value><<<flat.blocks, FLAT_THREADS, 0, s>>>(
+        lev_of<one.value>(flat), kry_of<one.value>(kd), ns, coef, cs, nullptr);
   });
   note_launches(1);
   return cudaGetLastError();
@@ -4282,7 +4307,8 @@ cudaError_t krd_apply(const Launch &quads, const DevRows &R, const KrySet &kd,
                       const KCtl *ctl, cudaStream_t s) {
   if (quads.empty()) return cudaSuccess;
   by_form(quads, [&](auto one) {
-    k_kr_apply_q<B, T, one.value><<<quads.blocks, QBLOCK, 0, s>>>(lev_of<one.value>(quads), kry_of<one.value>(kd), 0, 0, ctl);
+    k_kr_apply_q<B, T, one.value><<<quads.blocks, QBLOCK, 0, s>>>(
+        lev_of<one.value>(quads), quads.lev, kry_of<one.value>(kd), 0, 0, ctl);
   });
   note_launches(1);
   if (R.n > 0) {
@@ -4297,7 +4323,8 @@ cudaError_t krd_dots(const Launch &flat, const KrySet &kd, const KCtl *ctl, int 
                      double *out, cudaStream_t s) {
   if (flat.empty()) return cudaSuccess;
   by_form(flat, [&](auto one) {
-    k_kr_dots<B, one.value><<<flat.blocks, FLAT_THREADS, 0, s>>>(lev_of<one.value>(flat), kry_of<one.value>(kd), 0, 0, flat.blocks, part, ctl, phase);
+    k_kr_dots<B, one.value><<<flat.blocks, FLAT_THREADS, 0, s>>>(
+        lev_of<one.value>(flat), kry_of<one.value>(kd), 0, 0, flat.blocks, part, ctl, phase);
   });
   k_kr_reduce<<<dim3(flat.n, KR_MAXV + 1), 256, 0, s>>>(flat.off, part, flat.blocks, out, KR_CS, ctl, phase);
   note_launches(2);
@@ -4309,7 +4336,8 @@ cudaError_t krd_vaxpy(const Launch &flat, const DevRows &R, const KrySet &kd,
                       const KCtl *ctl, int phase, const double *coef, cudaStream_t s) {
   if (flat.empty()) return cudaSuccess;
   by_form(flat, [&](auto one) {
-    k_kr_vaxpy<B, T, one.value><<<flat.blocks, FLAT_THREADS, 0, s>>>(lev_of<one.value>(flat), kry_of<one.value>(kd), 0, 0, 0, coef, KR_CS, 0, ctl, phase);
+    k_kr_vaxpy<B, T, one.value><<<flat.blocks, FLAT_THREADS, 0, s>>>(
+        lev_of<one.value>(flat), flat.lev, kry_of<one.value>(kd), 0, 0, 0, coef, KR_CS, 0, ctl, phase);
   });
   note_launches(1);
   if (phase != KPH_REORTH && R.n > 0) {  // staged row constants (skipped on the device when not staged)
@@ -4324,7 +4352,8 @@ cudaError_t krd_update(const Launch &flat, const KrySet &kd, const KCtl *ctl, co
                        cudaStream_t s) {
   if (flat.empty()) return cudaSuccess;
   by_form(flat, [&](auto one) {
-    k_kr_update<B, one.value><<<flat.blocks, FLAT_THREADS, 0, s>>>(lev_of<one.value>(flat), kry_of<one.value>(kd), 0, coef, KR_CS, ctl);
+    k_kr_update<B, one.value><<<flat.blocks, FLAT_THREADS, 0, s>>>(
+        lev_of<one.value>(flat), kry_of<one.value>(kd), 0, coef, KR_CS, ctl);
   });
   note_launches(1);
   return cudaGetLastError();
