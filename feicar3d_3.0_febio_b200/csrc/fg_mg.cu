@@ -2691,24 +2691,35 @@ cudaError_t rows_residual(const DevRows &R, const DevLevel *lev0, double *maxabs
 
 // ---------------------------------------------------- coarsest solve
 // x = G rhs over the active cells of a problem's coarsest level, G the
-// generalised inverse of the coarsest operator (FP64).  One warp per row
-// of G, its lanes along the row: the row is read once, coalesced (a thread
-// per row read it by single dependent loads: 147 us for 125 cells).
+// generalised inverse of the coarsest operator (FP64).  A warp takes four
+// rows of G at a time, its lanes along them, so that a row is read once,
+// coalesced, with four rows' loads in flight: reading G is a matter of
+// latency.  k_coarsest on 64 problems, the largest of 512 cells: a row per
+// warp of 256 threads 289 us, a thread per row 157 us, this 139 us (125 cells
+// in one problem, a thread per row: 147 us).
+constexpr int COARSEST_THREADS = 1024;
 template <typename V, typename S>
 __device__ __forceinline__ void dense_rows(const double *G, int n, const V &rhs, const S &store) {
+  constexpr int R = 4;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  for (int r = warp; r < n; r += nw) {
-    const double *gr = G + (size_t)r * n;
-    double acc = 0.0;
-    for (int c = lane; c < n; c += 32) acc += gr[c] * rhs(c);
+  for (int r0 = R * warp; r0 < n; r0 += R * nw) {
+    double acc[R] = {};
+    for (int c = lane; c < n; c += 32) {
+      const double v = rhs(c);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-    if (lane == 0) store(r, acc);
+      for (int q = 0; q < R; ++q) acc[q] += G[(size_t)min(r0 + q, n - 1) * n + c] * v;
+    }
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) acc[q] += __shfl_down_sync(0xffffffffu, acc[q], o);
+      if (lane == 0 && r0 + q < n) store(r0 + q, acc[q]);
+    }
   }
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(COARSEST_THREADS)
 k_coarsest(const DevLevel *FG_RESTRICT levs, const double *const *G, const int *const *gidx, const int *gn) {
   extern __shared__ double sr[];
   const int p = blockIdx.x;
@@ -2731,7 +2742,7 @@ cudaError_t coarsest_solve(int nprob, const DevLevel *lev, const double *const *
     const cudaError_t e = allow_smem(k_coarsest<T>);
     if (e != cudaSuccess) return e;
   }
-  k_coarsest<T><<<nprob, 256, sm, s>>>(lev, G, gidx, gn);
+  k_coarsest<T><<<nprob, COARSEST_THREADS, sm, s>>>(lev, G, gidx, gn);
   note_launches(1);
   return cudaGetLastError();
 }
