@@ -2318,10 +2318,10 @@ k_restrict(const __grid_constant__ Lev<ONE> A, const DevLevel *FG_RESTRICT coars
 
 template <typename T>
 cudaError_t restrict_to(const Launch &Lr, const Launch &Lq, const Launch &Lc, cudaStream_t s) {
-  // FP64 batches keep the two passes: the fused one's registers leave too few
-  // blocks for their many small levels (64 problems, per batch solve: FP64
-  // 145.1 ms fused, 143.8 ms as two passes; mixed 117 ms either way)
-  if (!Lr.empty() && (sizeof(T) == 4 || Lr.n == 1)) {
+  // one pass wherever it can be: batches too (FP64 solves of 2, 8, 16 and 64
+  // cubes of 32 to 192 cells an edge: 7.60, 10.15, 28.62 and 234.1 ms, as two
+  // passes 7.75, 10.28, 28.80 and 234.4)
+  if (!Lr.empty()) {
     by_form(Lr, [&](auto one) {
       k_res_restrict<T, one.value><<<Lr.blocks, QBLOCK, 0, s>>>(
           lev_of<one.value>(Lr), Lr.lev, lev_of<one.value>(Lc), Lc.lev);
