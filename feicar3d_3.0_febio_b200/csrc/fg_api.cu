@@ -848,7 +848,7 @@ static fg_status build_cycle(fg_batch *b) {
   const bool cluster = (int)b->cases.size() <= CL_MAXPROBS;
   for (int L = cluster ? 0 : 1; L < b->maxdepth; ++L) {
     bool fits = true;
-    size_t most = 0, need = 0;
+    size_t most = 0, coarsest = 0;  // largest levels and largest coarsest system of any problem: what is launched
     std::vector<CycleProb> probs;
     std::vector<DevLevel> lv;
     for (auto *c : b->cases) {
@@ -862,21 +862,21 @@ static fg_status build_cycle(fg_batch *b) {
              (L + ns == 0 || (long long)c->lev[L + ns].nx * c->lev[L + ns].ny * c->lev[L + ns].nz > SC_MAXCELLS))
         ++ns;
       q.ns = ns;
-      size_t sum = 0, coarsest = 0;
+      size_t sum = 0;
       for (int l = 0; l < q.nl; ++l) {
         const HLevel &H = c->lev[L + l];
         const long long cells = (long long)H.nx * H.ny * H.nz;
         sum += k::cycle_bytes(H.nx, H.ny, H.nz, ts, l >= ns);
-        coarsest = (size_t)cells * sizeof(double);
+        if (l == q.nl - 1) coarsest = std::max(coarsest, ((size_t)cells * sizeof(double) + 15) & ~size_t(15));
         fits = fits && H.nx <= SC_MAXN && H.ny <= SC_MAXN && H.nz <= SC_MAXN && cells <= CL_MAXCELLS;
         lv.push_back(H.dl);
       }
-      fits = fits && L + ns > 0 && sum + coarsest <= SC_MAXBYTES;
+      fits = fits && L + ns > 0;
       most = std::max(most, sum);
-      need = std::max(need, sum + coarsest);
       probs.push_back(q);
     }
-    if (!fits || probs.empty()) continue;
+    const size_t need = most + coarsest;
+    if (!fits || probs.empty() || need > SC_MAXBYTES) continue;
     cy.n = (int)probs.size();
     cy.Lc = L;
     cy.bytes = most;
