@@ -30,3 +30,24 @@ _load_pkg()
 def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA device (B200, sm_100a)")
     config.addinivalue_line("markers", "slow: CPU test that takes more than a few seconds")
+
+
+@pytest.fixture(autouse=True)
+def _fields_written(request, monkeypatch):
+    """The tests fill their device fields on torch's stream, and a handle's
+    own stream is not ordered after it: the binding's functions on device
+    fields start here once torch's work is done."""
+    if request.node.get_closest_marker("gpu") is None:
+        return
+    import torch
+
+    from feicar_b200 import fg
+
+    def after_torch(call):
+        def ordered(*args, **kw):
+            torch.cuda.synchronize()
+            return call(*args, **kw)
+        return ordered
+
+    for name in [n for n in vars(fg) if n.endswith("_device") and callable(getattr(fg, n))]:
+        monkeypatch.setattr(fg, name, after_torch(getattr(fg, name)))
