@@ -489,11 +489,12 @@ k_ad_sweeps(Dims d, Met m, const int8_t *__restrict__ ib, const int8_t *__restri
 
 // the lines of anti-diagonal `diag` along AXIS (0: x lines (j,k), j + k =
 // diag; 1: y lines (i,k); 2: z lines (i,j)), one thread per line, gam and
-// the forward values in the thread's slot of `scr` (2 (n+1) doubles): for
-// lines longer than k_ad_sweeps' rows per thread hold
+// the forward values in the thread's slot of `scr` (2 (n+1) doubles), the
+// pivots formed along the line: for lines longer than k_ad_sweeps' rows per
+// thread hold, and where there is no memory for the pivots of all lines
 template <int AXIS>
 __global__ void k_ad_diag(Dims d, Met m, const int8_t *ib, const int8_t *gh, double *var, const double *r, Faces F,
-                          double half_dt, double omega, const double *binv, int diag, double *scr) {
+                          double half_dt, double omega, int diag, double *scr) {
   constexpr int P = AXIS == 0 ? 1 : 0, Q = AXIS == 2 ? 1 : 2;
   const int amax = AXIS == 0 ? d.ny - 1 : d.nx - 1;
   const int bmax = AXIS == 2 ? d.ny - 1 : d.nz - 1;
@@ -509,7 +510,7 @@ __global__ void k_ad_diag(Dims d, Met m, const int8_t *ib, const int8_t *gh, dou
   u[0] = var[base];  // row 0: the trivial equation u = var
   double c_prev = 0.0, bi = 1.0;
   for (int s = 1; s <= n; ++s) {
-    double am = 0.0, ap = 0.0, rh;
+    double am = 0.0, ac = 1.0, ap = 0.0, rh;
     const long long id = base + step * s;
     if (s == n) {
       rh = var[id];
@@ -522,13 +523,16 @@ __global__ void k_ad_diag(Dims d, Met m, const int8_t *ib, const int8_t *gh, dou
       rh = r[id] - (var[id - st[P]] * x.lo + var[id + st[P]] * x.hi + var[id - st[Q]] * y.lo +
                     var[id + st[Q]] * y.hi);
       const double rib = fluid(ib, gh, id);
+      // acx + acy + acz
+      const double sum = AXIS == 0 ? o.ac + x.ac + y.ac : AXIS == 1 ? x.ac + o.ac + y.ac : x.ac + y.ac + o.ac;
       am = o.lo * rib;
       ap = o.hi * rib;
+      ac = 1.0 + sum * rib;
       rh = rh * rib + var[id] * (1.0 - rib);
     }
     // CORE_TDMA.F90:22-27
     g[s] = c_prev * bi;
-    bi = binv[id];
+    bi = 1.0 / (ac - am * g[s]);
     u[s] = (rh - am * u[s - 1]) * bi;
     c_prev = ap;
   }
@@ -909,14 +913,13 @@ cudaError_t launch_sweeps(const ad::Dims &d, const ad::Met &m, const int8_t *ib,
 // a sweep along AXIS one anti-diagonal at a time
 template <int AXIS, int NC>
 void diag_sweep(const ad::Dims &d, const ad::Met &m, const int8_t *ib, const int8_t *gh, const ad::Comps<NC> &C,
-                const ad::Faces &F, double half_dt, double omega, const double *binv, double *scr, cudaStream_t s,
-                long long &launches) {
+                const ad::Faces &F, double half_dt, double omega, double *scr, cudaStream_t s, long long &launches) {
   const int np = AXIS == 0 ? d.ny - 1 : d.nx - 1, nq = AXIS == 2 ? d.ny - 1 : d.nz - 1;
   for (int e = 0; e < NC; ++e)
     for (int diag = 2; diag <= np + nq; ++diag) {
       const int nl = std::min(np, diag - 1) - std::max(1, diag - nq) + 1;
       ad::k_ad_diag<AXIS><<<(unsigned)((nl + 63) / 64), 64, 0, s>>>(d, m, ib, gh, C.v[e], C.r[e], F, half_dt, omega,
-                                                                    binv, diag, scr);
+                                                                    diag, scr);
       ++launches;
     }
 }
@@ -932,48 +935,60 @@ fg_status ad_sweeps(fg_case *c, const ad::Comps<NC> &C, const ad::Faces &F, cons
   const size_t nref = (size_t)(c->nx + 2) * (c->ny + 2) * (c->nz + 2);
   const int8_t *ib = c->d_refmask, *gh = c->d_refmask + nref;
   const double half_dt = prm->crank_nicolson ? 0.5 * prm->dt : 0.0, om = prm->omega_ad;
-  const int nmax = std::max(c->nx, std::max(c->ny, c->nz)), rows = sweep_rows(nmax);
-  // scratch: the pivots of the three directions; an error flag, a ticket and
-  // the columns' progress; for lines too long for k_ad_sweeps one line per
-  // thread of a diagonal
+  const int nmax = std::max(c->nx, std::max(c->ny, c->nz));
+  int rows = sweep_rows(nmax);
+  // scratch: the pivots of the three directions, an error flag, a ticket and
+  // the columns' progress; for lines too long for k_ad_sweeps, and where
+  // the three fields of pivots cannot be had, one line per thread of a
+  // diagonal
+  double *ws = nullptr;
+  cudaError_t e = cudaErrorMemoryAllocation;
   const size_t nsync = 2 + 3 * (size_t)nmax;
-  size_t nscr = 0;
+  if (rows) {
+    e = fg::dev_alloc(&ws, 3 * nref * sizeof(double) + nsync * sizeof(int));
+    if (e == cudaErrorMemoryAllocation) {
+      (void)cudaGetLastError();
+      rows = 0;
+    }
+  }
   if (!rows) {
     const int lmax = std::max(std::min(c->ny, c->nz), std::max(std::min(c->nx, c->nz), std::min(c->nx, c->ny)));
-    nscr = (size_t)lmax * 2 * (nmax + 1);
+    e = fg::dev_alloc(&ws, (size_t)lmax * 2 * (nmax + 1) * sizeof(double));
   }
-  double *ws = nullptr;
-  FG_CUDA(fg::dev_alloc(&ws, (3 * nref + nscr) * sizeof(double) + nsync * sizeof(int)));
-  double *binv = ws, *scr = ws + 3 * nref;
-  int *sync = reinterpret_cast<int *>(scr + nscr);
-  const ad::SweepSync sy = {sync, sync + 1, {sync + 2, sync + 2 + nmax, sync + 2 + 2 * nmax}};
+  FG_CUDA(e);
   cudaStream_t s = c->stream;
-  long long launches = 1;
-  cudaError_t e = cudaMemsetAsync(sync, 0, nsync * sizeof(int), s);
-  const size_t ft = 2 * sizeof(ad::FactorTile);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(ad::k_ad_factor, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ft);
-  if (e == cudaSuccess) {
-    auto groups = [](int np, int nq) { return (np + ad::FT_LINES - 1) / ad::FT_LINES * nq; };
-    const int nb = std::max(groups(d.ny - 1, d.nz - 1), std::max(groups(d.nx - 1, d.nz - 1), groups(d.nx - 1, d.ny - 1)));
-    ad::k_ad_factor<<<dim3(nb, 3), 32 + ad::FT_WORK, ft, s>>>(d, m, ib, gh, F, half_dt, binv, (long long)nref);
-    e = cudaGetLastError();
-  }
-  if (e == cudaSuccess && rows) {
-    launches += 1;
-    const long long nr = (long long)nref;
-    e = rows == 1   ? launch_sweeps<1, NC>(d, m, ib, gh, C, F, half_dt, om, binv, nr, sy, s)
-        : rows == 2 ? launch_sweeps<2, NC>(d, m, ib, gh, C, F, half_dt, om, binv, nr, sy, s)
-                    : launch_sweeps<4, NC>(d, m, ib, gh, C, F, half_dt, om, binv, nr, sy, s);
-  } else if (e == cudaSuccess) {
-    diag_sweep<0, NC>(d, m, ib, gh, C, F, half_dt, om, binv, scr, s, launches);
-    diag_sweep<1, NC>(d, m, ib, gh, C, F, half_dt, om, binv + nref, scr, s, launches);
-    diag_sweep<2, NC>(d, m, ib, gh, C, F, half_dt, om, binv + 2 * nref, scr, s, launches);
+  long long launches = 0;
+  int *sync = reinterpret_cast<int *>(ws + 3 * nref);
+  if (rows) {
+    const double *binv = ws;
+    const ad::SweepSync sy = {sync, sync + 1, {sync + 2, sync + 2 + nmax, sync + 2 + 2 * nmax}};
+    e = cudaMemsetAsync(sync, 0, nsync * sizeof(int), s);
+    const size_t ft = 2 * sizeof(ad::FactorTile);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(ad::k_ad_factor, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ft);
+    if (e == cudaSuccess) {
+      auto groups = [](int np, int nq) { return (np + ad::FT_LINES - 1) / ad::FT_LINES * nq; };
+      const int nb =
+          std::max(groups(d.ny - 1, d.nz - 1), std::max(groups(d.nx - 1, d.nz - 1), groups(d.nx - 1, d.ny - 1)));
+      ad::k_ad_factor<<<dim3(nb, 3), 32 + ad::FT_WORK, ft, s>>>(d, m, ib, gh, F, half_dt, ws, (long long)nref);
+      e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) {
+      launches = 2;
+      const long long nr = (long long)nref;
+      e = rows == 1   ? launch_sweeps<1, NC>(d, m, ib, gh, C, F, half_dt, om, binv, nr, sy, s)
+          : rows == 2 ? launch_sweeps<2, NC>(d, m, ib, gh, C, F, half_dt, om, binv, nr, sy, s)
+                      : launch_sweeps<4, NC>(d, m, ib, gh, C, F, half_dt, om, binv, nr, sy, s);
+    }
+  } else {
+    diag_sweep<0, NC>(d, m, ib, gh, C, F, half_dt, om, ws, s, launches);
+    diag_sweep<1, NC>(d, m, ib, gh, C, F, half_dt, om, ws, s, launches);
+    diag_sweep<2, NC>(d, m, ib, gh, C, F, half_dt, om, ws, s, launches);
     e = cudaGetLastError();
   }
   note_launches(launches);
   int gave_up = 0;
-  if (e == cudaSuccess) e = cudaMemcpyAsync(&gave_up, sync, sizeof(int), cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess && rows) e = cudaMemcpyAsync(&gave_up, sync, sizeof(int), cudaMemcpyDeviceToHost, s);
   const cudaError_t es = cudaStreamSynchronize(s);
   if (e == cudaSuccess) e = es;
   {

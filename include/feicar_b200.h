@@ -286,7 +286,13 @@ fg_status fg_ghostcell_velocity_device(fg_case *c, double *u, double *v, double 
  * solved as a wavefront, which gives the reference's lexicographic
  * Gauss-Seidel sweep bit for bit.  The ghost-cell
  * coefficients the z sweep stores (ghostNScoeff) are not kept: the
- * velocity ghost-cell update stays with the caller. */
+ * velocity ghost-cell update stays with the caller.
+ * A pass takes 24 bytes of device scratch per node, which the estimate of
+ * fg_case_estimate_bytes does not hold; where they cannot be had, and for
+ * lines of more than 2048 cells, the lines are solved one anti-diagonal at
+ * a time in a few lines' scratch, with the same result and many times
+ * slower.  FG_TIMEOUT: the wavefront's bounded waits ran out (a few
+ * seconds without progress); the component is then partly swept. */
 typedef struct fg_ad_params {
   double dt, reinv, omega_ad;
   int crank_nicolson;
@@ -348,7 +354,8 @@ fg_status fg_enforce_global_mass_consv_device(fg_case *c, double *face_u, double
  * its location.  An iteration count that reaches itermax_ad is reported
  * in the outputs, not as an error (the reference prints it and goes on);
  * ghost velocities that do not converge return FG_NOT_CONVERGED (the
- * reference stops the run there). */
+ * reference stops the run there).  Scratch and FG_TIMEOUT as
+ * fg_itsolv_ad_device's, for the three components together. */
 typedef struct fg_solve_ad_stats {
   int iterations;
   double residual;
