@@ -932,8 +932,8 @@ static fg_status build_batch(fg_batch *b) {
         vSn.push_back(c->lev[L + 1].dl);
         bc.push_back(k::blocks_ptile(d));  // the prolongation into level L
         bx.push_back(k::blocks_xline(d, s.maxnx, b->tune.var[L][0]));
-        by.push_back(k::blocks_tile(d, 1, s.maxny, b->tune.var[L][1]));
-        bz.push_back(k::blocks_tile(d, 2, s.maxnz, b->tune.var[L][2]));
+        by.push_back(k::blocks_tile(d, 1, s.maxny, s.maxnx, b->tune.var[L][1]));
+        bz.push_back(k::blocks_tile(d, 2, s.maxnz, s.maxnx, b->tune.var[L][2]));
         bn.push_back(k::blocks_cells(c->lev[L + 1].dl));
         bq.push_back(k::blocks_quads(d));
         br.push_back(k::blocks_restrict(d, c->lev[L + 1].dl));
@@ -1082,7 +1082,7 @@ static fg_status smooth(fg_batch *b, int L, cudaStream_t s) {
     const bool both = k::line_both_colours(axis, maxn, b->tune.var[L][axis]);
     for (int color = 0; color < (both ? 1 : 2); ++color) {
       const size_t e0 = prof_begin(b, s);
-      FG_K(k::line_sweep<T>(Lr, axis, color, om, maxn, b->tune.var[L][axis], s));
+      FG_K(k::line_sweep<T>(Lr, axis, color, om, maxn, ls.maxnx, b->tune.var[L][axis], s));
       prof_end(b, e0, cls, (both ? 2.0 : 1.0) * sweep_bytes<T>(ls.ncells, om), s);
     }
     if (L == 0) {
@@ -1832,7 +1832,8 @@ static fg_status rebuild_line_offsets(fg_batch *b, int L, int axis) {
     const DevLevel &d = b->cases[p]->lev[L].dl;
     lev.push_back(d);
     blocks.push_back(axis == 0 ? k::blocks_xline(d, s.maxnx, b->tune.var[L][0])
-                               : k::blocks_tile(d, axis, axis == 1 ? s.maxny : s.maxnz, b->tune.var[L][axis]));
+                               : k::blocks_tile(d, axis, axis == 1 ? s.maxny : s.maxnz, s.maxnx,
+                                                b->tune.var[L][axis]));
   }
   int **off = axis == 0 ? &s.d_off_x : axis == 1 ? &s.d_off_y : &s.d_off_z;
   Launch &Lr = axis == 0 ? s.xl : axis == 1 ? s.yl : s.zl;
@@ -1873,7 +1874,7 @@ static fg_status tune_lines(fg_batch *b) {
       const int maxn = axis == 0 ? ls.maxnx : axis == 1 ? ls.maxny : ls.maxnz;
       std::vector<int> cand;
       for (int v = 1; v <= (axis == 0 ? k::LV_NX : k::LV_NYZ); ++v) {
-        const int r = k::line_variant(axis, maxn, v);
+        const int r = k::line_variant(axis, maxn, ls.maxnx, v);
         if (std::find(cand.begin(), cand.end(), r) == cand.end()) cand.push_back(r);
       }
       double best = 1e300;
@@ -1886,7 +1887,7 @@ static fg_status tune_lines(fg_batch *b) {
         for (int rep = 0; rep < 4 && e == cudaSuccess; ++rep) {
           if (rep == 1) e = cudaEventRecord(e0, s);
           for (int color = 0; color < 2 && e == cudaSuccess; ++color)
-            e = k::line_sweep<T>(Lr, axis, color, om, maxn, v, s);
+            e = k::line_sweep<T>(Lr, axis, color, om, maxn, ls.maxnx, v, s);
         }
         if (e == cudaSuccess) e = cudaEventRecord(e1, s);
         if (e == cudaSuccess) e = cudaEventSynchronize(e1);
@@ -2947,7 +2948,7 @@ fg_status fg_batch_get_tuning(const fg_batch *b, fg_tuning *out) {
       const auto &ls = b->ls[L];
       const int maxn = a == 0 ? ls.maxnx : a == 1 ? ls.maxny : ls.maxnz;
       const bool lines = !ls.S.empty() && L < cycle_start(b);
-      out->line_variant[L][a] = lines ? k::line_variant(a, maxn, b->tune.var[L][a]) : 0;
+      out->line_variant[L][a] = lines ? k::line_variant(a, maxn, ls.maxnx, b->tune.var[L][a]) : 0;
       out->line_us[L][a] = b->tune.us[L][a];
     }
   out->nu1 = b->cfg.nu1;

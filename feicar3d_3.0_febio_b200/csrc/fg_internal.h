@@ -330,14 +330,16 @@ bool line_both_colours(int axis, int maxn, int variant);
 // FG_TIMEOUT (once) if a both-colour y/z sweep gave up a wait since the
 // last call
 fg_status wave_error_take();
-int line_variant(int axis, int maxn, int v);  // the family that runs
+// the family that runs; maxn, maxnx: the longest line of the level set along
+// `axis` and along x
+int line_variant(int axis, int maxn, int maxnx, int v);
 int blocks_xline(const DevLevel &L, int maxn, int variant);
 // y/z tiles: blocks depend on the kernel the level set's longest line picks
-int blocks_tile(const DevLevel &L, int axis, int maxn, int variant);
+int blocks_tile(const DevLevel &L, int axis, int maxn, int maxnx, int variant);
 size_t smem_line(int n, int tsize, int axis);
 
 template <typename T>
-cudaError_t line_sweep(const Launch &L, int axis, int color, double omega, int maxn, int variant,
+cudaError_t line_sweep(const Launch &L, int axis, int color, double omega, int maxn, int maxnx, int variant,
                        cudaStream_t s);
 // norm2[p] += ||r||^2 of entry p when norm2 != null (part: one double per block)
 template <typename T>

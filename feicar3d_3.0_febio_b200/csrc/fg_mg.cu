@@ -1257,11 +1257,16 @@ int blocks_cells(const DevLevel &L) {
 int xline_lanes(int maxn) { return maxn <= 16 ? 4 : maxn <= 32 ? 8 : maxn <= 64 ? 16 : 32; }
 // The line kernel family a level set's sweep along `axis` takes (LV_*):
 // the requested one when it can take lines of maxn cells, else the
-// default: the family measured fastest for that line length.  Short y/z lines
-// take the block-PCR tiles too (per sweep against the register tiles, B200:
-// 64 rows of 128x64x64 cells FP32 14.4 and 16.7 us, 49 rows of 101x49x38 12.6
-// and 15.3, the 56-row levels of 16 cubes 20.8 and 37.1, in FP64 29.0 and 50.2).
-int line_variant(int axis, int maxn, int v) {
+// default: the family measured fastest for that line length.  y/z lines of 17
+// rows and more take the block-PCR tiles.  Up to 16 rows the register tiles
+// of 64 cells along x are the faster ones once a line of x fills one, the PCR
+// tiles of 32 cells before that (a colour of a sweep, register / PCR tiles,
+// FP64: 400x400x4 cells 19.1 / 24.0 us, 400x400x16 21.9 / 25.6, 400x400x17
+// 42.2 / 24.7; 128x600x8 11.5 / 14.6, 80x600x8 11.2 / 10.7, 64x600x8 7.7 / 9.6,
+// 48x600x8 7.9 / 6.8, 24x600x8 7.7 / 6.1; FP32: 400x400x4 16.4 / 18.9,
+// 400x400x16 17.8 / 20.0, 400x400x17 34.4 / 19.3, 64x600x8 6.6 / 6.8, 48x600x8
+// 6.7 / 6.0, 24x600x8 6.7 / 5.2).
+int line_variant(int axis, int maxn, int maxnx, int v) {
   if (axis == 0) {
     if (v == LV_XREG && maxn > 128) v = LV_DEFAULT;
     if (v == LV_XREG32 && maxn > 128) v = LV_DEFAULT;
@@ -1273,21 +1278,21 @@ int line_variant(int axis, int maxn, int v) {
   if ((v == LV_YREG || pcr) && maxn > YZ_MAXROWS) v = LV_DEFAULT;
   if (pcr && v != LV_YPCR && v != LV_YWAVE && maxn < YP_MINROWS) v = LV_DEFAULT;
   if (v != LV_YREG && v != LV_YWARP && !pcr)
-    v = maxn <= YZ_MAXROWS ? LV_YPCR : LV_YWARP;
+    v = maxn <= 16 && maxnx >= 64 ? LV_YREG : maxn <= YZ_MAXROWS ? LV_YPCR : LV_YWARP;
   return v;
 }
 int blocks_xline(const DevLevel &L, int maxn, int variant) {
   const long long lines = (long long)((L.ny + 1) / 2) * L.nz;
-  const int v = line_variant(0, maxn, variant);
+  const int v = line_variant(0, maxn, maxn, variant);
   // k_xline_smem: one line per warp; k_xline_reg: 32 / lanes lines per warp
   const long long per_block = v == LV_XSMEM ? (long long)XS_WARPS
                               : v == LV_XREG32 ? (long long)XL_WARPS
                                                : (long long)XL_WARPS * (32 / xline_lanes(maxn));
   return (int)((lines + per_block - 1) / per_block);
 }
-int blocks_tile(const DevLevel &L, int axis, int maxn, int variant) {
+int blocks_tile(const DevLevel &L, int axis, int maxn, int maxnx, int variant) {
   // i-tile of k_yzline_reg (64 cells), k_yzline_pcr (16) or k_yzline (16)
-  const int v = line_variant(axis, maxn, variant);
+  const int v = line_variant(axis, maxn, maxnx, variant);
   const int w = v == LV_YREG ? 64 : (v == LV_YPCR || v == LV_YPCRH || v == LV_YPCR4 || v == LV_YWAVE) ? 2 * YP_LINES : TILE_I;
   const int ntx = (L.nx + w - 1) / w;
   return ntx * (axis == 1 ? L.nz : L.ny);
@@ -1752,7 +1757,7 @@ fg_status wave_error_take() {
 }
 
 bool line_both_colours(int axis, int maxn, int variant) {
-  return axis != 0 && line_variant(axis, maxn, variant) == LV_YWAVE;
+  return axis != 0 && line_variant(axis, maxn, maxn, variant) == LV_YWAVE;
 }
 
 template <typename T, int M, int CH>
@@ -1767,15 +1772,13 @@ static cudaError_t launch_yzreg(const Launch &Lr, int axis, int color, double om
   return cudaGetLastError();
 }
 
-// x lines always take the register kernel (lines up to 1024 cells; lines
-// per warp as xline_lanes); y/z lines up to YZ_MAXROWS cells take
-// k_yzline_reg, longer ones the shared-memory tile kernel (blocks_tile and
-// blocks_xline count blocks the same way)
+// the sweep in the family line_variant names (lines per warp of an x sweep as
+// xline_lanes; blocks_tile and blocks_xline count blocks the same way)
 template <typename T>
-cudaError_t line_sweep(const Launch &Lr, int axis, int color, double omega, int maxn, int variant,
+cudaError_t line_sweep(const Launch &Lr, int axis, int color, double omega, int maxn, int maxnx, int variant,
                        cudaStream_t s) {
   if (Lr.empty()) return cudaSuccess;
-  const int v = line_variant(axis, maxn, variant);
+  const int v = line_variant(axis, maxn, maxnx, variant);
   if (axis == 0) {
     if (v == LV_XREG) {
       if (maxn <= 16) return launch_xreg<T, 4, 4>(Lr, color, omega, s);
@@ -4642,8 +4645,8 @@ extern "C" fg_status fg_debug_check(long long *out) {
 }
 #endif
 
-template cudaError_t line_sweep<double>(const Launch &, int, int, double, int, int, cudaStream_t);
-template cudaError_t line_sweep<float>(const Launch &, int, int, double, int, int, cudaStream_t);
+template cudaError_t line_sweep<double>(const Launch &, int, int, double, int, int, int, cudaStream_t);
+template cudaError_t line_sweep<float>(const Launch &, int, int, double, int, int, int, cudaStream_t);
 template cudaError_t residual<double>(const Launch &, double *, double *, cudaStream_t);
 template cudaError_t prolong_add<double>(const Launch &, const Launch &, cudaStream_t);
 template cudaError_t prolong_add<float>(const Launch &, const Launch &, cudaStream_t);

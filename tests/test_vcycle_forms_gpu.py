@@ -92,6 +92,20 @@ def test_cluster_and_launches(cells, body, outlet, prec):
     c.close()
 
 
+@pytest.mark.parametrize("prec", [fg.FG_PREC_FP64, fg.FG_PREC_MIXED])
+@pytest.mark.parametrize("cells", [(63, 150, 16), (64, 150, 16), (64, 150, 17), (130, 2, 150), (200, 16, 140),
+                                   (65, 5, 200)])
+def test_families_of_short_lines(cells, prec):
+    """The default families of y/z lines around 16 rows and x lines around 64
+    cells against one family for all."""
+    c, f, p0 = _case(cells, prec)
+    one = _cycle(c, f, p0)
+    for fams in (LAUNCHES, {"x": 1, "y": 1, "z": 1}):
+        fg.case_set_tuning(c, fams)
+        _same(one, _cycle(c, f, p0), prec)
+    c.close()
+
+
 @pytest.mark.parametrize("nu", [(1, 1), (1, 0), (3, 2)])
 def test_smoothing_steps(nu):
     c, f, p0 = _case((33, 20, 27), fg.FG_PREC_FP64, 0.5, nu1=nu[0], nu2=nu[1])
