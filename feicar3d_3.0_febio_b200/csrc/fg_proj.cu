@@ -126,12 +126,33 @@ __device__ __forceinline__ int layer_of(const Dims &d, int vzg, int i, int j, in
 // sum div dV and of max |div|.  DIV = false: the flux alone.  The cells
 // next to a zero-gradient face are left out of the last two: the flux
 // correction changes their faces, and k_div_layer forms them again
-// afterwards.
+// afterwards.  The blocks past the columns' nz clear div's boundary layers
+// (indices 0, n and n + 1 of each axis) and the first block the counters of
+// the reductions that follow: small grids are bound by the number of
+// launches (24x16x16 cells, the call without and with an outflow correction:
+// 35 and 49 us; with a launch each for these and for the sums 47 and 65).
 template <bool DIV>
 __global__ void __launch_bounds__(PJ_I * PJ_J)
 k_div(Dims d, Met m, int kspan, int vzg, const int8_t *__restrict__ ib, const int8_t *__restrict__ gh,
       const double *__restrict__ fu, const double *__restrict__ fv, const double *__restrict__ fw, double dtinv,
-      double *__restrict__ div, double *pflux, double *psum, double *pmax) {
+      double *__restrict__ div, double *pflux, double *psum, double *pmax, int *count, int nz) {
+  const bool first = threadIdx.x == 0 && threadIdx.y == 0;
+  const int b = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
+  if (first && b == 0) count[0] = count[1] = 0;
+  if (DIV && blockIdx.z >= (unsigned)nz) {
+    const int n0 = gridDim.x * gridDim.y * nz;
+    const long long t = (long long)(b - n0) * (PJ_I * PJ_J) + threadIdx.x + PJ_I * threadIdx.y;
+    const long long nt = (long long)(gridDim.x * gridDim.y * gridDim.z - n0) * (PJ_I * PJ_J);
+    for (int a = 0; a < 3; ++a) {
+      const int n = a == 0 ? d.nx : a == 1 ? d.ny : d.nz;
+      const long long n1 = a == 0 ? d.NY : d.NX, n2 = a == 2 ? d.NY : d.nz + 2;
+      for (long long e = t; e < n1 * n2; e += nt) {
+        const int q = (int)(e / n1), p = (int)(e - n1 * q);
+        for (const int l : {0, n, n + 1}) div[a == 0 ? d.id(l, p, q) : a == 1 ? d.id(p, l, q) : d.id(p, q, l)] = 0.0;
+      }
+    }
+    return;
+  }
   const Col c = column(d, kspan);
   double flux = 0.0, s = 0.0, mx = 0.0;
   if (c.ok) {
@@ -157,8 +178,6 @@ k_div(Dims d, Met m, int kspan, int vzg, const int8_t *__restrict__ ib, const in
       f0 = f1;
     }
   }
-  const int b = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
-  const bool first = threadIdx.x == 0 && threadIdx.y == 0;
   if (vzg) {
     double none = 0.0;
     block_sum_max<PJ_I * PJ_J / 32>(flux, none);
@@ -168,18 +187,6 @@ k_div(Dims d, Met m, int kspan, int vzg, const int8_t *__restrict__ ib, const in
     block_sum_max<PJ_I * PJ_J / 32>(s, mx);
     if (first) { psum[b] = s; pmax[b] = mx; }
   }
-}
-
-// div's boundary layers (indices 0 and n, n + 1 of each axis) are zero; one
-// thread per (first, second) index pair of three planes of an axis
-__global__ void k_div_bounds(Dims d, double *div) {
-  const int a = blockIdx.y;
-  const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long n1 = a == 0 ? d.NY : d.NX, n2 = a == 2 ? d.NY : d.nz + 2;
-  if (e >= n1 * n2) return;
-  const int p = (int)(e % n1), q = (int)(e / n1);
-  const int n = a == 0 ? d.nx : a == 1 ? d.ny : d.nz;
-  for (const int l : {0, n, n + 1}) div[a == 0 ? d.id(l, p, q) : a == 1 ? d.id(p, l, q) : d.id(p, q, l)] = 0.0;
 }
 
 // div and its partials on the cells next to the zero-gradient faces, from
@@ -217,8 +224,8 @@ k_div_layer(Dims d, Met m, int vzg, const int8_t *__restrict__ ib, const int8_t 
   }
 }
 
-// Sums over the partials and what depends on them, RB blocks; the last one to
-// finish adds the blocks' results in order.  AREA: out[0] = -flux / (fluid
+// Sums over the partials and what depends on them, up to RB blocks; the last
+// one to finish adds the blocks' results in order.  AREA: out[0] = -flux / (fluid
 // area of the flagged faces), the outflow correction; else out[0] = sum of
 // psum, out[1] = maximum of pmax.
 constexpr int RB = 64;
@@ -227,8 +234,8 @@ __global__ void __launch_bounds__(256)
 k_reduce(Dims d, Met m, const int8_t *__restrict__ ib, int vzg, const double *psum, const double *pmax, int n,
          double *blk, int *count, double *out) {
   double s = 0.0, x = 0.0;
-  const int t0 = blockIdx.x * 256 + threadIdx.x;
-  for (int b = t0; b < n; b += RB * 256) {
+  const int t0 = blockIdx.x * 256 + threadIdx.x, nt = gridDim.x * 256, nblk = gridDim.x;
+  for (int b = t0; b < n; b += nt) {
     s += psum[b];
     if (!AREA) x = fmax(x, pmax[b]);
   }
@@ -238,7 +245,7 @@ k_reduce(Dims d, Met m, const int8_t *__restrict__ ib, int vzg, const double *ps
       const int a = f >> 1, up = f & 1;
       const int nu = a == 0 ? d.ny - 1 : d.nx - 1, nv = a == 2 ? d.ny - 1 : d.nz - 1;
       const int layer = a == 0 ? (up ? d.nx - 1 : 1) : a == 1 ? (up ? d.ny - 1 : 1) : (up ? d.nz - 1 : 1);
-      for (int e = t0; e < nu * nv; e += RB * 256) {
+      for (int e = t0; e < nu * nv; e += nt) {
         const int p = 1 + e % nu, q = 1 + e / nu;
         long long id;
         double w;
@@ -255,25 +262,39 @@ k_reduce(Dims d, Met m, const int8_t *__restrict__ ib, int vzg, const double *ps
   x = AREA ? warp_sum(x) : warp_max(x);
   if ((threadIdx.x & 31) == 0) { rs[threadIdx.x >> 5] = s; rx[threadIdx.x >> 5] = x; }
   __syncthreads();
+  auto store = [&](double a, double b) {
+    if (AREA) out[0] = -a / b;
+    else { out[0] = a; out[1] = b; }
+  };
   if (threadIdx.x == 0) {
     double a = 0.0, b = 0.0;
     for (int q = 0; q < 8; ++q) { a += rs[q]; b = AREA ? b + rx[q] : fmax(b, rx[q]); }
-    blk[2 * blockIdx.x] = a;
-    blk[2 * blockIdx.x + 1] = b;
-    __threadfence();
-    last = atomicAdd(count, 1) == RB - 1;
+    last = false;
+    if (nblk == 1) {
+      store(a, b);
+    } else {
+      blk[2 * blockIdx.x] = a;
+      blk[2 * blockIdx.x + 1] = b;
+      __threadfence();
+      last = atomicAdd(count, 1) == nblk - 1;
+    }
   }
   __syncthreads();
-  if (!last || threadIdx.x != 0) return;
+  if (!last) return;
   __threadfence();
-  double a = 0.0, b = 0.0;
-  for (int q = 0; q < RB; ++q) {
-    a += __ldcg(blk + 2 * q);
-    const double y = __ldcg(blk + 2 * q + 1);
-    b = AREA ? b + y : fmax(b, y);
+  __shared__ double fs[RB], fx[RB];  // read at once: one after another they cost a small grid 5 us
+  if (threadIdx.x < nblk) {
+    fs[threadIdx.x] = __ldcg(blk + 2 * threadIdx.x);
+    fx[threadIdx.x] = __ldcg(blk + 2 * threadIdx.x + 1);
   }
-  if (AREA) out[0] = -a / b;
-  else { out[0] = a; out[1] = b; }
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  double a = 0.0, b = 0.0;
+  for (int q = 0; q < nblk; ++q) {
+    a += fs[q];
+    b = AREA ? b + fx[q] : fmax(b, fx[q]);
+  }
+  store(a, b);
 }
 
 // the correction on the zero-gradient faces: the boundary arrays over
@@ -450,10 +471,20 @@ Cols columns(const fg_case *c) {
   q.grid.z = (c->nz - 1 + q.kspan - 1) / q.kspan;
   return q;
 }
-unsigned face_blocks(const fg_case *c, int extra) {
-  const long long big = (long long)(std::max(c->nx, c->ny) + extra) * (std::max(c->ny, c->nz) + extra);
-  return (unsigned)((big + 255) / 256);
+// slices of blocks that clear a field's boundary layers beside such columns:
+// about four index pairs of an axis's planes per thread
+unsigned boundary_slices(const fg_case *c, const Cols &q) {
+  const long long x = c->nx + 2, y = c->ny + 2, z = c->nz + 2;
+  const long long slice = 4ll * proj::PJ_I * proj::PJ_J * q.grid.x * q.grid.y;
+  return (unsigned)((x * y + y * z + x * z + slice - 1) / slice);
 }
+long long face_cells(const fg_case *c, int extra) {
+  const long long x = c->nx + extra, y = c->ny + extra, z = c->nz + extra;
+  return std::max(x * y, std::max(y * z, x * z));
+}
+unsigned face_blocks(const fg_case *c, int extra) { return (unsigned)((face_cells(c, extra) + 255) / 256); }
+// blocks of a reduction over n values, four per thread
+unsigned reduce_blocks(long long n) { return (unsigned)std::min<long long>(proj::RB, std::max(1ll, (n + 1023) / 1024)); }
 
 // device scratch of one call, given back when its stream has been waited for
 struct Scratch {
@@ -478,7 +509,8 @@ void enqueue_correction(fg_case *c, const proj::Met &m, const proj::Dims &d, int
                         double *fw, double *bcxu, double *bcyv, double *bczw, const double *part, double *blk,
                         int *count, double *cv) {
   cudaStream_t s = c->stream;
-  proj::k_reduce<true><<<proj::RB, 256, 0, s>>>(d, m, c->d_refmask, vzg, part, nullptr, nb, blk, count, cv);
+  proj::k_reduce<true><<<reduce_blocks(std::max<long long>(nb, face_cells(c, 0))), 256, 0, s>>>(
+      d, m, c->d_refmask, vzg, part, nullptr, nb, blk, count, cv);
   proj::k_massflux_apply<<<dim3(face_blocks(c, 1), 6), 256, 0, s>>>(d, vzg, cv, bcxu, bcyv, bczw, fu, fv, fw);
 }
 
@@ -529,24 +561,35 @@ fg_status fg_rhs_poisson_device(fg_case *c, double *face_u, double *face_v, doub
   int *count = reinterpret_cast<int *>(res + 3);
   cudaStream_t s = c->stream;
   const double dtinv = 1.0 / dt;
-  cudaError_t e = cudaMemsetAsync(count, 0, 2 * sizeof(int), s);
-  if (e == cudaSuccess) {
-    proj::k_div<true><<<q.grid, q.block, 0, s>>>(d, m, q.kspan, vzg, ib, gh, face_u, face_v, face_w, dtinv, div, flux,
-                                                 psum, pmax);
-    proj::k_div_bounds<<<dim3(face_blocks(c, 2), 3), 256, 0, s>>>(d, div);
-    if (vzg) {
-      enqueue_correction(c, m, d, vzg, nb, face_u, face_v, face_w, bcxu, bcyv, bczw, flux, blk, count, res + 2);
-      proj::k_div_layer<<<dim3(lb, 6), 256, 0, s>>>(d, m, vzg, ib, gh, face_u, face_v, face_w, dtinv, div, psum + nb,
-                                                    pmax + nb);
-    }
-    proj::k_reduce<false><<<proj::RB, 256, 0, s>>>(d, m, ib, 0, psum, pmax, nb + nl, blk + 2 * proj::RB, count + 1, res);
-    note_launches(vzg ? 6 : 3);
-    e = cudaGetLastError();
+  dim3 grid = q.grid;
+  grid.z += boundary_slices(c, q);
+  proj::k_div<true><<<grid, q.block, 0, s>>>(d, m, q.kspan, vzg, ib, gh, face_u, face_v, face_w, dtinv, div, flux, psum,
+                                             pmax, count, (int)q.grid.z);
+  if (vzg) {
+    enqueue_correction(c, m, d, vzg, nb, face_u, face_v, face_w, bcxu, bcyv, bczw, flux, blk, count, res + 2);
+    proj::k_div_layer<<<dim3(lb, 6), 256, 0, s>>>(d, m, vzg, ib, gh, face_u, face_v, face_w, dtinv, div, psum + nb,
+                                                  pmax + nb);
   }
-  double h[2] = {0.0, 0.0};
-  if (e == cudaSuccess) e = cudaMemcpyAsync(h, res, sizeof(h), cudaMemcpyDeviceToHost, s);
+  // a small grid's partials are fewer bytes than a launch is worth: summed
+  // here (24x16x16 cells, 60 partials, the call 35 us so and 42 with the
+  // reduction's launch; 64^3 cells, 1008 partials, 45 and 50 us)
+  const int npart = nb + nl;
+  const bool here = npart <= 1024;
+  if (!here)
+    proj::k_reduce<false><<<reduce_blocks(npart), 256, 0, s>>>(d, m, ib, 0, psum, pmax, npart, blk + 2 * proj::RB,
+                                                               count + 1, res);
+  note_launches((vzg ? 4 : 1) + (here ? 0 : 1));
+  cudaError_t e = cudaGetLastError();
+  double h[2] = {0.0, 0.0}, part[2 * 1024];
+  if (e == cudaSuccess)
+    e = here ? cudaMemcpyAsync(part, psum, 2 * npart * sizeof(double), cudaMemcpyDeviceToHost, s)
+             : cudaMemcpyAsync(h, res, sizeof(h), cudaMemcpyDeviceToHost, s);
   const cudaError_t es = cudaStreamSynchronize(s);
   if (e == cudaSuccess) e = es;
+  for (int q = 0; here && e == cudaSuccess && q < npart; ++q) {
+    h[0] += part[q];
+    h[1] = std::max(h[1], part[npart + q]);
+  }
   if (e != cudaSuccess) {
     set_last_error(cudaGetErrorString(e), __FILE__, __LINE__);
     return FG_CUDA_ERROR;
@@ -573,18 +616,15 @@ fg_status fg_enforce_global_mass_consv_device(fg_case *c, double *face_u, double
   const Cols q = columns(c);
   const int nb = q.blocks();
   Scratch w;
-  FG_CUDA(fg::dev_alloc(&w.p, ((size_t)nb + 2 * proj::RB + 2) * sizeof(double)));
+  FG_CUDA(fg::dev_alloc(&w.p, ((size_t)nb + 2 * proj::RB + 1 + 1) * sizeof(double)));
   double *blk = w.p + nb, *cv = blk + 2 * proj::RB;
   int *count = reinterpret_cast<int *>(cv + 1);
   cudaStream_t s = c->stream;
-  cudaError_t e = cudaMemsetAsync(count, 0, sizeof(int), s);
-  if (e == cudaSuccess) {
-    proj::k_div<false><<<q.grid, q.block, 0, s>>>(d, m, q.kspan, vzg, ib, gh, face_u, face_v, face_w, 0.0, nullptr, w.p,
-                                                  nullptr, nullptr);
-    enqueue_correction(c, m, d, vzg, nb, face_u, face_v, face_w, bcxu, bcyv, bczw, w.p, blk, count, cv);
-    note_launches(3);
-    e = cudaGetLastError();
-  }
+  proj::k_div<false><<<q.grid, q.block, 0, s>>>(d, m, q.kspan, vzg, ib, gh, face_u, face_v, face_w, 0.0, nullptr, w.p,
+                                                nullptr, nullptr, count, (int)q.grid.z);
+  enqueue_correction(c, m, d, vzg, nb, face_u, face_v, face_w, bcxu, bcyv, bczw, w.p, blk, count, cv);
+  note_launches(3);
+  cudaError_t e = cudaGetLastError();
   const cudaError_t es = cudaStreamSynchronize(s);
   if (e == cudaSuccess) e = es;
   if (e != cudaSuccess) {
