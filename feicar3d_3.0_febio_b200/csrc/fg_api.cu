@@ -839,7 +839,16 @@ static fg_status rebuild_line_offsets(fg_batch *b, int L, int axis);
 // kernel then takes 1.5-3 us where a launch takes about 5.  More problems
 // fill the GPU through the launches, each of which serves all of them; they
 // get one block each, from the first level below level 0 whose hierarchy
-// fits its shared memory.
+// fits its shared memory, however many cells that level has: with levels of
+// at most 2048 or 8192 cells 64 mixed problems of 32 to 192 cells an edge take
+// 141.4 ms, so 140.6 (FP64 180.0 and 179.9).
+// The line at CL_MAXPROBS: a cluster each against one block each, solves of
+// cubes of 16 to 40 cells an edge, FP64: 8 problems 2.98 and 3.35 ms, 12 3.02
+// and 3.56, 16 3.95 and 4.90, 17 3.99 and 4.95, 24 4.61 and 5.78, 32 6.01 and
+// 6.89, 64 11.8 and 11.0; of 40 to 96 cells 16 13.0 and 14.5, 24 20.9 and 21.3,
+// 32 30.0 and 29.6, 64 67.1 and 64.3 (mixed 16 14.0 and 15.4, 24 20.7 and 22.4,
+// 32 30.2 and 31.0, 64 68.5 and 66.3).  The clusters stay ahead to about 32
+// problems: the line errs on the side of the launches.
 static fg_status build_cycle(fg_batch *b) {
   Cycle &cy = b->cyc;
   cy = Cycle();

@@ -69,12 +69,13 @@ __device__ __forceinline__ long long ridx(const Grid &g, int i, int j, int k) {
 }
 
 // One thread per cell of a box of ni x nj x nk cells whose first cell is
-// (i0, j0, j0), blocks of 32 x 8 cells of a plane: the block's number is taken
-// apart in 32 bits, where a linear cell number per thread costs two 64-bit
-// divisions and as many remainders.  The passes are bound by the instructions
-// of one thread per cell.  256^3 cells: ghost marks 128 -> 114 us, dead marks
-// 69 -> 62 us, the commit 71 -> 56 us, and a smoothing step, whose neighbours
-// are unrolled per mode besides, 149 -> 93 to 108 us.
+// (i0, j0, j0): its second and third index start alike.  Blocks of 32 x 8
+// cells of a plane: the block's number is taken apart in 32 bits, where a
+// linear cell number per thread costs two 64-bit divisions and as many
+// remainders.  The passes are bound by the instructions of one thread per
+// cell.  256^3 cells: ghost marks 128 -> 114 us, dead marks 69 -> 62 us, the
+// commit 71 -> 56 us, and a smoothing step, whose neighbours are unrolled per
+// mode besides, 149 -> 93 to 108 us.
 constexpr int BX_I = 32, BX_J = 8;
 static unsigned box_blocks(int ni, int nj, int nk) {
   return (unsigned)((ni + BX_I - 1) / BX_I) * (unsigned)((nj + BX_J - 1) / BX_J) * (unsigned)nk;
@@ -346,8 +347,10 @@ __global__ void k_classify(Grid g, Bodies BB, const int *cells, int ncells, int8
 // A cell outside the band has the values of the last band cell before it in
 // its line (of the first one of the line where there is none before it), so a
 // warp fills a line 32 cells at a time from the ballot of its band cells.
-// Bound by its reads and writes of three bytes per cell; 256^3 cells: a
-// thread walking each line 265 us, this 39 us.
+// 256^3 cells: a thread walking each line 265 us, this 39 us; the three bytes
+// per cell would take 8 us at a copy's rate, so what bounds it is the chain of
+// a line's 32-cell pieces, each of which needs the last value of the one
+// before.
 constexpr int FILL_WARPS = 8;
 __global__ void __launch_bounds__(32 * FILL_WARPS)
 k_fill(Grid g, const int8_t *band, int8_t *ibt, int8_t *body) {
