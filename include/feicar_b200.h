@@ -377,7 +377,9 @@ fg_status fg_update_pressure_device(fg_case *c, double *pPrime, double *p);
  * reference prints wall time per solve_poisson call only,
  * CORE_TIME_STEP.F90:180-185) ----- */
 /* Orders the handle's work on the caller's cudaStream_t (NULL: back to a
- * stream of the handle's own). */
+ * stream of the handle's own).  The handle's own stream is not ordered
+ * after work on any other, the default stream included: without this call,
+ * device arrays handed in have to be complete. */
 fg_status fg_case_set_stream(fg_case *c, void *stream);
 /* Kernels this process has launched through the library so far. */
 fg_status fg_launch_count(long long *count);
